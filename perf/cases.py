@@ -189,3 +189,79 @@ def tolerance(case):
     if case["dtype"] == "fp32":
         return {"rel": 4e-6, "max": 1e-4}
     return {"rel": 0.03 if case["call"] == "layer" else 0.015, "max": 0.99}
+
+
+_EXACT_MOST = 7.2e10    # heads x tokens^2 that the 64-bit evaluation takes in about 20 seconds
+
+
+def _exact_mask(q, k, case):
+    """The selection for one query head: the permuted order of the keys and the block mask.
+
+    Scores are summed in 64 bits and rounded to the input type where the path is defined to round them (after the dot
+    product, after the division, and the pooled rows), because a block is kept or not by those rounded values."""
+    S, D = q.shape
+    bs, dt, f = case["block"], q.dtype, torch.float64
+    mean = case["call"] == "mean"
+    seg = bs if mean else case["segment"]
+    rnd = lambda x: x.to(dt).to(f)
+    idx = torch.arange(S, device=q.device)
+    if not mean:
+        L = S // seg * seg
+        p = torch.softmax(rnd(rnd(q[-bs:].to(f) @ k[:L].to(f).T) / math.sqrt(D)), dim=-1).mean(dim=0)
+        order = torch.sort(p.float().view(-1, seg), dim=-1, descending=True, stable=True).indices
+        idx[:L] = (order + torch.arange(0, L, seg, device=q.device)[:, None]).flatten()
+    nb = -(-S // bs)
+    pool = lambda x: rnd(torch.nn.functional.pad(x.to(f), (0, 0, 0, nb * bs - S)).view(nb, bs, D).mean(dim=1))
+    score = rnd(rnd(pool(q) @ pool(k[idx]).T) / math.sqrt(D))
+    blk = torch.arange(nb, device=q.device)
+    own = (blk[:, None] // (seg // bs)) == (blk // (seg // bs))
+    cand = blk <= blk[:, None] if mean else (blk <= blk[:, None]) & ~own
+    p = torch.nan_to_num(torch.softmax(score.masked_fill(~cand, -math.inf), dim=-1).float())
+    val, order = torch.sort(p, dim=-1, descending=True, stable=True)
+    reached = torch.cumsum(val.to(f), dim=-1).float() >= case["threshold"]
+    keep = (blk <= reached.int().argmax(dim=-1, keepdim=True)) & reached.any(dim=-1, keepdim=True)
+    mask = torch.zeros_like(keep).scatter(-1, order, keep) | own
+    mask[:, int((idx == 0).nonzero()) // bs] = True
+    return idx, mask
+
+
+def _exact_attention(q, k, v, case):
+    B, Hq, S, D = q.shape
+    group = Hq // k.shape[1]
+    out = torch.empty(B, Hq, S, D, dtype=torch.float64, device=q.device)
+    bs = case["block"]
+    seg = bs if case["call"] == "mean" else case["segment"]
+    for b in range(B):
+        for h in range(Hq):
+            qh, kh, vh = q[b, h], k[b, h // group], v[b, h // group]
+            pos = torch.arange(S, device=q.device)
+            idx, mask = (pos, None) if case["call"] != "mean" and S <= seg else _exact_mask(qh, kh, case)
+            kf, vf = kh[idx].double(), vh[idx].double()
+            for r0 in range(0, S, 2048):
+                r1 = min(r0 + 2048, S)
+                n = S if mask is None else min(S, -(-r1 // seg) * seg)     # later segments are never attended
+                s = qh[r0:r1].double() @ kf[:n].T
+                s.mul_(1.0 / math.sqrt(D)).masked_fill_(idx[:n] > pos[r0:r1, None], -math.inf)
+                if mask is not None:
+                    s.masked_fill_(~mask[pos[r0:r1] // bs][:, pos[:n] // bs], -math.inf)
+                out[b, h, r0:r1] = torch.softmax(s, dim=-1) @ vf[:n]
+    return out
+
+
+def exact(case, seed):
+    """What run() returns, summed in 64 bits."""
+    if case["batch"] * case["q_heads"] * case["tokens"] ** 2 > _EXACT_MOST:
+        return None
+    st = prepare(case, seed)
+    if case["call"] == "layer":
+        a, x = st["attn"], st["x"].double()
+        B, S, _ = x.shape
+        D, dt = case["head_dim"], st["x"].dtype
+        cos, sin = (t.double()[:, None] for t in st["pos"])
+        rnd = lambda t: t.to(dt).double()
+        heads = lambda lin: rnd(x @ lin.weight.double().T).view(B, S, -1, D).transpose(1, 2)
+        turn = lambda t: torch.cat((-t[..., D // 2:], t[..., :D // 2]), dim=-1)
+        q, k = (rnd(rnd(t * cos) + rnd(turn(t) * sin)).to(dt) for t in (heads(a.q_proj), heads(a.k_proj)))
+        o = rnd(_exact_attention(q, k, heads(a.v_proj).to(dt), case))
+        return o.transpose(1, 2).reshape(B, S, -1) @ a.o_proj.weight.double().T
+    return _exact_attention(*(st[n].cuda() for n in ("q", "k", "v")), case)
