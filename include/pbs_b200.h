@@ -71,7 +71,7 @@ typedef struct {
   int64_t block_mask;    /* uint8   : (B, Hq, nb, nb)                                               */
   int64_t tile_list;     /* uint32  : (B, Hq, ceil(S / 256), ceil(S / 128))                         */
   int64_t tile_count;    /* int32   : (B, Hq, ceil(S / 256))                                        */
-  int64_t status;        /* int32   : 8 words, device-side error flags                              */
+  int64_t status;        /* int32   : 8 words, device-side error flags and work counter             */
 } pbs_scratch_sizes_t;
 
 /* Device pointers of the scratch buffers, sized by pbs_scratch_sizes. */
@@ -225,7 +225,8 @@ int pbs_build_tile_lists(const pbs_shape_t* shape, const uint8_t* block_mask,
  * into the store).  Replaces the launch at pbs_attn/src/pbs.py:220-246 of the kernel
  * pbs_attn/src/kernels/permuted_block_sparse_attention.py:134-311.
  * status: 8 int32 words, zero on entry; word 0 becomes non-zero if a bounded device-side
- * wait ran out (the output is then invalid).  out_replicas: NULL or extra destinations. */
+ * wait ran out (the output is then invalid), word 7 is the tcgen05 kernel's work counter and is zero
+ * again when it returns.  Two launches at once need two sets of words.  out_replicas: NULL or extra destinations. */
 int pbs_attn_fwd(const pbs_shape_t* shape,
                  const void* q, const int64_t q_strides[4],
                  const void* perm_k, const void* perm_v, const int32_t* key_indices,

@@ -7,9 +7,10 @@
 //
 // Work item = 256 consecutive queries of one (b, h): two 128-row query tiles that share every K/V
 // tile staged in shared memory.  The item's tile list (built by tile_list_kernel) names the 128-key
-// tiles that either query tile selected.  A persistent CTA (one per SM) walks its items with
-// twelve warps in four roles:
-//   warp 0      TMA producer: Q tiles, then K and V tiles of the list into two 2-deep rings
+// tiles that either query tile selected.  A persistent CTA (one per SM) draws its items from a queue
+// and walks them with twelve warps in four roles:
+//   warp 0      draws the items and tells the other roles; TMA producer: Q tiles, then K and V tiles of the list
+//               into two 2-deep rings
 //   warps 1, 3  MMA issuers, one per query tile.  A 128-key tile is two half-steps of 64 keys with
 //               their own 64 TMEM columns: S_h = Q K_h^T (SS, both operands K-major, 128B swizzle,
 //               M=128 N=64) and O += P_h V_h (TS: P_h read from TMEM, V MN-major from shared memory)
@@ -38,6 +39,7 @@ namespace {
 constexpr int kThreads = 384;
 constexpr int NK = 2;                     // K ring depth
 constexpr int NV = 2;                     // V ring depth
+constexpr int kSched = 4;                 // items the producer may be ahead of the slowest role
 constexpr uint32_t kTmemCols = 512;
 constexpr float kRescaleThreshold = 8.f;  // log2 units: O is rescaled only when the max grows by more
 
@@ -217,29 +219,8 @@ struct Bars {
   uint64_t k_full[NK], k_empty[NK];
   uint64_t v_full[NV], v_empty[NV];
   uint64_t s_full[2][2], p_full[2][2], o_full[2][2];   // [query tile][key half]
+  uint64_t item_full[kSched], item_empty[kSched];
   uint64_t drain;                                       // teardown after an abort: both issuers' MMAs retired
-};
-
-struct Params {
-  const int32_t* idx;         // (B*Hq, S)
-  const uint32_t* list;       // (B*Hq, G, T)
-  const int32_t* count;       // (B*Hq, G)
-  void* out;
-  Strides os;
-  int Hq, S, G, T, n_items;
-  int bs;
-  float scale_log2e;
-  int32_t* status;
-  void* extra_out[PBS_MAX_OUT_REPLICAS];   // further destinations of the output (same strides), e.g. on peer GPUs
-  int n_extra;
-  unsigned long long wait_ns;   // limit of every device-side wait
-  int drop_arrive;              // diagnostic: CTA 0's first softmax warpgroup skips one arrive (a wait then runs out)
-};
-
-struct Ctl {
-  uint32_t tmem_base;
-  volatile int abort_flag;
-  unsigned long long wait_ns;
 };
 
 // Work order.  Within a head the query groups are taken in the order G-1, 0, G-2, 1, ... and a CTA
@@ -248,16 +229,69 @@ struct Ctl {
 // (a) the CTAs stay balanced without a dynamic queue and (b) all CTAs start their long group at the
 // same time and walk up the head's key range together -- a K/V tile is then fetched from HBM once
 // and served to the other CTAs from L2, instead of every CTA sweeping at its own position.
-// n-th item of this CTA -> position in that order, or -1 past the end.
-__device__ __forceinline__ int item_position(int n, int n_items) {
-  const int pos = 2 * ((int)blockIdx.x + (n >> 1) * (int)gridDim.x) + (n & 1);
-  return pos < n_items ? pos : -1;
+// The pairs rarely fill the last wave of CTAs, a pair is too coarse to share out, and where the selection is sparse
+// the groups of a length differ.  So the work is a queue that CTAs draw from: first the pairs, all but those of
+// the last full wave and what is left over; those are dealt out group by group, the longest of all heads left first.
+// Measured against fixed pairs (this kernel alone, 32 heads): 4 x 2048 tokens 229 -> 208 us, 6001 sparse tokens
+// 253 -> 224, 8192 tokens 533 -> 486 (head_dim 64: 448 -> 384), 32768 sparse tokens 4.25 -> 4.13 ms; with 13 waves or
+// more of equal pairs nothing changes (4 heads of 131072 tokens: 14.3 ms both ways).
+struct Schedule {
+  int n_items, G, BH, pairs;        // pairs: entries of the queue that are pairs
+};
+// Queue entry q, its j-th item (j = 1 only for pairs); false past the end.
+__device__ __forceinline__ bool queue_item(const Schedule& w, int q, int j, int& bh, int& g) {
+  if (q < w.pairs) {
+    const int pos = 2 * q + j, r = pos % w.G;
+    bh = pos / w.G;
+    g = (r & 1) ? (r >> 1) : (w.G - 1 - (r >> 1));
+    return true;
+  }
+  const int first = 2 * w.pairs;                           // positions the pairs have taken
+  int k = q - w.pairs;
+  if (j || k >= w.n_items - first) return false;
+  // the first head left may have lost its longest and its shortest groups to the pairs: [lo, hi] remain
+  const int bh0 = first / w.G, r0 = first % w.G;
+  const int lo = r0 >> 1, hi = w.G - 1 - ((r0 + 1) >> 1);
+  const int whole = w.BH - bh0 - 1;                        // heads after it, with all their groups
+  const int above = (w.G - 1 - hi) * whole, within = (hi - lo + 1) * (whole + 1);
+  if (k < above) {
+    g = w.G - 1 - k / whole;
+    bh = bh0 + 1 + k % whole;
+  } else if ((k -= above) < within) {
+    g = hi - k / (whole + 1);
+    bh = bh0 + k % (whole + 1);
+  } else {
+    k -= within;
+    g = lo - 1 - k / whole;
+    bh = bh0 + 1 + k % whole;
+  }
+  return true;
 }
-__device__ __forceinline__ void item_decode(int pos, int G, int& bh, int& g) {
-  bh = pos / G;
-  const int r = pos % G;
-  g = (r & 1) ? (r >> 1) : (G - 1 - (r >> 1));
-}
+
+struct Params {
+  const int32_t* idx;         // (B*Hq, S)
+  const uint32_t* list;       // (B*Hq, G, T)
+  const int32_t* count;       // (B*Hq, G)
+  void* out;
+  Strides os;
+  int Hq, S, G, T;
+  Schedule work;
+  int bs;
+  float scale_log2e;
+  int32_t* status;
+  int32_t* queue;               // draws so far; zero before and after a launch
+  void* extra_out[PBS_MAX_OUT_REPLICAS];   // further destinations of the output (same strides), e.g. on peer GPUs
+  int n_extra;
+  unsigned long long wait_ns;   // limit of every device-side wait
+  int drop_arrive;              // diagnostic: CTA 0's first softmax warpgroup skips one arrive (a wait then runs out)
+};
+
+struct Ctl {
+  int2 item[kSched];            // (b, h) and query group of the items handed to the other roles; x < 0: no more
+  uint32_t tmem_base;
+  volatile int abort_flag;
+  unsigned long long wait_ns;
+};
 
 // Bounded wait: false when the CTA is aborting (this wait or another one ran out of time).
 __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, Ctl* ctl, int32_t* status, int code) {
@@ -279,6 +313,20 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, Ctl* ctl
 // The same for a whole converged warp: every lane polls, the verdict is made warp-uniform.
 __device__ __forceinline__ bool wait_bar_warp(uint32_t bar, uint32_t parity, Ctl* ctl, int32_t* status, int code) {
   return __all_sync(0xffffffffu, wait_bar(bar, parity, ctl, status, code));
+}
+
+// The n-th item of this CTA, for the roles that the producer feeds (a whole converged warp calls it).
+// False past the last one, or when a wait ran out (then ok is false).
+__device__ __forceinline__ bool next_item(int n, Bars* bars, Ctl* ctl, int32_t* status, bool& ok, int& bh, int& g) {
+  const int s = n % kSched;
+  ok = wait_bar_warp(smem_u32(&bars->item_full[s]), (n / kSched) & 1u, ctl, status, 12);
+  if (!ok) return false;
+  const int2 it = ctl->item[s];
+  __syncwarp();
+  if (elect_one()) mbar_arrive(smem_u32(&bars->item_empty[s]));
+  bh = it.x;
+  g = it.y;
+  return bh >= 0;
 }
 
 template <int D>
@@ -324,6 +372,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     }
     for (int i = 0; i < NK; ++i) { mbar_init(smem_u32(&bars->k_full[i]), 1); mbar_init(smem_u32(&bars->k_empty[i]), 2); }
     for (int i = 0; i < NV; ++i) { mbar_init(smem_u32(&bars->v_full[i]), 1); mbar_init(smem_u32(&bars->v_empty[i]), 2); }
+    for (int i = 0; i < kSched; ++i) { mbar_init(smem_u32(&bars->item_full[i]), 1); mbar_init(smem_u32(&bars->item_empty[i]), 10); }
     mbar_init(smem_u32(&bars->drain), 2);
     ctl->abort_flag = 0;
     ctl->wait_ns = p.wait_ns;
@@ -349,12 +398,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   constexpr uint32_t kIdescPV = (1u << 4) | (kFmt << 7) | (kFmt << 10) | (1u << 16) | (((uint32_t)D >> 3) << 17) | ((128u >> 4) << 24);
 
 
-#if PBS_SETMAXNREG
-  // The softmax warps hold a half-step of S in registers; the four warps of the other roles need few.
-  if (warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PBS_SETMAXNREG));
-  else asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(((64512 - 128 * PBS_SETMAXNREG) / 256) & ~7));
-#endif
-
   if (warp == 0) {
     // =========================================================================== TMA producer
     // The whole warp walks the lists (uniform control flow); one elected lane issues the copies.
@@ -362,9 +405,24 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       uint32_t kc = 0, vc = 0, qc[2] = {0, 0};
       bool ok = true;
       const uint64_t pol_kv = l2_policy_evict_last(), pol_q = l2_policy_evict_first();
-      for (int it = 0, pos; (pos = item_position(it, p.n_items)) >= 0 && ok; ++it) {
-        int bh, g;
-        item_decode(pos, p.G, bh, g);
+      // The items of this CTA: its first queue entry is its own number, each further one is drawn while the entry before
+      // it is loaded.
+      int q = (int)blockIdx.x, q_next = 0, j = 0;
+      for (int it = 0, bh, g; ok; ++it) {
+        const bool more = queue_item(p.work, q, j, bh, g);
+        if (more && j == 0 && elect_one()) {
+          // one draw per entry of the queue; the last one leaves the counter at zero for the next launch
+          const int drawn = atomicAdd(p.queue, 1);
+          if (drawn == p.work.n_items - p.work.pairs - 1) atomicExch(p.queue, 0);
+          q_next = (int)gridDim.x + drawn;
+        }
+        ok = wait_bar_warp(smem_u32(&bars->item_empty[it % kSched]), ((it / kSched) & 1u) ^ 1u, ctl, p.status, 13);
+        if (!ok) break;
+        if (elect_one()) {
+          ctl->item[it % kSched] = more ? make_int2(bh, g) : make_int2(-1, 0);
+          mbar_arrive(smem_u32(&bars->item_full[it % kSched]));
+        }
+        if (!more) break;
         const int b = bh / p.Hq, h = bh % p.Hq;
         for (int i = 0; i < 2 && ok; ++i) {
           const int r0 = g * 256 + i * 128;
@@ -409,6 +467,13 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             }
             ++vc;
           }
+        }
+        if (j == 0 && q < p.work.pairs) {
+          j = 1;
+        } else {
+          j = 0;
+          q = __reduce_max_sync(0xffffffffu, q_next);      // only the elected lane has drawn, the others hold 0
+          q_next = 0;
         }
       }
     }
@@ -456,9 +521,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         tc_commit(bar_ofull[h]);
       };
 
-      for (int it = 0, pos; (pos = item_position(it, p.n_items)) >= 0 && ok; ++it) {
-        int bh, g;
-        item_decode(pos, p.G, bh, g);
+      for (int it = 0, bh, g; ok && next_item(it, bars, ctl, p.status, ok, bh, g); ++it) {
         const int n = p.count[(int64_t)bh * p.G + g];
         const uint32_t* lst = p.list + ((int64_t)bh * p.G + g) * p.T;
         const bool have = g * 256 + i * 128 < p.S;
@@ -542,9 +605,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     uint32_t sc = 0;                                       // list entries done by this warpgroup
     bool ok = true;
 
-    for (int it = 0, pos; (pos = item_position(it, p.n_items)) >= 0 && ok; ++it) {
-      int bh, g;
-      item_decode(pos, p.G, bh, g);
+    for (int it = 0, bh, g; ok && next_item(it, bars, ctl, p.status, ok, bh, g); ++it) {
       const int r0 = g * 256 + i * 128;
       if (r0 >= p.S) continue;
       const int b = bh / p.Hq, h = bh % p.Hq;
@@ -812,7 +873,6 @@ int run_tc(const Dims& d, const void* q, Strides qs, const void* pk, const void*
   Params p;
   p.idx = idx; p.list = list; p.count = count; p.out = out; p.os = os;
   p.Hq = d.Hq; p.S = d.S; p.G = (d.S + 255) / 256; p.T = (d.S + 127) / 128;
-  p.n_items = d.B * d.Hq * p.G;
   p.bs = d.bs;
   p.scale_log2e = (float)(1.4426950408889634 / sqrt((double)d.D));
   p.status = status;
@@ -829,8 +889,11 @@ int run_tc(const Dims& d, const void* q, Strides qs, const void* pk, const void*
   const int smem = Smem<D>::kTotal;
   cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (ce != cudaSuccess) return cuda_fail(ce, "attn_tc_kernel smem attribute");
-  const int pairs = (p.n_items + 1) / 2;
-  const int grid = pairs < sm_count ? pairs : sm_count;
+  p.queue = status + 7;
+  const int items = d.B * d.Hq * p.G;
+  const int grid = items < sm_count ? items : sm_count;
+  const int waves = items / 2 / grid;                      // full waves of pairs
+  p.work = Schedule{items, p.G, d.B * d.Hq, grid * (items == 2 * grid * waves ? waves : (waves > 0 ? waves - 1 : 0))};
   kern<<<grid, kThreads, smem, st>>>(mq, mk, mv, p);
   PBS_CUDA_CHECK_LAUNCH("attn_tc_kernel");
   return PBS_OK;
