@@ -308,6 +308,8 @@ int pbs_attn_fwd(const pbs_shape_t* shape, const void* q, const int64_t q_stride
   if (attn_impl != PBS_ATTN_SIMT && attn_impl != PBS_ATTN_AUTO) { set_error("attn_impl %d unknown", attn_impl); return PBS_ERR_ARG; }
   if (replicated) { set_error("output replicas are written by the tcgen05 attention kernel only; this call runs the generic kernel"); return PBS_ERR_UNSUPPORTED; }
   PBS_NONNULL(block_mask);
+  if (attn_impl == PBS_ATTN_AUTO && attn_fp32_supported(d, shape->dtype))
+    return launch_attn_fp32(d, q, qs, perm_k, perm_v, key_indices, block_mask, out, os, (cudaStream_t)stream);
   return launch_attn_simt(d, shape->dtype, q, qs, perm_k, perm_v, key_indices, block_mask, out, os, (cudaStream_t)stream);
 }
 
@@ -348,7 +350,7 @@ int pbs_prefill_fwd(const pbs_shape_t* shape, const void* q, const int64_t q_str
               "and non-zero batch / head strides of q");
     return PBS_ERR_UNSUPPORTED;
   }
-  if (impl == PBS_ATTN_AUTO) impl = tc_ok ? PBS_ATTN_TCGEN05 : PBS_ATTN_SIMT;
+  if (impl == PBS_ATTN_AUTO && tc_ok) impl = PBS_ATTN_TCGEN05;      // else pbs_attn_fwd picks between the other two
   if (impl == PBS_ATTN_TCGEN05) { PBS_NONNULL(sc->tile_list); PBS_NONNULL(sc->tile_count); }
   PBS_TRY(check_replicas(options->out_replicas, shape->dtype, out_strides));
   if (impl != PBS_ATTN_TCGEN05 && options->out_replicas && options->out_replicas->count > 0) {

@@ -205,6 +205,9 @@ int launch_fill_mask_ones(const Dims& d, uint8_t* mask, cudaStream_t st);
 int launch_build_tile_lists(const Dims& d, const uint8_t* mask, uint32_t* list, int32_t* count, cudaStream_t st);
 int launch_attn_simt(const Dims& d, int dt, const void* q, Strides qs, const void* pk, const void* pv,
                      const int32_t* idx, const uint8_t* mask, void* out, Strides os, cudaStream_t st);
+bool attn_fp32_supported(const Dims& d, int dt);
+int launch_attn_fp32(const Dims& d, const void* q, Strides qs, const void* pk, const void* pv, const int32_t* idx,
+                     const uint8_t* mask, void* out, Strides os, cudaStream_t st);
 bool attn_tc_supported(const Dims& d, int dt);
 void set_attn_wait(unsigned long long wait_ns, int drop_arrive);
 int launch_attn_tc(const Dims& d, int dt, const void* q, Strides qs, const void* pk, const void* pv,

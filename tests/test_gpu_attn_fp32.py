@@ -1,0 +1,36 @@
+"""The register-tiled fp32 attention kernel ("auto") against the generic kernel ("simt") on the same selection."""
+import pytest
+import torch
+
+from pbs_attn_b200.synth import Workload, make_qkv
+
+pytestmark = pytest.mark.gpu
+
+
+# tails of the 32-row query tile and the 64-key step, both head sizes (two buffers / one), both block sizes, one token,
+# the dense fallback, rows that keep nothing ("mean" without the own block) and a strided query tensor
+@pytest.mark.parametrize("tokens,head_dim,block,segment,kind", [
+    (1, 64, 64, 64, "pbs"), (33, 64, 64, 128, "pbs"), (250, 128, 128, 256, "pbs"), (640, 64, 64, 128, "pbs"),
+    (1500, 64, 128, 256, "strided"), (1023, 128, 64, 64, "pbs"), (2047, 128, 128, 512, "strided"),
+    (1500, 64, 64, 64, "mean"), (777, 128, 128, 128, "mean")])
+def test_fp32_kernel_equals_generic_kernel(tokens, head_dim, block, segment, kind):
+    from pbs_attn_b200.prefill import MeanPooling_prefill, permuted_block_sparse_attn_fwd
+    w = Workload("fp32", 2, 4, 2, head_dim, tokens, "fp32", block, segment, 0.7, 5e5, sinks=4)
+    q, k, v = make_qkv(w, seed=tokens, device="cuda")
+    if kind == "strided":
+        q, k, v = (t.transpose(1, 2).contiguous().transpose(1, 2) for t in (q, k, v))
+    got = []
+    for impl in ("auto", "simt"):
+        if kind == "mean":
+            # 2 is never reached: the rows of heads 0 and 2 keep nothing and come out zero
+            thr = torch.tensor([2.0, 0.3, 2.0, 0.6], device="cuda")
+            got.append(MeanPooling_prefill(q, k, v, block, segment, thr, force_select_first_block=False,
+                                           force_select_current_block=False, attn_impl=impl))
+        else:
+            got.append(permuted_block_sparse_attn_fwd(q, k, v, block, segment, 0.7, True, attn_impl=impl))
+    a, b = (t.double() for t in got)
+    if kind == "mean":
+        assert not a[:, ::2].any() and not b[:, ::2].any()
+    # both sum up to 2047 products of unit size in fp32 (2^-24 relative each, in different orders) and take exp2 of the sums
+    assert (a - b).norm() <= 4e-6 * b.norm()
+    assert (a - b).abs().max() <= 2e-5
