@@ -67,9 +67,15 @@ int check_tensor(const char* name, const void* p, const int64_t* st, int dt, Str
 #define PBS_TRY(x) do { int rc__ = (x); if (rc__ != PBS_OK) return rc__; } while (0)
 #define PBS_NONNULL(p) do { if (!(p)) { set_error(#p " is null"); return PBS_ERR_ARG; } } while (0)
 
-// The TMA descriptor of the query tensor cannot describe a broadcast (zero-stride) batch or head dimension.
-bool q_layout_fits_tc(const Dims& d, const Strides& qs) {
-  return (d.Hq == 1 || qs.h > 0) && (d.B == 1 || qs.b > 0);
+// A TMA descriptor cannot describe a broadcast (zero-stride) batch or head dimension.
+bool layout_fits_tc(const Dims& d, int heads, const Strides& st) {
+  return (heads == 1 || st.h > 0) && (d.B == 1 || st.b > 0);
+}
+bool q_layout_fits_tc(const Dims& d, const Strides& qs) { return layout_fits_tc(d, d.Hq, qs); }
+
+KvSource permuted_kv(const Dims& d, const void* perm_k, const void* perm_v) {
+  const Strides st{(int64_t)d.Hq * d.S * d.D, (int64_t)d.S * d.D, d.D};
+  return KvSource{perm_k, perm_v, st, st, 1};
 }
 
 int check_replicas(const pbs_out_replicas_t* r, int dt, const int64_t* out_strides) {
@@ -302,7 +308,7 @@ int pbs_attn_fwd(const pbs_shape_t* shape, const void* q, const int64_t q_stride
   }
   if (attn_impl == PBS_ATTN_TCGEN05 || (attn_impl == PBS_ATTN_AUTO && tc_ok)) {
     PBS_NONNULL(tile_list); PBS_NONNULL(tile_count); PBS_NONNULL(status);
-    return launch_attn_tc(d, shape->dtype, q, qs, perm_k, perm_v, key_indices, tile_list, tile_count, out, os,
+    return launch_attn_tc(d, shape->dtype, q, qs, permuted_kv(d, perm_k, perm_v), key_indices, tile_list, tile_count, out, os,
                           status, out_replicas, (cudaStream_t)stream);
   }
   if (attn_impl != PBS_ATTN_SIMT && attn_impl != PBS_ATTN_AUTO) { set_error("attn_impl %d unknown", attn_impl); return PBS_ERR_ARG; }
@@ -360,23 +366,34 @@ int pbs_prefill_fwd(const pbs_shape_t* shape, const void* q, const int64_t q_str
 
   // ---- enqueue
   cudaStream_t st = (cudaStream_t)stream;
-  cudaError_t e = cudaMemsetAsync(sc->status, 0, 8 * sizeof(int32_t), st);
-  if (e != cudaSuccess) return cuda_fail(e, "clear status");
-  if (dense) {
-    PBS_TRY(pbs_segment_permute(&attn_shape, nullptr, k, k_strides, v, v_strides, sc->key_indices, sc->perm_k,
-                                sc->perm_v, sc->pooled_k, PBS_POOL_MEAN, sc->first_block, stream));
-    PBS_TRY(launch_fill_mask_ones(d, sc->block_mask, st));
+  // Keys in original order need no copy: the tcgen05 kernel reads K and V in place where its descriptors can.
+  const bool identity = dense || options->no_permutation;
+  const bool in_place = identity && impl == PBS_ATTN_TCGEN05 && layout_fits_tc(d, d.Hkv, ks) && layout_fits_tc(d, d.Hkv, vs);
+  if (dense && in_place) {
+    PBS_TRY(launch_dense_setup(d, sc->key_indices, sc->first_block, sc->block_mask, sc->tile_list, sc->tile_count, sc->status, st));
   } else {
-    if (!options->no_permutation)
+    cudaError_t e = cudaMemsetAsync(sc->status, 0, 8 * sizeof(int32_t), st);
+    if (e != cudaSuccess) return cuda_fail(e, "clear status");
+    if (!identity)
       PBS_TRY(pbs_key_importance(shape, q, q_strides, k, k_strides, sc->logits, sc->partials, sc->rowstats,
                                  sc->importance, stream));
-    PBS_TRY(pbs_segment_permute(shape, options->no_permutation ? nullptr : sc->importance, k, k_strides, v, v_strides, sc->key_indices, sc->perm_k,
-                                sc->perm_v, sc->pooled_k, options->key_pool_mode, sc->first_block, stream));
-    PBS_TRY(pbs_pool_queries(shape, q, q_strides, sc->pooled_q, options->query_pool_mode, stream));
-    PBS_TRY(pbs_select_blocks(shape, sc->pooled_q, sc->pooled_k, sc->first_block, options, sc->block_mask, nullptr, stream));
+    Dims order = d;
+    if (identity) { order.nseg = 0; order.L = 0; }
+    PBS_TRY(launch_segment_permute(order, shape->dtype, identity ? nullptr : sc->importance, k, ks, v, vs, sc->key_indices,
+                                   in_place ? nullptr : sc->perm_k, in_place ? nullptr : sc->perm_v, sc->pooled_k,
+                                   dense ? PBS_POOL_MEAN : options->key_pool_mode, sc->first_block, st));
+    if (dense) {
+      PBS_TRY(launch_fill_mask_ones(d, sc->block_mask, st));
+    } else {
+      PBS_TRY(pbs_pool_queries(shape, q, q_strides, sc->pooled_q, options->query_pool_mode, stream));
+      PBS_TRY(pbs_select_blocks(shape, sc->pooled_q, sc->pooled_k, sc->first_block, options, sc->block_mask, nullptr, stream));
+    }
+    if (impl == PBS_ATTN_TCGEN05)
+      PBS_TRY(pbs_build_tile_lists(&attn_shape, sc->block_mask, sc->tile_list, sc->tile_count, stream));
   }
-  if (impl == PBS_ATTN_TCGEN05)
-    PBS_TRY(pbs_build_tile_lists(&attn_shape, sc->block_mask, sc->tile_list, sc->tile_count, stream));
+  if (in_place)
+    return launch_attn_tc(d, shape->dtype, q, qs, KvSource{k, v, ks, vs, d.group}, nullptr, sc->tile_list, sc->tile_count, out, os,
+                          sc->status, options->out_replicas, st);
   return pbs_attn_fwd(&attn_shape, q, q_strides, sc->perm_k, sc->perm_v, sc->key_indices, sc->block_mask,
                       sc->tile_list, sc->tile_count, out, out_strides, impl, sc->status, options->out_replicas, stream);
 }

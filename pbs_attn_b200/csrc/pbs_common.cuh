@@ -193,6 +193,8 @@ int launch_key_importance(const Dims& d, int dt, const void* q, Strides qs, cons
 int launch_segment_permute(const Dims& d, int dt, const float* importance, const void* k, Strides ks,
                            const void* v, Strides vs, int32_t* idx, void* perm_k, void* perm_v,
                            void* pooled_k, int pool_mode, int32_t* first_block, cudaStream_t st);
+int launch_dense_setup(const Dims& d, int32_t* idx, int32_t* first_block, uint8_t* mask, uint32_t* list, int32_t* count,
+                       int32_t* status, cudaStream_t st);
 int launch_pool_queries(const Dims& d, int dt, const void* q, Strides qs, void* pooled_q, int pool_mode,
                         cudaStream_t st);
 int launch_rope(int dt, int B, int H, int S, int D, void* x, Strides xs, const void* cosp, const void* sinp,
@@ -210,8 +212,15 @@ int launch_attn_fp32(const Dims& d, const void* q, Strides qs, const void* pk, c
                      const uint8_t* mask, void* out, Strides os, cudaStream_t st);
 bool attn_tc_supported(const Dims& d, int dt);
 void set_attn_wait(unsigned long long wait_ns, int drop_arrive);
-int launch_attn_tc(const Dims& d, int dt, const void* q, Strides qs, const void* pk, const void* pv,
-                   const int32_t* idx, const uint32_t* list, const int32_t* count, void* out, Strides os,
-                   int32_t* status, const pbs_out_replicas_t* replicas, cudaStream_t st);
+// Keys and values as the attention reads them: (B, Hq / group, S, D) with any strides, query head h uses head h / group.
+struct KvSource {
+  const void* k;
+  const void* v;
+  Strides ks, vs;
+  int group;
+};
+int launch_attn_tc(const Dims& d, int dt, const void* q, Strides qs, const KvSource& kv, const int32_t* idx,
+                   const uint32_t* list, const int32_t* count, void* out, Strides os, int32_t* status,
+                   const pbs_out_replicas_t* replicas, cudaStream_t st);
 
 }  // namespace pbs

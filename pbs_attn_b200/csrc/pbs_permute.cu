@@ -72,9 +72,9 @@ segment_permute_kernel(const float* __restrict__ importance,
   const int c = threadIdx.x % cpr;
   const T* kb = k + (int64_t)b * ks.b + (int64_t)(h / group) * ks.h;
   const T* vb = v + (int64_t)b * vs.b + (int64_t)(h / group) * vs.h;
-  T* pk = perm_k + ((int64_t)bh * S + seg0) * D;
-  T* pv = perm_v + ((int64_t)bh * S + seg0) * D;
-  if (threadIdx.x < rows_per_pass * cpr) {
+  if (perm_k && threadIdx.x < rows_per_pass * cpr) {       // null: the attention reads K and V where they are
+    T* pk = perm_k + ((int64_t)bh * S + seg0) * D;
+    T* pv = perm_v + ((int64_t)bh * S + seg0) * D;
     for (int i = threadIdx.x / cpr; i < n; i += rows_per_pass) {
       const int src = order[i];
       const uint4 kq = *reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(kb + (int64_t)src * ks.s) + c * 16);

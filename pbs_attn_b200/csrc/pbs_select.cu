@@ -492,6 +492,32 @@ tile_list_kernel(const uint8_t* __restrict__ mask, uint32_t* __restrict__ list, 
   if (threadIdx.x == 0) count[(int64_t)bh * ngroups + g] = wbase;
 }
 
+// Everything the attention kernel needs for plain causal attention over keys in original order: identity order, all
+// blocks on, and the tile lists.  Key tiles above the diagonal are left out of the lists and only the diagonal one is
+// masked by element (with block_size 64 all four sub-blocks are on).  One CTA per (b, h); a few hundred bytes each, so
+// the launch is what it costs: it takes the place of three (gather of K and V, mask, lists) and of the copy of K and V.
+__global__ void __launch_bounds__(128)
+dense_setup_kernel(int32_t* __restrict__ idx, int32_t* __restrict__ first_block, uint8_t* __restrict__ mask,
+                   uint32_t* __restrict__ list, int32_t* __restrict__ count, int32_t* __restrict__ status, int S, int bs, int nb) {
+  const int bh = blockIdx.x;
+  const int ngroups = (S + 255) / 256, ntiles = (S + 127) / 128;
+  if (bh == 0 && threadIdx.x < 8) status[threadIdx.x] = 0;
+  if (threadIdx.x == 0) first_block[bh] = 0;
+  for (int i = threadIdx.x; i < S; i += blockDim.x) idx[(int64_t)bh * S + i] = i;
+  for (int i = threadIdx.x; i < nb * nb; i += blockDim.x) mask[(int64_t)bh * nb * nb + i] = 1;
+  const uint32_t bits = bs == 64 ? 0xFu : 1u;
+  for (int i = threadIdx.x; i < ngroups * ntiles; i += blockDim.x) {
+    const int g = i / ntiles, t = i % ntiles;
+    uint32_t e = 0;
+    for (int m = 0; m < 2; ++m) {
+      const int qt = 2 * g + m;
+      if (qt < ntiles && t <= qt) e |= (1u << (16 + m)) | (bits << (20 + 4 * m)) | (t == qt ? 1u << (18 + m) : 0u);
+    }
+    if (e) list[((int64_t)bh * ngroups + g) * ntiles + t] = e | (uint32_t)t;
+    if (t == 0) count[(int64_t)bh * ngroups + g] = min(2 * g + 2, ntiles);
+  }
+}
+
 template <int DT, int CPR, int KPT>
 int run_select_tiled(const Dims& d, const void* pooled_q, const void* pooled_k, const int32_t* first_block,
                      const pbs_options_t& opt, uint8_t* mask, float* scores, cudaStream_t st) {
@@ -598,6 +624,13 @@ int launch_fill_mask_ones(const Dims& d, uint8_t* mask, cudaStream_t st) {
   const int64_t n = (int64_t)d.B * d.Hq * d.nb * d.nb;
   fill_ones_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(mask, n);
   PBS_CUDA_CHECK_LAUNCH("fill_ones_kernel");
+  return PBS_OK;
+}
+
+int launch_dense_setup(const Dims& d, int32_t* idx, int32_t* first_block, uint8_t* mask, uint32_t* list, int32_t* count,
+                       int32_t* status, cudaStream_t st) {
+  dense_setup_kernel<<<d.B * d.Hq, 128, 0, st>>>(idx, first_block, mask, list, count, status, d.S, d.bs, d.nb);
+  PBS_CUDA_CHECK_LAUNCH("dense_setup_kernel");
   return PBS_OK;
 }
 
