@@ -198,7 +198,7 @@ select_kernel(const typename Elem<DT>::T* __restrict__ pooled_q, const typename 
 
 
 // ---------------------------------------------------------------------------------------------
-// Tiled variant: one CTA = 16 consecutive q blocks of one (b, h).
+// Tiled variant: one CTA = 16 (or 8) consecutive q blocks of one (b, h).
 //
 // Phase A computes the pooled logits of the 16 rows against 64-kv-block chunks of pooled K that
 // arrive in shared memory by cp.async (each pooled-K row is then read once per 16 rows instead of
@@ -211,7 +211,6 @@ select_kernel(const typename Elem<DT>::T* __restrict__ pooled_q, const typename 
 // equal to it are added in kv-block order until the running sum reaches the threshold -- the set a
 // stable descending sort followed by a running sum selects.
 // ---------------------------------------------------------------------------------------------
-constexpr int TS_ROWS = 16;       // q blocks per CTA
 constexpr int TS_CHUNK = 64;      // kv blocks per staged chunk
 
 template <int N>
@@ -230,8 +229,9 @@ __device__ __forceinline__ double warp_sum_double(double v) {
   return v;
 }
 
-// CPR: 16-byte pieces per pooled row; KPT: kv blocks per lane held in registers (32 * KPT >= nb)
-template <int DT, int CPR, int KPT>
+// CPR: 16-byte pieces per pooled row; KPT: kv blocks per lane held in registers (32 * KPT >= nb); TS_ROWS: q blocks
+// per CTA (16 or 8)
+template <int DT, int CPR, int KPT, int TS_ROWS>
 __global__ void __launch_bounds__(256)
 select_tiled_kernel(const typename Elem<DT>::T* __restrict__ pooled_q, const typename Elem<DT>::T* __restrict__ pooled_k,
                     const int32_t* __restrict__ first_block, const float* __restrict__ thr_per_head, float thr_scalar,
@@ -274,8 +274,9 @@ select_tiled_kernel(const typename Elem<DT>::T* __restrict__ pooled_q, const typ
     Qs[i] = qb0 + r < nb ? E::ld(pooled_q + ((int64_t)bh * nb + qb0 + r) * D + d) : 0.f;
   }
 
-  // ---- phase A: logits.  Thread = (row, kv lane): row t / 16, kv blocks t % 16 + 16 a of the chunk.
-  const int arow = threadIdx.x >> 4, aj0 = threadIdx.x & 15;
+  // ---- phase A: logits.  Thread = (row, kv lane): kv blocks lane + LPR a of the chunk.
+  constexpr int LPR = 256 / TS_ROWS;
+  const int arow = threadIdx.x / LPR, aj0 = threadIdx.x % LPR;
   for (int c = 0; c < nchunks; ++c) {
     if (c + 1 < nchunks) {
       load_chunk((c + 1) & 1, c + 1);
@@ -287,8 +288,8 @@ select_tiled_kernel(const typename Elem<DT>::T* __restrict__ pooled_q, const typ
     const T* Kt = Kc + (c & 1) * TS_CHUNK * LDK;
     const float* qr = Qs + arow * D;
 #pragma unroll
-    for (int a = 0; a < TS_CHUNK / 16; ++a) {
-      const int j = aj0 + 16 * a;
+    for (int a = 0; a < TS_CHUNK / LPR; ++a) {
+      const int j = aj0 + LPR * a;
       const int kb = c * TS_CHUNK + j;
       if (kb >= ncmax) continue;
       float piece[CPR];
@@ -370,20 +371,36 @@ select_tiled_kernel(const typename Elem<DT>::T* __restrict__ pooled_q, const typ
         if (k < kmax) tot += (double)pv[k];
       tot = warp_sum_double(tot);
       if ((float)tot >= thr) {
-        // cut = largest probability value v with (float) sum{p >= v} >= thr (bit pattern order)
+        // cut = largest probability value v with (float) sum{p >= v} >= thr (bit pattern order).  All values share
+        // the bits above the highest one in which the smallest and the largest differ; from there two bits are
+        // fixed at a time, the three trial sums of a step being independent of one another: a step is a chain of
+        // shuffles, and twice as many single-bit steps took twice as long.
         const uint32_t umax = __float_as_uint(pmax);
         uint32_t cut = umax;
         if (thr > 0.f && umax != 0u) {
-          cut = 0u;
-          for (int b = 31 - __clz(umax); b >= 0; --b) {
-            const uint32_t cand = cut | (1u << b);
-            if (cand > umax) continue;
-            double g = 0.0;
+          uint32_t umin = umax;
 #pragma unroll
-            for (int k = 0; k < KPT; ++k)
-              if (k < kmax && __float_as_uint(pv[k]) >= cand) g += (double)pv[k];
-            g = warp_sum_double(g);
-            if ((float)g >= thr) cut = cand;
+          for (int k = 0; k < KPT; ++k)
+            if (k < kmax && 32 * k + lane < ncand) umin = min(umin, __float_as_uint(pv[k]));
+          umin = __reduce_min_sync(0xffffffffu, umin);
+          int b = umax == umin ? 0 : 32 - __clz(umax ^ umin);    // bits to fix
+          b += b & 1;
+          cut = b >= 32 ? 0u : umax & ~((1u << b) - 1u);
+          while (b > 0) {
+            b -= 2;
+            double g[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+            for (int k = 0; k < KPT; ++k) {
+              if (k < kmax) {
+                const uint32_t u = __float_as_uint(pv[k]);
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                  if (u >= (cut | ((uint32_t)(c + 1) << b))) g[c] += (double)pv[k];
+              }
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) g[c] = warp_sum_double(g[c]);
+            cut |= ((float)g[2] >= thr ? 3u : (float)g[1] >= thr ? 2u : (float)g[0] >= thr ? 1u : 0u) << b;
           }
         }
         // everything above the cut; then the blocks equal to it, in kv-block order, until reached
@@ -518,20 +535,20 @@ dense_setup_kernel(int32_t* __restrict__ idx, int32_t* __restrict__ first_block,
   }
 }
 
-template <int DT, int CPR, int KPT>
+template <int DT, int CPR, int KPT, int ROWS>
 int run_select_tiled(const Dims& d, const void* pooled_q, const void* pooled_k, const int32_t* first_block,
                      const pbs_options_t& opt, uint8_t* mask, float* scores, cudaStream_t st) {
   using T = typename Elem<DT>::T;
   constexpr int EPV = 16 / (int)sizeof(T);
   const int ncpad = ((d.nb + TS_CHUNK - 1) / TS_CHUNK) * TS_CHUNK;
-  const size_t smem = (size_t)TS_ROWS * d.D * sizeof(float) + (size_t)2 * TS_CHUNK * (d.D + EPV) * sizeof(T) +
-                      (size_t)TS_ROWS * ncpad * sizeof(T);
-  auto kern = select_tiled_kernel<DT, CPR, KPT>;
+  const size_t smem = (size_t)ROWS * d.D * sizeof(float) + (size_t)2 * TS_CHUNK * (d.D + EPV) * sizeof(T) +
+                      (size_t)ROWS * ncpad * sizeof(T);
+  auto kern = select_tiled_kernel<DT, CPR, KPT, ROWS>;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_fail(e, "select_tiled_kernel smem attribute");
   }
-  kern<<<dim3((d.nb + TS_ROWS - 1) / TS_ROWS, d.B * d.Hq), 256, smem, st>>>(
+  kern<<<dim3((d.nb + ROWS - 1) / ROWS, d.B * d.Hq), 256, smem, st>>>(
       (const T*)pooled_q, (const T*)pooled_k, first_block, opt.threshold_per_head, opt.threshold, opt.select_all,
       opt.force_select_first_block, opt.diagonal_candidates, opt.no_own_segment ? 0 : 1, mask, scores, d.Hq, d.nb, d.bps,
       (float)sqrt((double)d.D), ncpad);
@@ -539,13 +556,20 @@ int run_select_tiled(const Dims& d, const void* pooled_q, const void* pooled_k, 
   return PBS_OK;
 }
 
+// 16 rows a CTA read pooled K half as often as 8, but a warp then works off two rows one after the other.  As long as
+// all CTAs of 8 rows are resident at once (three a SM, 148 SMs) the second row is pure latency: with the two-bit steps of
+// the search, 128 heads x 16 blocks 26 -> 16 us; beyond that line (32 heads x 128 blocks of 64) 16 rows stay as fast.
 template <int DT, int CPR>
 int run_select_tiled_k(const Dims& d, const void* pooled_q, const void* pooled_k, const int32_t* first_block,
                        const pbs_options_t& opt, uint8_t* mask, float* scores, cudaStream_t st) {
-  if (d.nb <= 256) return run_select_tiled<DT, CPR, 8>(d, pooled_q, pooled_k, first_block, opt, mask, scores, st);
-  if (d.nb <= 512) return run_select_tiled<DT, CPR, 16>(d, pooled_q, pooled_k, first_block, opt, mask, scores, st);
-  if (d.nb <= 1024) return run_select_tiled<DT, CPR, 32>(d, pooled_q, pooled_k, first_block, opt, mask, scores, st);
-  return run_select_tiled<DT, CPR, 64>(d, pooled_q, pooled_k, first_block, opt, mask, scores, st);
+  if (d.nb <= 256) {
+    if ((int64_t)((d.nb + 7) / 8) * d.B * d.Hq <= 3 * 148)
+      return run_select_tiled<DT, CPR, 8, 8>(d, pooled_q, pooled_k, first_block, opt, mask, scores, st);
+    return run_select_tiled<DT, CPR, 8, 16>(d, pooled_q, pooled_k, first_block, opt, mask, scores, st);
+  }
+  if (d.nb <= 512) return run_select_tiled<DT, CPR, 16, 16>(d, pooled_q, pooled_k, first_block, opt, mask, scores, st);
+  if (d.nb <= 1024) return run_select_tiled<DT, CPR, 32, 16>(d, pooled_q, pooled_k, first_block, opt, mask, scores, st);
+  return run_select_tiled<DT, CPR, 64, 16>(d, pooled_q, pooled_k, first_block, opt, mask, scores, st);
 }
 
 // The tiled kernel covers pooled rows of 8, 16 or 32 16-byte pieces and up to 2048 blocks per row.
