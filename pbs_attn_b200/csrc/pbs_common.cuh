@@ -60,24 +60,6 @@ static inline Dims make_dims(const pbs_shape_t& s) {
   return d;
 }
 
-// Sum in the order of the CPU reduction the reference's means go through: items are added
-// sequentially into a level-0 accumulator that is flushed into level 1 every 16 items, level 1
-// into level 2 every 256, and the levels are added up at the end.  Keeping the same order keeps
-// pooled means bit-identical to the reference's.
-struct CascadeSum {
-  float a0 = 0.f, a1 = 0.f, a2 = 0.f;
-  int n = 0;
-  __device__ __forceinline__ void add(float x) {
-    a0 += x;
-    ++n;
-    if ((n & 15) == 0) {
-      a1 += a0; a0 = 0.f;
-      if ((n & 255) == 0) { a2 += a1; a1 = 0.f; }
-    }
-  }
-  __device__ __forceinline__ float total() const { return (a0 + a1) + a2; }
-};
-
 // Monotone map float -> uint32 (larger float = larger key); NaN sorts above +inf like torch.sort.
 __device__ __forceinline__ uint32_t float_order_key(float x) {
   if (x != x) return 0xFFFFFFFFu;

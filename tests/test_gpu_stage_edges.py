@@ -49,3 +49,17 @@ def test_selection_equals_the_general_kernel(heads, nb, thr):
     finally:
         lib.pbs_debug_set_select_impl(0)
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("block", [16, 48, 96, 128, 240, 256])
+@pytest.mark.parametrize("dtype,D", [("bf16", 128), ("fp16", 8), ("fp32", 64), ("fp32", 256)])
+@pytest.mark.parametrize("mode", ["mean", "max"])
+def test_pooled_keys_equal_the_reference_order(block, dtype, D, mode):
+    from pbs_attn_b200.prefill import Plan
+    S, segment = 3 * 4 * block + block + 5, 4 * block
+    q, k, v = _inputs(dtype, 2, D, S, block, segment)
+    plan = Plan(1, 2, 1, S, D, block, segment, q.dtype, q.device)
+    plan.segment_permute(k, v, mode, identity=True)
+    want = pbs_oracle._pool(pbs_oracle._pad_to_block(pbs_oracle.repeat_kv(k.cpu(), 2), block), block, mode)
+    assert torch.equal(plan.perm_k.cpu(), pbs_oracle.repeat_kv(k.cpu(), 2)) and torch.equal(plan.perm_v.cpu(), pbs_oracle.repeat_kv(v.cpu(), 2))
+    assert torch.equal(plan.pooled_k.cpu(), want)
