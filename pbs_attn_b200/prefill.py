@@ -30,12 +30,12 @@ def _strides(t: torch.Tensor):
 def _readable(t: torch.Tensor, need_distinct_heads: bool = False) -> torch.Tensor:
     """Returns ``t`` if the kernels can read it in place (unit head-dim stride, 16-byte aligned
     rows), else a contiguous copy."""
-    e = t.element_size()
-    ok = (t.stride(3) == 1 and t.data_ptr() % 16 == 0 and t.stride(2) > 0
-          and all((s * e) % 16 == 0 and s >= 0 for s in t.stride()[:3]))
+    sb, sh, ss, sd = t.stride()
+    # the row pieces are 16 bytes, a power of two of elements: one test of the strides' common low bits covers all three
+    ok = sd == 1 and ss > 0 and sb >= 0 and sh >= 0 and ((sb | sh | ss) * t.element_size()) % 16 == 0 and t.data_ptr() % 16 == 0
     if ok and need_distinct_heads:
         # the TMA descriptor of the query tensor cannot describe broadcast (stride-0) batch / head dims
-        ok = all(st > 0 or n == 1 for st, n in zip(t.stride()[:2], t.shape[:2]))
+        ok = (sb > 0 or t.shape[0] == 1) and (sh > 0 or t.shape[1] == 1)
     return t if ok else t.contiguous()
 
 
@@ -93,6 +93,8 @@ class Plan:
         self._status_pending = []          # [(event, slot)], oldest first
         self._status_next = 0
 
+    _status_rows = _status_words = None     # views of the ring, made on first use: per-slot tensors and a numpy array
+
     # ------------------------------------------------------------------ helpers
     def _stream(self):
         return C.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
@@ -113,17 +115,18 @@ class Plan:
             elif not ev.query():
                 break
             self._status_pending.pop(0)
-            words = self._status_ring[slot].tolist()
-            if words[0] != 0:
+            if self._status_words[slot, 0] != 0:
                 self._status_pending.clear()
-                self._raise_status(words)
+                self._raise_status(self._status_words[slot].tolist())
 
-    def _queue_status_copy(self):
+    def _queue_status_copy(self, stream):
+        if self._status_rows is None:
+            self._status_rows, self._status_words = self._status_ring.unbind(0), self._status_ring.numpy()
         slot = self._status_next
         self._status_next = (slot + 1) % _STATUS_SLOTS
-        self._status_ring[slot].copy_(self.status, non_blocking=True)
+        self._status_rows[slot].copy_(self.status, non_blocking=True)
         ev = torch.cuda.Event()
-        ev.record(torch.cuda.current_stream(self.device))
+        ev.record(stream)
         self._status_pending.append((ev, slot))
 
     def options(self, threshold, force_select_first_block=True, query_pool_mode="mean", key_pool_mode="mean",
@@ -215,12 +218,14 @@ class Plan:
     def run(self, q, k, v, out, opt: _cabi.Options):
         """The whole path.  Never synchronises: a device-side error of an EARLIER call (its status words
         have reached the host by now) is raised here; this call's own status is queued for the next."""
-        self._inspect_landed_status()
+        if self._status_pending:
+            self._inspect_landed_status()
         with self._on_device():
+            stream = torch.cuda.current_stream(self.device)
             _cabi.check(self.lib.pbs_prefill_fwd(C.byref(self.shape), _ptr(q), _strides(q), _ptr(k), _strides(k),
                                                  _ptr(v), _strides(v), _ptr(out), _strides(out), C.byref(opt),
-                                                 C.byref(self.scratch), self._stream()), "pbs_prefill_fwd")
-            self._queue_status_copy()
+                                                 C.byref(self.scratch), C.c_void_p(stream.cuda_stream)), "pbs_prefill_fwd")
+            self._queue_status_copy(stream)
         return out
 
 
