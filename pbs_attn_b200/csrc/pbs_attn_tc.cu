@@ -9,8 +9,6 @@
 // tile staged in shared memory.  The item's tile list (built by tile_list_kernel) names the 128-key
 // tiles that either query tile selected.  A persistent CTA (one per SM) draws its items from a queue
 // and walks them with twelve warps in four roles:
-// K and V come through tensor maps of any strides with the query heads of a group on one head, so a call whose keys keep
-// their order needs no copy of them (a copy costs 97 us of 1.6 ms at 16384 tokens, and 19 of 57 us below one segment).
 //   warp 0      draws the items and tells the other roles; TMA producer: Q tiles, then K and V tiles of the list
 //               into two 2-deep rings
 //   warps 1, 3  MMA issuers, one per query tile.  A 128-key tile is two half-steps of 64 keys with
@@ -22,6 +20,8 @@
 //               row that outgrew the lazy-rescale threshold makes the warp rescale O in TMEM and start
 //               over), row sum, P_h written back over the first 32 columns of S_h as packed 16-bit
 //               pairs; final O / l epilogue to global through a per-warp transposition tile
+// K and V come through tensor maps of any strides with the query heads of a group on one head, so a call whose keys keep
+// their order needs no copy of them (a copy costs 97 us of 1.6 ms at 16384 tokens, and 19 of 57 us below one segment).
 // An issuer runs, per list entry and half h: O += P_h V_h, then S_h of the next entry into the
 // columns P_h vacated.  So while a softmax warpgroup works on one half, the MMAs of the other half
 // (and of the other query tile) run, and the next S is ready when the warpgroup comes back for it.
