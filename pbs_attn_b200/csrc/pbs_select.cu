@@ -372,9 +372,11 @@ select_tiled_kernel(const typename Elem<DT>::T* __restrict__ pooled_q, const typ
       tot = warp_sum_double(tot);
       if ((float)tot >= thr) {
         // cut = largest probability value v with (float) sum{p >= v} >= thr (bit pattern order).  All values share
-        // the bits above the highest one in which the smallest and the largest differ; from there two bits are
-        // fixed at a time, the three trial sums of a step being independent of one another: a step is a chain of
-        // shuffles, and twice as many single-bit steps took twice as long.
+        // the bits above the highest one in which the smallest and the largest differ.  From there a short row fixes two
+        // bits at a time, the three trial sums of a step being independent of one another: a step is a chain of
+        // shuffles, and twice as many single-bit steps took twice as long.  With more than 8 values a lane the sums
+        // themselves cost more than the chain (1024 blocks: 0.75 ms before, 0.89 with two bits, 0.73 with one).
+        constexpr int BITS = KPT <= 8 ? 2 : 1;
         const uint32_t umax = __float_as_uint(pmax);
         uint32_t cut = umax;
         if (thr > 0.f && umax != 0u) {
@@ -384,23 +386,28 @@ select_tiled_kernel(const typename Elem<DT>::T* __restrict__ pooled_q, const typ
             if (k < kmax && 32 * k + lane < ncand) umin = min(umin, __float_as_uint(pv[k]));
           umin = __reduce_min_sync(0xffffffffu, umin);
           int b = umax == umin ? 0 : 32 - __clz(umax ^ umin);    // bits to fix
-          b += b & 1;
+          if (b % BITS) ++b;
           cut = b >= 32 ? 0u : umax & ~((1u << b) - 1u);
           while (b > 0) {
-            b -= 2;
-            double g[3] = {0.0, 0.0, 0.0};
+            b -= BITS;
+            constexpr int TRIALS = (1 << BITS) - 1;
+            double g[TRIALS];
+#pragma unroll
+            for (int c = 0; c < TRIALS; ++c) g[c] = 0.0;
 #pragma unroll
             for (int k = 0; k < KPT; ++k) {
               if (k < kmax) {
                 const uint32_t u = __float_as_uint(pv[k]);
 #pragma unroll
-                for (int c = 0; c < 3; ++c)
+                for (int c = 0; c < TRIALS; ++c)
                   if (u >= (cut | ((uint32_t)(c + 1) << b))) g[c] += (double)pv[k];
               }
             }
+            uint32_t digit = 0u;                           // the trial sums fall with the digit
 #pragma unroll
-            for (int c = 0; c < 3; ++c) g[c] = warp_sum_double(g[c]);
-            cut |= ((float)g[2] >= thr ? 3u : (float)g[1] >= thr ? 2u : (float)g[0] >= thr ? 1u : 0u) << b;
+            for (int c = 0; c < TRIALS; ++c)
+              if ((float)warp_sum_double(g[c]) >= thr) digit = c + 1;
+            cut |= digit << b;
           }
         }
         // everything above the cut; then the blocks equal to it, in kv-block order, until reached
