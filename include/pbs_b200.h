@@ -253,7 +253,8 @@ int pbs_ipc_release(void* base_ptr);
 int pbs_enable_peer_access(int32_t peer_device);
 
 /* Whole path: stages 1a..3b in order on one stream.  For S <= segment_size it runs dense
- * causal attention like the reference (pbs_attn/src/pbs.py:175-182).
+ * causal attention like the reference (pbs_attn/src/pbs.py:175-182).  out and its replicas may share
+ * memory with k and v: they are copied before the attention starts wherever they overlap.
  * Replaces permuted_block_sparse_attn_fwd, pbs_attn/src/pbs.py:132-257. */
 int pbs_prefill_fwd(const pbs_shape_t* shape,
                     const void* q, const int64_t q_strides[4],

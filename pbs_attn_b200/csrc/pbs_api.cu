@@ -73,6 +73,29 @@ bool layout_fits_tc(const Dims& d, int heads, const Strides& st) {
 }
 bool q_layout_fits_tc(const Dims& d, const Strides& qs) { return layout_fits_tc(d, d.Hq, qs); }
 
+// The bytes from the first to the last element of a (B, heads, S, D) tensor.
+struct Extent {
+  uintptr_t lo, hi;
+  bool meets(const Extent& o) const { return lo < o.hi && o.lo < hi; }
+};
+Extent extent(const Dims& d, int heads, int dt, const void* p, const Strides& st) {
+  const int64_t last = (int64_t)(d.B - 1) * st.b + (int64_t)(heads - 1) * st.h + (int64_t)(d.S - 1) * st.s + d.D;
+  return Extent{(uintptr_t)p, (uintptr_t)p + (uintptr_t)(last * elem_bytes(dt))};
+}
+
+// May the attention write into K or V (or a tensor woven into them)?  Its CTAs store rows of the result while others still
+// load keys and values, so such a call has to go through the copies of K and V.
+bool output_meets_kv(const Dims& d, int dt, const void* out, const Strides& os, const pbs_out_replicas_t* r, const void* k,
+                     const Strides& ks, const void* v, const Strides& vs) {
+  const Extent ke = extent(d, d.Hkv, dt, k, ks), ve = extent(d, d.Hkv, dt, v, vs);
+  const int copies = r ? r->count : 0;
+  for (int i = -1; i < copies; ++i) {
+    const Extent oe = extent(d, d.Hq, dt, i < 0 ? out : r->out[i], os);
+    if (oe.meets(ke) || oe.meets(ve)) return true;
+  }
+  return false;
+}
+
 KvSource permuted_kv(const Dims& d, const void* perm_k, const void* perm_v) {
   const Strides st{(int64_t)d.Hq * d.S * d.D, (int64_t)d.S * d.D, d.D};
   return KvSource{perm_k, perm_v, st, st, 1};
@@ -366,9 +389,11 @@ int pbs_prefill_fwd(const pbs_shape_t* shape, const void* q, const int64_t q_str
 
   // ---- enqueue
   cudaStream_t st = (cudaStream_t)stream;
-  // Keys in original order need no copy: the tcgen05 kernel reads K and V in place where its descriptors can.
+  // Keys in original order need no copy: the tcgen05 kernel reads K and V in place where its descriptors can and the
+  // result goes elsewhere.
   const bool identity = dense || options->no_permutation;
-  const bool in_place = identity && impl == PBS_ATTN_TCGEN05 && layout_fits_tc(d, d.Hkv, ks) && layout_fits_tc(d, d.Hkv, vs);
+  const bool in_place = identity && impl == PBS_ATTN_TCGEN05 && layout_fits_tc(d, d.Hkv, ks) && layout_fits_tc(d, d.Hkv, vs) &&
+                        !output_meets_kv(d, shape->dtype, out, os, options->out_replicas, k, ks, v, vs);
   if (dense && in_place) {
     PBS_TRY(launch_dense_setup(d, sc->key_indices, sc->first_block, sc->block_mask, sc->tile_list, sc->tile_count, sc->status, st));
   } else {

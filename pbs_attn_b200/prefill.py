@@ -319,7 +319,8 @@ def permuted_block_sparse_attn_fwd(
       * ``intermediates``: a dict that receives the permutation, block mask and plan
         (used by the parity tests);
       * ``out``: a preallocated result tensor of q's shape and dtype (any strides the kernels can
-        write: unit head-dim stride, 16-byte aligned rows), e.g. a head slice of a larger tensor;
+        write: unit head-dim stride, 16-byte aligned rows), e.g. a head slice of a larger tensor; it may
+        share memory with key_states or value_states;
       * ``out_replicas``: further destinations with ``out``'s strides that the attention kernel
         writes as well (buffers on peer GPUs of a head-sharded call, see ``peer_gather``).
     Runs on the current CUDA stream without synchronising.

@@ -5,6 +5,7 @@ import os
 import re
 
 import pytest
+import torch
 
 from pbs_attn_b200 import _cabi
 
@@ -85,7 +86,6 @@ def test_null_and_layout_arguments_are_rejected_before_any_launch(lib):
 
 
 def test_cpu_tensors_are_refused():
-    import torch
     from pbs_attn_b200.prefill import permuted_block_sparse_attn_fwd
     q = torch.zeros(1, 2, 512, 64)
     with pytest.raises(RuntimeError, match="CUDA"):
@@ -156,3 +156,24 @@ def test_key_importance_checks_scratch_alignment(lib):
 def test_wait_limit_knob_rejects_negative_values(lib):
     assert lib.pbs_debug_set_attn_wait(-1, 0) == -3
     assert lib.pbs_debug_set_attn_wait(0, 0) == 0
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="makes up addresses: only where nothing can be launched")
+@pytest.mark.parametrize("out,replica,copied", [
+    ("apart", None, False), ("k", None, True), ("v", None, True), ("last row of v", None, True), ("right behind v", None, False),
+    ("apart", "k", True), ("apart", "v", True), ("apart", "apart", False)])
+def test_dense_call_copies_keys_and_values_that_the_result_overlaps(lib, out, replica, copied):
+    """The first enqueue fails here, and its name tells the route: the copying one clears the status words first, the one
+    that reads K and V in place starts with its set-up kernel."""
+    S, H, D = 300, 4, 128
+    sh = _shape(dtype=_cabi.BF16, head_dim=D, block_size=128, segment_size=512, q_heads=H, kv_heads=H, seq_len=S)
+    st = _cabi.Strides4(S * H * D, D, H * D, 1)
+    size = 2 * S * H * D
+    at = {"k": 1 << 30, "v": 3 << 29, "apart": 1 << 31}
+    at.update({"last row of v": at["v"] + size - 2 * D, "right behind v": at["v"] + size})
+    reps = None if replica is None else C.pointer(_cabi.OutReplicas(1, 0, (C.c_void_p * _cabi.MAX_OUT_REPLICAS)(at[replica] + 256)))
+    opt = _options(out_replicas=reps)
+    rc = lib.pbs_prefill_fwd(C.byref(sh), C.c_void_p(1 << 29), st, C.c_void_p(at["k"]), st, C.c_void_p(at["v"]), st,
+                             C.c_void_p(at[out]), st, C.byref(opt), C.byref(_scratch()), None)
+    assert rc == -4
+    assert lib.pbs_last_error_string().startswith(b"clear status" if copied else b"dense_setup_kernel")

@@ -48,3 +48,31 @@ def test_in_place_equals_copied(tokens, kind, call, head_dim, block, segment):
     d = (got[0].float() - got[1].float()).abs()
     # P and the result are rounded to bf16 in both (2^-9 relative each); |v| stays below 6
     assert torch.isfinite(d).all() and d.max() <= 5e-2 and d.mean() <= 2e-3
+
+
+# the result over K or V, whole or shifted by rows, and a second copy of the result over V
+@pytest.mark.parametrize("tokens", [257, 300, 1000, 2048, 4096])
+@pytest.mark.parametrize("where", ["k", "v", "v shifted", "replica on v"])
+@pytest.mark.parametrize("call", ["dense", "mean"])
+def test_result_may_overlap_keys_or_values(tokens, where, call):
+    from pbs_attn_b200 import _cabi
+    from pbs_attn_b200.prefill import Plan
+    w = Workload("overlap", 1, 8, 8, 128, tokens, "bf16", 128, 128, 0.7, 5e5, sinks=4)
+    q, k, v = make_qkv(w, seed=tokens, device="cuda")
+    plan = Plan(1, 8, 8, tokens, 128, 128, 4096 if call == "dense" else 128, q.dtype, q.device)
+    kind = dict(no_permutation=True, diagonal_candidates=True) if call == "mean" else {}
+    want = plan.run(q, k, v, torch.empty_like(q), plan.options(0.7, attn_impl="tcgen05", **kind))
+    buf = torch.empty(tokens + 64, 8, 128, dtype=q.dtype, device=q.device)       # (S, H, D) rows: a shift stays aligned
+    seen = lambda t0: buf[t0 : t0 + tokens].transpose(0, 1)[None]
+    shared = seen(64 if where == "v shifted" else 0).copy_(k if where == "k" else v)
+    kk, vv = (shared, v) if where == "k" else (k, shared)
+    out, reps = seen(0), None
+    if where == "replica on v":
+        out = torch.empty_like(seen(0))
+        reps = _cabi.OutReplicas(1, 0, (_cabi.C.c_void_p * _cabi.MAX_OUT_REPLICAS)(shared.data_ptr()))
+    plan.run(q, kk, vv, out, plan.options(0.7, attn_impl="tcgen05", out_replicas=reps, **kind))
+    torch.cuda.synchronize()
+    plan.check_status()
+    assert torch.equal(out, want)
+    if reps is not None:
+        assert torch.equal(seen(0), want)
