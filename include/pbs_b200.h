@@ -124,6 +124,9 @@ typedef struct {
                                       (block-level causal mask incl. the diagonal, MeanPooling.py:43-48) */
   int32_t no_own_segment;          /* 1: the q block's own segment is NOT forced on (MeanPooling with
                                       force_select_current_block=False, MeanPooling.py:55-58 skipped)  */
+  int32_t kv_in_place;             /* 1: where keys keep their order (seq_len <= segment_size, or no_permutation) the
+                                      attention may read k and v themselves; the call then leaves perm_k and perm_v
+                                      (and pooled_k if seq_len <= segment_size) as they were.  0: it fills them     */
   const pbs_out_replicas_t* out_replicas; /* NULL, or extra destinations of the output (tcgen05 kernel only) */
 } pbs_options_t;
 
@@ -254,7 +257,9 @@ int pbs_enable_peer_access(int32_t peer_device);
 
 /* Whole path: stages 1a..3b in order on one stream.  For S <= segment_size it runs dense
  * causal attention like the reference (pbs_attn/src/pbs.py:175-182).  out and its replicas may share
- * memory with k and v: they are copied before the attention starts wherever they overlap.
+ * memory with k and v: they are copied before the attention starts wherever they overlap.  Afterwards
+ * key_indices, perm_k, perm_v, pooled_k, first_block and block_mask hold this call's order, keys and
+ * selection, so that pbs_attn_fwd can follow, but for what options->kv_in_place leaves out.
  * Replaces permuted_block_sparse_attn_fwd, pbs_attn/src/pbs.py:132-257. */
 int pbs_prefill_fwd(const pbs_shape_t* shape,
                     const void* q, const int64_t q_strides[4],

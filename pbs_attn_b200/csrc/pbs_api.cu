@@ -29,6 +29,9 @@ int cuda_fail(cudaError_t e, const char* what) {
 
 namespace {
 
+// kv_in_place took the place of padding: structs of callers built without it keep their layout.
+static_assert(sizeof(pbs_options_t) == 56 && offsetof(pbs_options_t, out_replicas) == 48, "pbs_options_t layout");
+
 int check_shape(const pbs_shape_t* s) {
   if (!s) { set_error("shape is null"); return PBS_ERR_ARG; }
   if (s->dtype < PBS_BF16 || s->dtype > PBS_FP32) { set_error("dtype %d is not bf16/fp16/fp32", s->dtype); return PBS_ERR_ARG; }
@@ -389,11 +392,11 @@ int pbs_prefill_fwd(const pbs_shape_t* shape, const void* q, const int64_t q_str
 
   // ---- enqueue
   cudaStream_t st = (cudaStream_t)stream;
-  // Keys in original order need no copy: the tcgen05 kernel reads K and V in place where its descriptors can and the
-  // result goes elsewhere.
+  // Keys in original order need no copy: the tcgen05 kernel reads K and V in place where its descriptors can, the
+  // result goes elsewhere and the caller has no use for the copies.
   const bool identity = dense || options->no_permutation;
-  const bool in_place = identity && impl == PBS_ATTN_TCGEN05 && layout_fits_tc(d, d.Hkv, ks) && layout_fits_tc(d, d.Hkv, vs) &&
-                        !output_meets_kv(d, shape->dtype, out, os, options->out_replicas, k, ks, v, vs);
+  const bool in_place = identity && options->kv_in_place && impl == PBS_ATTN_TCGEN05 && layout_fits_tc(d, d.Hkv, ks) &&
+                        layout_fits_tc(d, d.Hkv, vs) && !output_meets_kv(d, shape->dtype, out, os, options->out_replicas, k, ks, v, vs);
   if (dense && in_place) {
     PBS_TRY(launch_dense_setup(d, sc->key_indices, sc->first_block, sc->block_mask, sc->tile_list, sc->tile_count, sc->status, st));
   } else {

@@ -93,6 +93,7 @@ class Plan:
         self._status_pending = []          # [(event, slot)], oldest first
         self._status_next = 0
 
+    _kv_left_out = False                    # the last whole-path call may have left perm_k / perm_v as they were
     _status_rows = _status_words = None     # views of the ring, made on first use: per-slot tensors and a numpy array
 
     # ------------------------------------------------------------------ helpers
@@ -131,7 +132,9 @@ class Plan:
 
     def options(self, threshold, force_select_first_block=True, query_pool_mode="mean", key_pool_mode="mean",
                 attn_impl="auto", no_permutation=False, diagonal_candidates=False, no_own_segment=False,
-                out_replicas: Optional[_cabi.OutReplicas] = None) -> _cabi.Options:
+                out_replicas: Optional[_cabi.OutReplicas] = None, kv_in_place=False) -> _cabi.Options:
+        """``kv_in_place``: the call need not leave copies of K and V in ``perm_k`` / ``perm_v`` where keys keep
+        their order (``attn_fwd`` on its own then has nothing to work on)."""
         for m in (query_pool_mode, key_pool_mode):
             if m not in _cabi.POOL:
                 raise ValueError(f"Invalid pool mode: {m}")
@@ -147,7 +150,7 @@ class Plan:
             thr = float(threshold)
         opt = _cabi.Options(thr_ptr, thr, select_all, int(bool(force_select_first_block)),
                             _cabi.POOL[query_pool_mode], _cabi.POOL[key_pool_mode], _cabi.ATTN_IMPL[attn_impl],
-                            int(bool(no_permutation)), int(bool(diagonal_candidates)), int(bool(no_own_segment)),
+                            int(bool(no_permutation)), int(bool(diagonal_candidates)), int(bool(no_own_segment)), int(bool(kv_in_place)),
                             C.pointer(out_replicas) if out_replicas is not None else None)
         opt._keep = out_replicas            # the struct must outlive the call
         return opt
@@ -184,6 +187,7 @@ class Plan:
                                                      _ptr(self.key_indices), _ptr(self.perm_k), _ptr(self.perm_v),
                                                      _ptr(self.pooled_k), _cabi.POOL[key_pool_mode],
                                                      _ptr(self.first_block), self._stream()), "pbs_segment_permute")
+        self._kv_left_out = False
 
     def pool_queries(self, q, query_pool_mode="mean"):
         with self._on_device():
@@ -207,6 +211,9 @@ class Plan:
                                                       _ptr(self.tile_count), self._stream()), "pbs_build_tile_lists")
 
     def attn_fwd(self, q, out, attn_impl="auto"):
+        if self._kv_left_out:
+            raise RuntimeError("perm_k and perm_v do not hold the last call's keys and values: it read them in place "
+                               "(segment_permute, or a call with intermediates or without kv_in_place, fills them)")
         self.status.zero_()
         with self._on_device():
             _cabi.check(self.lib.pbs_attn_fwd(C.byref(self.shape), _ptr(q), _strides(q), _ptr(self.perm_k), _ptr(self.perm_v),
@@ -225,6 +232,8 @@ class Plan:
             _cabi.check(self.lib.pbs_prefill_fwd(C.byref(self.shape), _ptr(q), _strides(q), _ptr(k), _strides(k),
                                                  _ptr(v), _strides(v), _ptr(out), _strides(out), C.byref(opt),
                                                  C.byref(self.scratch), C.c_void_p(stream.cuda_stream)), "pbs_prefill_fwd")
+            self._kv_left_out = bool(opt.kv_in_place and (opt.no_permutation or self.dense) and self.dtype != torch.float32
+                                     and opt.attn_impl != _cabi.ATTN_IMPL["simt"])
             self._queue_status_copy(stream)
         return out
 
@@ -317,7 +326,7 @@ def permuted_block_sparse_attn_fwd(
       * ``use_triton`` is accepted and ignored (there is one backend);
       * ``attn_impl`` picks the attention kernel ("auto", "tcgen05", "simt");
       * ``intermediates``: a dict that receives the permutation, block mask and plan
-        (used by the parity tests);
+        (used by the parity tests); the plan's buffers then hold all results of the stages;
       * ``out``: a preallocated result tensor of q's shape and dtype (any strides the kernels can
         write: unit head-dim stride, 16-byte aligned rows), e.g. a head slice of a larger tensor; it may
         share memory with key_states or value_states;
@@ -340,7 +349,7 @@ def permuted_block_sparse_attn_fwd(
     v = _readable(value_states)
     plan = get_plan(q, num_kv_heads, block_size, segment_size)
     opt = plan.options(threshold, force_select_first_block, query_pool_mode, key_pool_mode, attn_impl,
-                       out_replicas=out_replicas)
+                       out_replicas=out_replicas, kv_in_place=intermediates is None)
     if out is None:
         out = torch.empty_like(q)
     elif out.shape != q.shape or out.dtype != q.dtype or out.device != q.device:
@@ -396,7 +405,8 @@ def MeanPooling_prefill(
     if not isinstance(threshold, torch.Tensor):
         threshold = float(threshold)        # the baseline has no "int 1 selects everything" rule
     opt = plan.options(threshold, force_select_first_block, "mean", "mean", attn_impl,
-                       no_permutation=True, diagonal_candidates=True, no_own_segment=not force_select_current_block)
+                       no_permutation=True, diagonal_candidates=True, no_own_segment=not force_select_current_block,
+                       kv_in_place=intermediates is None)
     out = torch.empty_like(q)
     plan.run(q, k, v, out, opt)
     if intermediates is not None:
@@ -479,7 +489,7 @@ def permuted_block_sparse_attn_fwd_host(
         _HOST_PIPES.clear()
         pipe = _HOST_PIPES[key] = _HostPipeline(B, hq_c, hkv_c, S, D, query_states.dtype, dev)
     plan = get_plan(pipe.q[0], hkv_c, block_size, segment_size)
-    opt = plan.options(threshold, force_select_first_block, query_pool_mode, key_pool_mode)
+    opt = plan.options(threshold, force_select_first_block, query_pool_mode, key_pool_mode, kv_in_place=True)
     main = torch.cuda.current_stream(dev)
     start = torch.cuda.Event()
     start.record(main)

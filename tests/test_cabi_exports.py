@@ -105,7 +105,7 @@ def _scratch(**null):
 def _options(**kw):
     d = dict(threshold_per_head=None, threshold=0.9, select_all=0, force_select_first_block=1, query_pool_mode=0,
              key_pool_mode=0, attn_impl=0, no_permutation=0, diagonal_candidates=0, no_own_segment=0,
-             out_replicas=None)
+             kv_in_place=0, out_replicas=None)
     d.update(kw)
     return _cabi.Options(*[d[n] for n, _ in _cabi.Options._fields_])
 
@@ -172,8 +172,14 @@ def test_dense_call_copies_keys_and_values_that_the_result_overlaps(lib, out, re
     at = {"k": 1 << 30, "v": 3 << 29, "apart": 1 << 31}
     at.update({"last row of v": at["v"] + size - 2 * D, "right behind v": at["v"] + size})
     reps = None if replica is None else C.pointer(_cabi.OutReplicas(1, 0, (C.c_void_p * _cabi.MAX_OUT_REPLICAS)(at[replica] + 256)))
-    opt = _options(out_replicas=reps)
+    opt = _options(kv_in_place=1, out_replicas=reps)
     rc = lib.pbs_prefill_fwd(C.byref(sh), C.c_void_p(1 << 29), st, C.c_void_p(at["k"]), st, C.c_void_p(at["v"]), st,
                              C.c_void_p(at[out]), st, C.byref(opt), C.byref(_scratch()), None)
     assert rc == -4
     assert lib.pbs_last_error_string().startswith(b"clear status" if copied else b"dense_setup_kernel")
+
+
+def test_in_place_switch_lies_in_what_was_padding():
+    """Callers built without the field pass the same bytes in the same places; its zero fills all scratch."""
+    o = _cabi.Options
+    assert C.sizeof(o) == 56 and o.kv_in_place.offset == 44 and o.out_replicas.offset == 48

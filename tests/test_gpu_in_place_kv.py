@@ -1,5 +1,5 @@
 """Calls whose keys keep their order (the dense fallback, MeanPooling) read K and V where the caller has them; compared
-with the generic kernel, which goes through the copy."""
+with the same call through the copies, and with the generic kernel."""
 import pytest
 import torch
 
@@ -28,7 +28,7 @@ def _layout(t, kind):
 @pytest.mark.parametrize("call,head_dim,block,segment", [("dense", 128, 128, 512), ("dense", 64, 64, 512), ("dense", 64, 128, 512),
                                                           ("mean", 128, 128, 128), ("mean", 64, 64, 64)])
 def test_in_place_equals_copied(tokens, kind, call, head_dim, block, segment):
-    from pbs_attn_b200.prefill import MeanPooling_prefill, permuted_block_sparse_attn_fwd
+    from pbs_attn_b200.prefill import MeanPooling_prefill, get_plan, permuted_block_sparse_attn_fwd
     w = Workload("inplace", 2, 4, 2, head_dim, tokens, "bf16", block, segment, 0.7, 5e5, sinks=4)
     q, k, v = make_qkv(w, seed=tokens, device="cuda")
     if kind == "broadcast":                     # a zero head stride: the copy is kept
@@ -36,16 +36,17 @@ def test_in_place_equals_copied(tokens, kind, call, head_dim, block, segment):
     else:
         q, k, v = (_layout(t, kind) for t in (q, k, v))
     got, inters = [], []
-    for impl in ("tcgen05", "simt"):
-        inter = {}
+    plan = get_plan(q, k.shape[1], block, segment)
+    for impl, inter in (("tcgen05", None), ("tcgen05", {}), ("simt", {})):      # only calls without intermediates read in place
         if call == "mean":
             got.append(MeanPooling_prefill(q, k, v, block, segment, 0.7, attn_impl=impl, intermediates=inter))
         else:
             got.append(permuted_block_sparse_attn_fwd(q, k, v, block, segment, 0.7, True, attn_impl=impl, intermediates=inter))
-        inter["plan"].check_status()
-        inters.append((inter["key_indices"].clone(), inter["block_mask"].clone(), inter["plan"].first_block.clone()))
-    assert all(torch.equal(a, b) for a, b in zip(*inters))
-    d = (got[0].float() - got[1].float()).abs()
+        plan.check_status()
+        inters.append((plan.key_indices.clone(), plan.block_mask.clone(), plan.first_block.clone()))
+    assert all(torch.equal(a, b) for other in inters[1:] for a, b in zip(inters[0], other))
+    assert torch.equal(got[0], got[1])
+    d = (got[0].float() - got[2].float()).abs()
     # P and the result are rounded to bf16 in both (2^-9 relative each); |v| stays below 6
     assert torch.isfinite(d).all() and d.max() <= 5e-2 and d.mean() <= 2e-3
 
@@ -61,7 +62,7 @@ def test_result_may_overlap_keys_or_values(tokens, where, call):
     q, k, v = make_qkv(w, seed=tokens, device="cuda")
     plan = Plan(1, 8, 8, tokens, 128, 128, 4096 if call == "dense" else 128, q.dtype, q.device)
     kind = dict(no_permutation=True, diagonal_candidates=True) if call == "mean" else {}
-    want = plan.run(q, k, v, torch.empty_like(q), plan.options(0.7, attn_impl="tcgen05", **kind))
+    want = plan.run(q, k, v, torch.empty_like(q), plan.options(0.7, attn_impl="tcgen05", kv_in_place=True, **kind))
     buf = torch.empty(tokens + 64, 8, 128, dtype=q.dtype, device=q.device)       # (S, H, D) rows: a shift stays aligned
     seen = lambda t0: buf[t0 : t0 + tokens].transpose(0, 1)[None]
     shared = seen(64 if where == "v shifted" else 0).copy_(k if where == "k" else v)
@@ -70,9 +71,37 @@ def test_result_may_overlap_keys_or_values(tokens, where, call):
     if where == "replica on v":
         out = torch.empty_like(seen(0))
         reps = _cabi.OutReplicas(1, 0, (_cabi.C.c_void_p * _cabi.MAX_OUT_REPLICAS)(shared.data_ptr()))
-    plan.run(q, kk, vv, out, plan.options(0.7, attn_impl="tcgen05", out_replicas=reps, **kind))
+    plan.run(q, kk, vv, out, plan.options(0.7, attn_impl="tcgen05", out_replicas=reps, kv_in_place=True, **kind))
     torch.cuda.synchronize()
     plan.check_status()
     assert torch.equal(out, want)
     if reps is not None:
         assert torch.equal(seen(0), want)
+
+
+@pytest.mark.parametrize("call", ["dense", "mean"])
+def test_stages_after_a_call_work_on_its_keys_and_values(call):
+    from pbs_attn_b200.prefill import MeanPooling_prefill, get_plan, permuted_block_sparse_attn_fwd, release_plans
+    release_plans()
+    block, segment, tokens = 128, (128 if call == "mean" else 512), 500
+    fn = MeanPooling_prefill if call == "mean" else permuted_block_sparse_attn_fwd
+    args = (block, segment, 0.7, True)
+    inputs = [make_qkv(Workload("stages", 1, 4, 2, 128, tokens, "bf16", block, segment, 0.7, 5e5, sinks=4), seed=s, device="cuda")
+              for s in (1, 2)]
+    again = torch.empty_like(inputs[0][0])
+    fn(*inputs[0], *args)                       # reads in place: nothing to go on with, and that is said
+    plan = get_plan(inputs[0][0], 2, block, segment)
+    with pytest.raises(RuntimeError, match="in place"):
+        plan.attn_fwd(inputs[0][0], again)
+    for q, k, v in inputs:
+        inter = {}
+        want = fn(q, k, v, *args, intermediates=inter)
+        assert inter["plan"] is plan
+        plan.attn_fwd(q, again, "simt")
+        d = (again.float() - want.float()).abs()
+        # P and the result are rounded to bf16 in both (2^-9 relative each); |v| stays below 6
+        assert torch.isfinite(d).all() and d.max() <= 5e-2 and d.mean() <= 2e-3
+        assert torch.equal(plan.perm_k, k.repeat_interleave(2, dim=1)) and torch.equal(plan.perm_v, v.repeat_interleave(2, dim=1))
+    fn(*inputs[0], *args)
+    plan.segment_permute(inputs[0][1], inputs[0][2], identity=True)
+    plan.attn_fwd(inputs[0][0], again)          # filled again
