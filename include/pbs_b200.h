@@ -71,7 +71,7 @@ typedef struct {
   int64_t block_mask;    /* uint8   : (B, Hq, nb, nb)                                               */
   int64_t tile_list;     /* uint32  : (B, Hq, ceil(S / 256), ceil(S / 128))                         */
   int64_t tile_count;    /* int32   : (B, Hq, ceil(S / 256))                                        */
-  int64_t status;        /* int32   : 8 words, device-side error flags and work counter             */
+  int64_t status;        /* int32   : 8 words, device-side error flags                              */
 } pbs_scratch_sizes_t;
 
 /* Device pointers of the scratch buffers, sized by pbs_scratch_sizes. */
@@ -228,8 +228,7 @@ int pbs_build_tile_lists(const pbs_shape_t* shape, const uint8_t* block_mask,
  * into the store).  Replaces the launch at pbs_attn/src/pbs.py:220-246 of the kernel
  * pbs_attn/src/kernels/permuted_block_sparse_attention.py:134-311.
  * status: 8 int32 words, zero on entry; word 0 becomes non-zero if a bounded device-side
- * wait ran out (the output is then invalid), word 7 is the tcgen05 kernel's work counter and is zero
- * again when it returns.  Two launches at once need two sets of words.  out_replicas: NULL or extra destinations. */
+ * wait ran out (the output is then invalid).  out_replicas: NULL or extra destinations. */
 int pbs_attn_fwd(const pbs_shape_t* shape,
                  const void* q, const int64_t q_strides[4],
                  const void* perm_k, const void* perm_v, const int32_t* key_indices,
@@ -259,7 +258,8 @@ int pbs_enable_peer_access(int32_t peer_device);
  * causal attention like the reference (pbs_attn/src/pbs.py:175-182).  out and its replicas may share
  * memory with k and v: they are copied before the attention starts wherever they overlap.  Afterwards
  * key_indices, perm_k, perm_v, pooled_k, first_block and block_mask hold this call's order, keys and
- * selection, so that pbs_attn_fwd can follow, but for what options->kv_in_place leaves out.
+ * selection, so that pbs_attn_fwd can follow, but for what options->kv_in_place leaves out.  The call
+ * clears the status words first and uses word 7 as a counter: one call at a time per scratch.
  * Replaces permuted_block_sparse_attn_fwd, pbs_attn/src/pbs.py:132-257. */
 int pbs_prefill_fwd(const pbs_shape_t* shape,
                     const void* q, const int64_t q_strides[4],

@@ -334,8 +334,9 @@ int pbs_attn_fwd(const pbs_shape_t* shape, const void* q, const int64_t q_stride
   }
   if (attn_impl == PBS_ATTN_TCGEN05 || (attn_impl == PBS_ATTN_AUTO && tc_ok)) {
     PBS_NONNULL(tile_list); PBS_NONNULL(tile_count); PBS_NONNULL(status);
+    // no work queue: the status words may be shared by launches that overlap
     return launch_attn_tc(d, shape->dtype, q, qs, permuted_kv(d, perm_k, perm_v), key_indices, tile_list, tile_count, out, os,
-                          status, out_replicas, (cudaStream_t)stream);
+                          status, nullptr, out_replicas, (cudaStream_t)stream);
   }
   if (attn_impl != PBS_ATTN_SIMT && attn_impl != PBS_ATTN_AUTO) { set_error("attn_impl %d unknown", attn_impl); return PBS_ERR_ARG; }
   if (replicated) { set_error("output replicas are written by the tcgen05 attention kernel only; this call runs the generic kernel"); return PBS_ERR_UNSUPPORTED; }
@@ -419,9 +420,11 @@ int pbs_prefill_fwd(const pbs_shape_t* shape, const void* q, const int64_t q_str
     if (impl == PBS_ATTN_TCGEN05)
       PBS_TRY(pbs_build_tile_lists(&attn_shape, sc->block_mask, sc->tile_list, sc->tile_count, stream));
   }
-  if (in_place)
-    return launch_attn_tc(d, shape->dtype, q, qs, KvSource{k, v, ks, vs, d.group}, nullptr, sc->tile_list, sc->tile_count, out, os,
-                          sc->status, options->out_replicas, st);
+  // The scratch serves one call at a time and its status words were cleared above, so word 7 can count the draws.
+  if (impl == PBS_ATTN_TCGEN05)
+    return launch_attn_tc(d, shape->dtype, q, qs, in_place ? KvSource{k, v, ks, vs, d.group} : permuted_kv(d, sc->perm_k, sc->perm_v),
+                          in_place ? nullptr : sc->key_indices, sc->tile_list, sc->tile_count, out, os, sc->status, sc->status + 7,
+                          options->out_replicas, st);
   return pbs_attn_fwd(&attn_shape, q, q_strides, sc->perm_k, sc->perm_v, sc->key_indices, sc->block_mask,
                       sc->tile_list, sc->tile_count, out, out_strides, impl, sc->status, options->out_replicas, stream);
 }

@@ -8,7 +8,7 @@
 // Work item = 256 consecutive queries of one (b, h): two 128-row query tiles that share every K/V
 // tile staged in shared memory.  The item's tile list (built by tile_list_kernel) names the 128-key
 // tiles that either query tile selected.  A persistent CTA (one per SM) draws its items from a queue
-// and walks them with twelve warps in four roles:
+// (in the stage call a CTA takes one entry of it) and walks them with twelve warps in four roles:
 //   warp 0      draws the items and tells the other roles; TMA producer: Q tiles, then K and V tiles of the list
 //               into two 2-deep rings
 //   warps 1, 3  MMA issuers, one per query tile.  A 128-key tile is two half-steps of 64 keys with
@@ -222,12 +222,16 @@ struct Bars {
 // Work order.  Within a head the query groups are taken in the order G-1, 0, G-2, 1, ... and a CTA
 // takes two consecutive positions at a time, i.e. a long group followed by the short group that
 // complements it: every such pair has the same number of key tiles (2G + 2 in the dense case), so
-// (a) the CTAs stay balanced without a dynamic queue and (b) all CTAs start their long group at the
-// same time and walk up the head's key range together -- a K/V tile is then fetched from HBM once
-// and served to the other CTAs from L2, instead of every CTA sweeping at its own position.
+// all CTAs start their long group at the same time and walk up the head's key range together -- a K/V
+// tile is then fetched from HBM once and served to the other CTAs from L2, instead of every CTA
+// sweeping at its own position.
 // The pairs rarely fill the last wave of CTAs, a pair is too coarse to share out, and where the selection is sparse
 // the groups of a length differ.  So the work is a queue that CTAs draw from: first the pairs, all but those of
 // the last full wave and what is left over; those are dealt out group by group, the longest of all heads left first.
+// The counter of the draws has to belong to one launch alone.  The whole-path call has such a word (its scratch serves one
+// call at a time and is cleared at its start); the stage call has not, because its status words may be shared by launches
+// that overlap.  It starts a CTA per entry instead, in the same order, which costs a start-up an entry: 4 x 2048 tokens
+// 209 us (queue 200, fixed pairs 222), 6001 sparse tokens 221 (221, 246), head_dim 64 378 (378, 441), longer ones alike.
 // Measured against fixed pairs (this kernel alone, 32 heads): 4 x 2048 tokens 229 -> 208 us, 6001 sparse tokens
 // 253 -> 224, 8192 tokens 533 -> 486 (head_dim 64: 448 -> 384), 32768 sparse tokens 4.25 -> 4.13 ms; with 13 waves or
 // more of equal pairs nothing changes (4 heads of 131072 tokens: 14.3 ms both ways).
@@ -276,7 +280,7 @@ struct Params {
   int bs;
   float scale_log2e;
   int32_t* status;
-  int32_t* queue;               // draws so far; zero before and after a launch
+  int32_t* queue;               // draws so far, zero before and after a launch; null: a CTA has one entry
   void* extra_out[PBS_MAX_OUT_REPLICAS];   // further destinations of the output (same strides), e.g. on peer GPUs
   int n_extra;
   unsigned long long wait_ns;   // limit of every device-side wait
@@ -402,16 +406,20 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       uint32_t kc = 0, vc = 0, qc[2] = {0, 0};
       bool ok = true;
       const uint64_t pol_kv = l2_policy_evict_last(), pol_q = l2_policy_evict_first();
-      // The items of this CTA: its first queue entry is its own number, each further one is drawn while the entry before
-      // it is loaded.
+      // The items of this CTA: its first queue entry is its own number, each further one (with a counter) is drawn while
+      // the entry before it is loaded.
       int q = (int)blockIdx.x, q_next = 0, j = 0;
       for (int it = 0, bh, g; ok; ++it) {
         const bool more = queue_item(p.work, q, j, bh, g);
         if (more && j == 0 && elect_one()) {
-          // one draw per entry of the queue; the last one leaves the counter at zero for the next launch
-          const int drawn = atomicAdd(p.queue, 1);
-          if (drawn == p.work.n_items - p.work.pairs - 1) atomicExch(p.queue, 0);
-          q_next = (int)gridDim.x + drawn;
+          if (p.queue) {
+            // one draw per entry of the queue; the last one leaves the counter at zero
+            const int drawn = atomicAdd(p.queue, 1);
+            if (drawn == p.work.n_items - p.work.pairs - 1) atomicExch(p.queue, 0);
+            q_next = (int)gridDim.x + drawn;
+          } else {
+            q_next = p.work.n_items;                       // past the end
+          }
         }
         ok = wait_bar_warp(smem_u32(&bars->item_empty[it % kSched]), ((it / kSched) & 1u) ^ 1u, ctl, p.status, 13);
         if (!ok) break;
@@ -850,7 +858,7 @@ int make_map(CUtensorMap* map, int dt, const void* base, const Dims& d, int head
 
 template <int DT, int D>
 int run_tc(const Dims& d, const void* q, Strides qs, const KvSource& kv, const int32_t* idx,
-           const uint32_t* list, const int32_t* count, void* out, Strides os, int32_t* status,
+           const uint32_t* list, const int32_t* count, void* out, Strides os, int32_t* status, int32_t* queue,
            const pbs_out_replicas_t* replicas, cudaStream_t st) {
   CUtensorMap mq, mk, mv;
   int rc = make_map(&mq, DT, q, d, d.Hq, qs);
@@ -876,12 +884,12 @@ int run_tc(const Dims& d, const void* q, Strides qs, const KvSource& kv, const i
   const int smem = Smem<D>::kTotal;
   cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (ce != cudaSuccess) return cuda_fail(ce, "attn_tc_kernel smem attribute");
-  p.queue = status + 7;
+  p.queue = queue;
   const int items = d.B * d.Hq * p.G;
-  const int grid = items < sm_count ? items : sm_count;
-  const int waves = items / 2 / grid;                      // full waves of pairs
-  p.work = Schedule{items, p.G, d.B * d.Hq, grid * (items == 2 * grid * waves ? waves : (waves > 0 ? waves - 1 : 0))};
-  kern<<<grid, kThreads, smem, st>>>(mq, mk, mv, p);
+  const int resident = items < sm_count ? items : sm_count;
+  const int waves = items / 2 / resident;                  // full waves of pairs
+  p.work = Schedule{items, p.G, d.B * d.Hq, resident * (items == 2 * resident * waves ? waves : (waves > 0 ? waves - 1 : 0))};
+  kern<<<queue ? resident : items - p.work.pairs, kThreads, smem, st>>>(mq, mk, mv, p);
   PBS_CUDA_CHECK_LAUNCH("attn_tc_kernel");
   return PBS_OK;
 }
@@ -899,13 +907,14 @@ bool attn_tc_supported(const Dims& d, int dt) {
 }
 
 int launch_attn_tc(const Dims& d, int dt, const void* q, Strides qs, const KvSource& kv, const int32_t* idx,
-                   const uint32_t* list, const int32_t* count, void* out, Strides os, int32_t* status, const pbs_out_replicas_t* replicas, cudaStream_t st) {
+                   const uint32_t* list, const int32_t* count, void* out, Strides os, int32_t* status, int32_t* queue,
+                   const pbs_out_replicas_t* replicas, cudaStream_t st) {
   if (dt == PBS_BF16) {
-    if (d.D == 128) return run_tc<PBS_BF16, 128>(d, q, qs, kv, idx, list, count, out, os, status, replicas, st);
-    return run_tc<PBS_BF16, 64>(d, q, qs, kv, idx, list, count, out, os, status, replicas, st);
+    if (d.D == 128) return run_tc<PBS_BF16, 128>(d, q, qs, kv, idx, list, count, out, os, status, queue, replicas, st);
+    return run_tc<PBS_BF16, 64>(d, q, qs, kv, idx, list, count, out, os, status, queue, replicas, st);
   }
-  if (d.D == 128) return run_tc<PBS_FP16, 128>(d, q, qs, kv, idx, list, count, out, os, status, replicas, st);
-  return run_tc<PBS_FP16, 64>(d, q, qs, kv, idx, list, count, out, os, status, replicas, st);
+  if (d.D == 128) return run_tc<PBS_FP16, 128>(d, q, qs, kv, idx, list, count, out, os, status, queue, replicas, st);
+  return run_tc<PBS_FP16, 64>(d, q, qs, kv, idx, list, count, out, os, status, queue, replicas, st);
 }
 
 }  // namespace pbs

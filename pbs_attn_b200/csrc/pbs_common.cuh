@@ -201,8 +201,10 @@ struct KvSource {
   Strides ks, vs;
   int group;
 };
+// queue: a zero word that no other launch uses meanwhile, for resident CTAs that draw their work; null: a CTA per
+// share of the work.
 int launch_attn_tc(const Dims& d, int dt, const void* q, Strides qs, const KvSource& kv, const int32_t* idx,
-                   const uint32_t* list, const int32_t* count, void* out, Strides os, int32_t* status,
+                   const uint32_t* list, const int32_t* count, void* out, Strides os, int32_t* status, int32_t* queue,
                    const pbs_out_replicas_t* replicas, cudaStream_t st);
 
 }  // namespace pbs

@@ -29,3 +29,35 @@ def test_every_item_once_and_counter_back_at_zero(groups, heads):
     d = (first.float() - generic.float()).abs()
     # both kernels round P and the result to bf16 (2^-9 relative each); a row attends to 128 keys or more of unit variance
     assert torch.isfinite(d).all() and d.max() <= 2e-2 and d.mean() <= 1e-3
+
+
+# 512 items, more than three waves of CTAs
+def test_stage_call_needs_no_words_of_its_own():
+    """pbs_attn_fwd on status words that an earlier call left behind, and twice at once on one set of them."""
+    from pbs_attn_b200 import _cabi
+    from pbs_attn_b200.prefill import Plan, _ptr, _strides
+    S, H = 4096, 32
+    w = Workload("words", 1, H, 8, 128, S, "bf16", 128, 256, 0.8, 5e5, sinks=4)
+    q, k, v = make_qkv(w, seed=5, device="cuda")
+    plan = Plan(1, H, 8, S, 128, 128, 256, q.dtype, q.device)
+    want = plan.run(q, k, v, torch.empty_like(q), plan.options(0.8, attn_impl="tcgen05"))
+    plan.check_status()
+
+    def stage(words, stream):
+        out = torch.full_like(q, float("nan"))
+        stream.wait_stream(torch.cuda.current_stream())
+        _cabi.check(plan.lib.pbs_attn_fwd(_cabi.C.byref(plan.shape), _ptr(q), _strides(q), _ptr(plan.perm_k), _ptr(plan.perm_v),
+                                          _ptr(plan.key_indices), _ptr(plan.block_mask), _ptr(plan.tile_list), _ptr(plan.tile_count),
+                                          _ptr(out), _strides(out), _cabi.ATTN_IMPL["tcgen05"], _ptr(words), None,
+                                          _cabi.C.c_void_p(stream.cuda_stream)), "pbs_attn_fwd")
+        return out
+
+    left = torch.tensor([0] + [5] * 7, dtype=torch.int32, device="cuda")
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    outs = [stage(left, streams[0])]
+    torch.cuda.synchronize()
+    shared = torch.zeros(8, dtype=torch.int32, device="cuda")
+    outs += [stage(shared, s) for s in streams for _ in range(4)]
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, want) for o in outs)
+    assert left.tolist() == [0] + [5] * 7 and not shared.any()
