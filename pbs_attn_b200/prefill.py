@@ -94,7 +94,7 @@ class Plan:
         self._status_next = 0
 
     _kv_left_out = False                    # the last whole-path call may have left perm_k / perm_v as they were
-    _status_rows = _status_words = None     # views of the ring, made on first use: per-slot tensors and a numpy array
+    _status_rows = _status_words = None     # views of the ring, made on first use: per-slot tensors and an array of ints
 
     # ------------------------------------------------------------------ helpers
     def _stream(self):
@@ -116,13 +116,15 @@ class Plan:
             elif not ev.query():
                 break
             self._status_pending.pop(0)
-            if self._status_words[slot, 0] != 0:
+            if self._status_words[8 * slot] != 0:
                 self._status_pending.clear()
-                self._raise_status(self._status_words[slot].tolist())
+                self._raise_status(self._status_words[8 * slot : 8 * slot + 8])
 
     def _queue_status_copy(self, stream):
         if self._status_rows is None:
-            self._status_rows, self._status_words = self._status_ring.unbind(0), self._status_ring.numpy()
+            ring = self._status_ring                        # the views live as long as the plan, and so does the ring
+            self._status_words = (C.c_int32 * ring.numel()).from_address(ring.data_ptr())
+            self._status_rows = ring.unbind(0)
         slot = self._status_next
         self._status_next = (slot + 1) % _STATUS_SLOTS
         self._status_rows[slot].copy_(self.status, non_blocking=True)

@@ -146,3 +146,21 @@ def test_status_ring_bounds_the_host_run_ahead(monkeypatch):
     assert len(plan._status_pending) <= prefill._STATUS_SLOTS
     slots = [s for _, s in plan._status_pending]
     assert len(set(slots)) == len(slots)
+
+
+def test_status_words_are_read_without_numpy(monkeypatch):
+    """torch works without numpy installed; so does a call and the check of its status."""
+    def no_numpy(self, *a, **k):
+        raise RuntimeError("Numpy is not available")
+
+    monkeypatch.setattr(torch.Tensor, "numpy", no_numpy)
+    plan = fake_plan(monkeypatch)
+    q = torch.zeros(1, 4, 1024, 128, dtype=torch.bfloat16)
+    out, opt = torch.zeros_like(q), plan.options(0.9)
+    for _ in range(3):
+        plan.run(q, q, q, out, opt)
+    ev, slot = plan._status_pending[1]
+    plan._status_ring[slot] = torch.tensor([9, 0, 0, 0, 0, 0, 0, 3], dtype=torch.int32)
+    plan._status_pending[0][0].done = ev.done = True
+    with pytest.raises(_cabi.PbsError, match=r"\[9, 0, 0, 0, 0, 0, 0, 3\].*code 9"):
+        plan.run(q, q, q, out, opt)
