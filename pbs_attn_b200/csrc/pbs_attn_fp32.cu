@@ -9,8 +9,9 @@
 // 8 shared-memory reads of 16 bytes, and the 16 lanes that share rows reduce them by shuffles and pass P through
 // shared memory without a block-wide barrier.  The products of two neighbouring head-dim elements go into two partial
 // sums (packed fp32 pairs), which are added at the end of the row.
-// 4 heads x 2048 tokens, head_dim 64, block 64 (1.0 G FMA): 1200 us with pbs_attn_simt.cu's kernel (one row and 8 keys a
-// thread, operands re-read for every FMA), 130 us here.
+// Measured against pbs_attn_simt.cu's kernel (one row and 8 keys a thread, operands re-read for every FMA), 2048 tokens, block 64:
+// 4 heads of 64 (1.1 G FMA) 1079 -> 127 us, 8 heads of 128 (4.6 G FMA) 1955 -> 277 us = 33 TFLOP/s; 8192 tokens 8230 -> 1032
+// and (block 128) 19880 -> 3456 us = 38 TFLOP/s.
 #include "pbs_common.cuh"
 
 namespace pbs {
@@ -37,7 +38,7 @@ template <int D>
 __global__ void __launch_bounds__(FT, 2)
 attn_fp32_kernel(const float* __restrict__ q, Strides qs, const float* __restrict__ pk, const float* __restrict__ pv,
                  const int32_t* __restrict__ idx, const uint8_t* __restrict__ mask, float* __restrict__ out, Strides os,
-                 int Hq, int S, int bs, int seg, int nb, float scale_log2e) {
+                 int Hq, int S, int bs, int nb, float scale_log2e) {
   using SM = Fp32Smem<D>;
   constexpr int LD = SM::kLd, NBUF = SM::kBuf, C4 = D / 4, OC = D / 16;
   extern __shared__ __align__(16) float sm[];
@@ -140,8 +141,10 @@ attn_fp32_kernel(const float* __restrict__ q, Strides qs, const float* __restric
           sp[i][j] = __ffma2_rn(make_float2(a[i].z, a[i].w), make_float2(c[j].z, c[j].w), sp[i][j]);
         }
     }
-    // online softmax; keys of the rows' own segment may lie after the query
-    const bool own = first_key(s) / seg >= r0 / seg;
+    // online softmax; every key's position counts, because the order of a stage call need not stay inside the segments
+    int kp[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) kp[j] = kpos[buf * FN + tx + 16 * j];
     float p[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -150,7 +153,7 @@ attn_fp32_kernel(const float* __restrict__ q, Strides qs, const float* __restric
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         float x = (sp[i][j].x + sp[i][j].y) * scale_log2e;
-        if (own && kpos[buf * FN + tx + 16 * j] > qpos) x = -CUDART_INF_F;
+        if (kp[j] > qpos) x = -CUDART_INF_F;
         p[i][j] = x;
         mt = fmaxf(mt, x);
       }
@@ -215,7 +218,7 @@ int run_fp32(const Dims& d, const void* q, Strides qs, const void* pk, const voi
   cudaError_t e = cudaFuncSetAttribute(attn_fp32_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return cuda_fail(e, "attn_fp32_kernel smem attribute");
   attn_fp32_kernel<D><<<dim3(d.B * d.Hq, (d.S + FM - 1) / FM), FT, smem, st>>>(
-      (const float*)q, qs, (const float*)pk, (const float*)pv, idx, mask, (float*)out, os, d.Hq, d.S, d.bs, d.seg, d.nb,
+      (const float*)q, qs, (const float*)pk, (const float*)pv, idx, mask, (float*)out, os, d.Hq, d.S, d.bs, d.nb,
       (float)(1.4426950408889634 / sqrt((double)d.D)));
   PBS_CUDA_CHECK_LAUNCH("attn_fp32_kernel");
   return PBS_OK;

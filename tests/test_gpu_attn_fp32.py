@@ -34,3 +34,24 @@ def test_fp32_kernel_equals_generic_kernel(tokens, head_dim, block, segment, kin
     # both sum up to 2047 products of unit size in fp32 (2^-24 relative each, in different orders) and take exp2 of the sums
     assert (a - b).norm() <= 4e-6 * b.norm()
     assert (a - b).abs().max() <= 2e-5
+
+
+@pytest.mark.parametrize("tokens,head_dim", [(130, 128), (700, 64), (700, 128)])
+def test_any_order_of_the_keys(tokens, head_dim):
+    """The stage call with an order that crosses segments and all blocks on: plain causal attention."""
+    from pbs_attn_b200.prefill import Plan
+    w = Workload("order", 1, 4, 2, head_dim, tokens, "fp32", 64, 128, 0.7, 5e5, sinks=4)
+    q, k, v = make_qkv(w, seed=tokens, device="cuda")
+    plan = Plan(1, 4, 2, tokens, head_dim, 64, 128, q.dtype, q.device)
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    order = torch.stack([torch.randperm(tokens, generator=g, device="cuda") for _ in range(4)])[None]
+    k, v = (t.repeat_interleave(2, dim=1) for t in (k, v))
+    plan.key_indices.copy_(order)
+    plan.block_mask.fill_(1)
+    for dst, src in ((plan.perm_k, k), (plan.perm_v, v)):
+        dst.copy_(src.gather(2, order[..., None].expand_as(src)))
+    out = torch.empty_like(q)
+    plan.attn_fwd(q, out)
+    want = torch.nn.functional.scaled_dot_product_attention(q.double(), k.double(), v.double(), is_causal=True)
+    # sums of up to 700 products of unit size in fp32 (2^-24 relative each), exp2 of the sums
+    assert (out.double() - want).norm() <= 4e-6 * want.norm()
