@@ -27,6 +27,13 @@ int cuda_fail(cudaError_t e, const char* what) {
   return PBS_ERR_CUDA;
 }
 
+int device_sms() {
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
+    n = 148;
+  return n;
+}
+
 namespace {
 
 // kv_in_place took the place of padding: structs of callers built without it keep their layout.

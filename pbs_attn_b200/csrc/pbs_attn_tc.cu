@@ -876,10 +876,7 @@ int run_tc(const Dims& d, const void* q, Strides qs, const KvSource& kv, const i
   for (int x = 0; x < PBS_MAX_OUT_REPLICAS; ++x) p.extra_out[x] = x < p.n_extra ? replicas->out[x] : nullptr;
   p.wait_ns = g_wait_ns.load(std::memory_order_relaxed);
   p.drop_arrive = g_drop_arrive.load(std::memory_order_relaxed);
-  int dev = 0, sm_count = 0;                               // of the device this launch goes to
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      sm_count <= 0)
-    sm_count = 148;
+  const int sm_count = device_sms();
   auto kern = attn_tc_kernel<DT, D>;
   const int smem = Smem<D>::kTotal;
   cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

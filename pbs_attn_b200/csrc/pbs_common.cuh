@@ -170,6 +170,7 @@ void count_launch();
   } while (0)
 
 // Stage launchers (defined one per .cu file).
+int device_sms();             // SMs of the current device, the one a launch goes to
 int launch_key_importance(const Dims& d, int dt, const void* q, Strides qs, const void* k, Strides ks,
                           void* logits, void* partials, void* rowstats, float* importance, cudaStream_t st);
 int launch_segment_permute(const Dims& d, int dt, const float* importance, const void* k, Strides ks,

@@ -200,14 +200,14 @@ select_kernel(const typename Elem<DT>::T* __restrict__ pooled_q, const typename 
 // ---------------------------------------------------------------------------------------------
 // Tiled variant: one CTA = 16 (or 8) consecutive q blocks of one (b, h).
 //
-// Phase A computes the pooled logits of the 16 rows against 64-kv-block chunks of pooled K that
-// arrive in shared memory by cp.async (each pooled-K row is then read once per 16 rows instead of
+// Phase A computes the pooled logits of the CTA's rows against 64-kv-block chunks of pooled K that
+// arrive in shared memory by cp.async (each pooled-K row is then read once per 16 or 8 rows instead of
 // once per row).  The dot product keeps the summation order of select_kernel: 16-byte pieces are
 // summed front to back, the piece sums are combined in the order of a butterfly over the pieces.
 // Phases B-D run one warp per row: fp32 softmax (the exponent sum is taken in the same order as the
 // 256-thread reduction of select_kernel), then the cut of the cumulative-threshold selection is
-// found WITHOUT sorting: the bits of the cut probability are fixed one at a time, each step summing
-// (in double) the probabilities at or above the trial value; blocks above the cut are kept, blocks
+// found WITHOUT sorting: the bits of the cut probability are fixed one or two at a time, each step summing
+// (in double) the probabilities at or above the trial values; blocks above the cut are kept, blocks
 // equal to it are added in kv-block order until the running sum reaches the threshold -- the set a
 // stable descending sort followed by a running sum selects.
 // ---------------------------------------------------------------------------------------------
@@ -243,9 +243,9 @@ select_tiled_kernel(const typename Elem<DT>::T* __restrict__ pooled_q, const typ
   constexpr int D = CPR * EPV;
   constexpr int LDK = D + EPV;                             // padded pooled-K row in shared memory
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float* Qs = reinterpret_cast<float*>(smem_raw);          // [16][D] fp32
+  float* Qs = reinterpret_cast<float*>(smem_raw);          // [TS_ROWS][D] fp32
   T* Kc = reinterpret_cast<T*>(Qs + TS_ROWS * D);          // [2][64][LDK]
-  T* lg = Kc + 2 * TS_CHUNK * LDK;                         // [16][ncpad] rounded logits
+  T* lg = Kc + 2 * TS_CHUNK * LDK;                         // [TS_ROWS][ncpad] rounded logits
 
   const int qb0 = blockIdx.x * TS_ROWS;
   const int bh = blockIdx.y;
@@ -309,7 +309,7 @@ select_tiled_kernel(const typename Elem<DT>::T* __restrict__ pooled_q, const typ
   }
   if (nchunks == 0) __syncthreads();
 
-  // ---- phases B-D: one warp per row (rows 2 * warp and 2 * warp + 1)
+  // ---- phases B-D: one warp per row (16 rows: 2 * warp and 2 * warp + 1)
   const float thr = thr_per_head ? thr_per_head[h] : thr_scalar;
   for (int rr = 0; rr < TS_ROWS / 8; ++rr) {
     const int r = warp * (TS_ROWS / 8) + rr;
@@ -563,14 +563,16 @@ int run_select_tiled(const Dims& d, const void* pooled_q, const void* pooled_k, 
   return PBS_OK;
 }
 
-// 16 rows a CTA read pooled K half as often as 8, but a warp then works off two rows one after the other.  As long as
-// all CTAs of 8 rows are resident at once (three a SM, 148 SMs) the second row is pure latency: with the two-bit steps of
-// the search, 128 heads x 16 blocks 26 -> 16 us; beyond that line (32 heads x 128 blocks of 64) 16 rows stay as fast.
+// 16 rows a CTA read pooled K half as often as 8, but a warp then works off two rows one after the other, which is pure
+// latency while the SMs have room.  Up to three CTAs of 8 rows a SM they were faster in all forms tried (8 / 16 rows, us, 444 CTAs
+// or just below on 148 SMs): bf16 D = 128, 16 blocks a row 17.7 / 25.7, 64 blocks 20.6 / 31.3, 128 blocks 27.8 / 39.6, 256 blocks 39.8 / 54.4;
+// fp32 D = 128 16.8 / 21.7, 20.1 / 29.0, 29.6 / 39.3, 48.2 / 55.2.  At four a SM wide rows (32 pieces, two or three CTAs resident) lose:
+// fp32 D = 128 26.7 / 21.8, 33.7 / 29.1, 42.5 / 36.6, 56.6 / 60.4; at eight all do: bf16 D = 128 40.3 / 36.1 .. 83.9 / 90.6.
 template <int DT, int CPR>
 int run_select_tiled_k(const Dims& d, const void* pooled_q, const void* pooled_k, const int32_t* first_block,
                        const pbs_options_t& opt, uint8_t* mask, float* scores, cudaStream_t st) {
   if (d.nb <= 256) {
-    if ((int64_t)((d.nb + 7) / 8) * d.B * d.Hq <= 3 * 148)
+    if ((int64_t)((d.nb + 7) / 8) * d.B * d.Hq <= 3 * device_sms())
       return run_select_tiled<DT, CPR, 8, 8>(d, pooled_q, pooled_k, first_block, opt, mask, scores, st);
     return run_select_tiled<DT, CPR, 8, 16>(d, pooled_q, pooled_k, first_block, opt, mask, scores, st);
   }

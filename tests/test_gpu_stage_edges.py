@@ -28,14 +28,17 @@ def test_importance_is_the_softmax_of_its_own_logits(tiles, dtype, D):
     assert ((imp.double() - want).abs() <= 2e-6 * want).all()
 
 
-# 8-row CTAs up to 444 of them, 16-row CTAs beyond (nb <= 256), and the larger register counts
+# 8-row CTAs up to 444 of them (148 SMs), 16-row CTAs beyond (nb <= 256), and the larger register counts; pooled rows of
+# 8, 16 and 32 16-byte pieces
 @pytest.mark.parametrize("heads,nb", [(1, 3), (27, 128), (28, 128), (55, 64), (56, 64), (13, 256), (14, 256), (2, 300), (2, 600), (1, 1030)])
 @pytest.mark.parametrize("thr", [0.0, 0.3, 0.9, 1.0, 2.0])
-def test_selection_equals_the_general_kernel(heads, nb, thr):
+@pytest.mark.parametrize("dtype,D,diagonal", [(torch.bfloat16, 64, False), (torch.bfloat16, 128, False), (torch.float16, 128, True),
+                                              (torch.bfloat16, 256, True), (torch.float32, 64, True), (torch.float32, 128, False)])
+def test_selection_equals_the_general_kernel(heads, nb, thr, dtype, D, diagonal):
     from pbs_attn_b200 import _cabi
     from pbs_attn_b200.prefill import Plan
     lib = _cabi.load()
-    plan = Plan(1, heads, 1, nb * 64 - 7, 64, 64, 128, torch.bfloat16, "cuda")
+    plan = Plan(1, heads, 1, nb * 64 - 7, D, 64, 128, dtype, "cuda")
     g = torch.Generator(device="cuda").manual_seed(nb)
     plan.pooled_q.copy_(torch.randn(plan.pooled_q.shape, generator=g, device="cuda"))
     plan.pooled_k.copy_(torch.randn(plan.pooled_k.shape, generator=g, device="cuda").round())    # ties among the scores
@@ -44,7 +47,7 @@ def test_selection_equals_the_general_kernel(heads, nb, thr):
     try:
         for impl in (0, 1):
             lib.pbs_debug_set_select_impl(impl)
-            scores = plan.select_blocks(plan.options(thr), want_scores=True)
+            scores = plan.select_blocks(plan.options(thr, diagonal_candidates=diagonal), want_scores=True)
             got.append((plan.block_mask.clone(), scores))
     finally:
         lib.pbs_debug_set_select_impl(0)
