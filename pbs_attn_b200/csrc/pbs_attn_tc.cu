@@ -34,6 +34,7 @@
 #include <atomic>
 
 #include "pbs_common.cuh"
+#include "pbs_schedule.h"
 
 namespace pbs {
 namespace {
@@ -219,55 +220,6 @@ struct Bars {
   uint64_t drain;                                       // teardown after an abort: both issuers' MMAs retired
 };
 
-// Work order.  Within a head the query groups are taken in the order G-1, 0, G-2, 1, ... and a CTA
-// takes two consecutive positions at a time, i.e. a long group followed by the short group that
-// complements it: every such pair has the same number of key tiles (2G + 2 in the dense case), so
-// all CTAs start their long group at the same time and walk up the head's key range together -- a K/V
-// tile is then fetched from HBM once and served to the other CTAs from L2, instead of every CTA
-// sweeping at its own position.
-// The pairs rarely fill the last wave of CTAs, a pair is too coarse to share out, and where the selection is sparse
-// the groups of a length differ.  So the work is a queue that CTAs draw from: first the pairs, all but those of
-// the last full wave and what is left over; those are dealt out group by group, the longest of all heads left first.
-// The counter of the draws has to belong to one launch alone.  The whole-path call has such a word (its scratch serves one
-// call at a time and is cleared at its start); the stage call has not, because its status words may be shared by launches
-// that overlap.  It starts a CTA per entry instead, in the same order, which costs a start-up an entry: 4 x 2048 tokens
-// 209 us (queue 200, fixed pairs 222), 6001 sparse tokens 221 (221, 246), head_dim 64 378 (378, 441), longer ones alike.
-// Measured against fixed pairs (this kernel alone, 32 heads): 4 x 2048 tokens 229 -> 208 us, 6001 sparse tokens
-// 253 -> 224, 8192 tokens 533 -> 486 (head_dim 64: 448 -> 384), 32768 sparse tokens 4.25 -> 4.13 ms; with 13 waves or
-// more of equal pairs nothing changes (4 heads of 131072 tokens: 14.3 ms both ways).
-struct Schedule {
-  int n_items, G, BH, pairs;        // pairs: entries of the queue that are pairs
-};
-// Queue entry q, its j-th item (j = 1 only for pairs); false past the end.
-__device__ __forceinline__ bool queue_item(const Schedule& w, int q, int j, int& bh, int& g) {
-  if (q < w.pairs) {
-    const int pos = 2 * q + j, r = pos % w.G;
-    bh = pos / w.G;
-    g = (r & 1) ? (r >> 1) : (w.G - 1 - (r >> 1));
-    return true;
-  }
-  const int first = 2 * w.pairs;                           // positions the pairs have taken
-  int k = q - w.pairs;
-  if (j || k >= w.n_items - first) return false;
-  // the first head left may have lost its longest and its shortest groups to the pairs: [lo, hi] remain
-  const int bh0 = first / w.G, r0 = first % w.G;
-  const int lo = r0 >> 1, hi = w.G - 1 - ((r0 + 1) >> 1);
-  const int whole = w.BH - bh0 - 1;                        // heads after it, with all their groups
-  const int above = (w.G - 1 - hi) * whole, within = (hi - lo + 1) * (whole + 1);
-  if (k < above) {
-    g = w.G - 1 - k / whole;
-    bh = bh0 + 1 + k % whole;
-  } else if ((k -= above) < within) {
-    g = hi - k / (whole + 1);
-    bh = bh0 + k % (whole + 1);
-  } else {
-    k -= within;
-    g = lo - 1 - k / whole;
-    bh = bh0 + 1 + k % whole;
-  }
-  return true;
-}
-
 struct Params {
   const int32_t* idx;         // (B*Hq, S) original position of each key slot; null: the identity
   int kv_group;               // query heads that share a K/V head of the tensor maps
@@ -415,7 +367,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
           if (p.queue) {
             // one draw per entry of the queue; the last one leaves the counter at zero
             const int drawn = atomicAdd(p.queue, 1);
-            if (drawn == p.work.n_items - p.work.pairs - 1) atomicExch(p.queue, 0);
+            if (drawn == entries(p.work) - 1) atomicExch(p.queue, 0);
             q_next = (int)gridDim.x + drawn;
           } else {
             q_next = p.work.n_items;                       // past the end
@@ -882,11 +834,8 @@ int run_tc(const Dims& d, const void* q, Strides qs, const KvSource& kv, const i
   cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (ce != cudaSuccess) return cuda_fail(ce, "attn_tc_kernel smem attribute");
   p.queue = queue;
-  const int items = d.B * d.Hq * p.G;
-  const int resident = items < sm_count ? items : sm_count;
-  const int waves = items / 2 / resident;                  // full waves of pairs
-  p.work = Schedule{items, p.G, d.B * d.Hq, resident * (items == 2 * resident * waves ? waves : (waves > 0 ? waves - 1 : 0))};
-  kern<<<queue ? resident : items - p.work.pairs, kThreads, smem, st>>>(mq, mk, mv, p);
+  p.work = make_schedule(d.B * d.Hq, p.G, sm_count);
+  kern<<<queue ? p.work.ctas : entries(p.work), kThreads, smem, st>>>(mq, mk, mv, p);
   PBS_CUDA_CHECK_LAUNCH("attn_tc_kernel");
   return PBS_OK;
 }

@@ -22,6 +22,13 @@ def _layout(t, kind):
     return t
 
 
+def _same_but_for_rounding(a, b, scale):
+    """P and the result are rounded to bf16 in both, 2^-8 relative each: with sum P |v| = scale (itself rounded twice) they
+    differ by no more than 2 * 2^-8 (scale + |result|)."""
+    d = (a.float() - b.float()).abs()
+    assert (d <= 2.0 ** -7 * 1.02 * (scale.float() + b.float().abs())).all() and d.mean() <= 2e-3
+
+
 # one token, edges of the 128-row tile and of the 256-row group, tails of a block, both block and head sizes
 @pytest.mark.parametrize("tokens", [1, 2, 127, 128, 129, 187, 256, 300, 512])
 @pytest.mark.parametrize("kind", ["plain", "strided", "heads_first", "wide", "broadcast"])
@@ -46,9 +53,11 @@ def test_in_place_equals_copied(tokens, kind, call, head_dim, block, segment):
         inters.append((plan.key_indices.clone(), plan.block_mask.clone(), plan.first_block.clone()))
     assert all(torch.equal(a, b) for other in inters[1:] for a, b in zip(inters[0], other))
     assert torch.equal(got[0], got[1])
-    d = (got[0].float() - got[2].float()).abs()
-    # P and the result are rounded to bf16 in both (2^-9 relative each); |v| stays below 6
-    assert torch.isfinite(d).all() and d.max() <= 5e-2 and d.mean() <= 2e-3
+    if call == "mean":
+        scale = MeanPooling_prefill(q, k, v.abs(), block, segment, 0.7, attn_impl="simt")
+    else:
+        scale = permuted_block_sparse_attn_fwd(q, k, v.abs(), block, segment, 0.7, True, attn_impl="simt")
+    _same_but_for_rounding(got[0], got[2], scale)
 
 
 # the result over K or V, whole or shifted by rows, and a second copy of the result over V
@@ -98,9 +107,8 @@ def test_stages_after_a_call_work_on_its_keys_and_values(call):
         want = fn(q, k, v, *args, intermediates=inter)
         assert inter["plan"] is plan
         plan.attn_fwd(q, again, "simt")
-        d = (again.float() - want.float()).abs()
-        # P and the result are rounded to bf16 in both (2^-9 relative each); |v| stays below 6
-        assert torch.isfinite(d).all() and d.max() <= 5e-2 and d.mean() <= 2e-3
+        _same_but_for_rounding(again, want, fn(q, k, v.abs(), *args, attn_impl="simt"))
+        fn(q, k, v, *args, intermediates=inter)
         assert torch.equal(plan.perm_k, k.repeat_interleave(2, dim=1)) and torch.equal(plan.perm_v, v.repeat_interleave(2, dim=1))
     fn(*inputs[0], *args)
     plan.segment_permute(inputs[0][1], inputs[0][2], identity=True)
