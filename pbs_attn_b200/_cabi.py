@@ -47,6 +47,7 @@ class Options(C.Structure):
                 ("key_pool_mode", C.c_int32), ("attn_impl", C.c_int32), ("no_permutation", C.c_int32),
                 ("diagonal_candidates", C.c_int32), ("no_own_segment", C.c_int32), ("kv_in_place", C.c_int32),
                 ("out_replicas", C.POINTER(OutReplicas))]
+    reads_kv_in_place = False       # the host's note beside kv_in_place: a call of this plan may make use of it
 
 
 Strides4 = C.c_int64 * 4

@@ -152,9 +152,11 @@ class Plan:
             thr = float(threshold)
         opt = _cabi.Options(thr_ptr, thr, select_all, int(bool(force_select_first_block)),
                             _cabi.POOL[query_pool_mode], _cabi.POOL[key_pool_mode], _cabi.ATTN_IMPL[attn_impl],
-                            int(bool(no_permutation)), int(bool(diagonal_candidates)), int(bool(no_own_segment)), int(bool(kv_in_place)),
+                            int(bool(no_permutation)), int(bool(diagonal_candidates)), int(bool(no_own_segment)), kv_in_place,
                             C.pointer(out_replicas) if out_replicas is not None else None)
         opt._keep = out_replicas            # the struct must outlive the call
+        if kv_in_place and (no_permutation or self.dense) and self.dtype != torch.float32 and attn_impl != "simt":
+            opt.reads_kv_in_place = True
         return opt
 
     def check_status(self):
@@ -234,8 +236,7 @@ class Plan:
             _cabi.check(self.lib.pbs_prefill_fwd(C.byref(self.shape), _ptr(q), _strides(q), _ptr(k), _strides(k),
                                                  _ptr(v), _strides(v), _ptr(out), _strides(out), C.byref(opt),
                                                  C.byref(self.scratch), C.c_void_p(stream.cuda_stream)), "pbs_prefill_fwd")
-            self._kv_left_out = bool(opt.kv_in_place and (opt.no_permutation or self.dense) and self.dtype != torch.float32
-                                     and opt.attn_impl != _cabi.ATTN_IMPL["simt"])
+            self._kv_left_out = opt.reads_kv_in_place
             self._queue_status_copy(stream)
         return out
 
