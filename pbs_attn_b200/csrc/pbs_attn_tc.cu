@@ -232,7 +232,7 @@ struct Params {
   int bs;
   float scale_log2e;
   int32_t* status;
-  int32_t* queue;               // draws so far, zero before and after a launch; null: a CTA has one entry
+  int32_t* queue;               // draws so far, zero before and after a launch
   void* extra_out[PBS_MAX_OUT_REPLICAS];   // further destinations of the output (same strides), e.g. on peer GPUs
   int n_extra;
   unsigned long long wait_ns;   // limit of every device-side wait
@@ -299,7 +299,9 @@ struct Smem {
 // ---------------------------------------------------------------------------------------------
 // The kernel
 // ---------------------------------------------------------------------------------------------
-template <int DT, int D>
+// QUEUE: CTAs draw their work with the counter p.queue; else each has one entry.  Its own instance, because the test in the
+// kernel cost the whole-path call 0.1 to 0.5 %.
+template <int DT, int D, bool QUEUE>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                const __grid_constant__ CUtensorMap map_v, Params p) {
@@ -358,13 +360,13 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       uint32_t kc = 0, vc = 0, qc[2] = {0, 0};
       bool ok = true;
       const uint64_t pol_kv = l2_policy_evict_last(), pol_q = l2_policy_evict_first();
-      // The items of this CTA: its first queue entry is its own number, each further one (with a counter) is drawn while
+      // The items of this CTA: its first queue entry is its own number, each further one (of a queue) is drawn while
       // the entry before it is loaded.
       int q = (int)blockIdx.x, q_next = 0, j = 0;
       for (int it = 0, bh, g; ok; ++it) {
         const bool more = queue_item(p.work, q, j, bh, g);
         if (more && j == 0 && elect_one()) {
-          if (p.queue) {
+          if constexpr (QUEUE) {
             // one draw per entry of the queue; the last one leaves the counter at zero
             const int drawn = atomicAdd(p.queue, 1);
             if (drawn == entries(p.work) - 1) atomicExch(p.queue, 0);
@@ -829,7 +831,7 @@ int run_tc(const Dims& d, const void* q, Strides qs, const KvSource& kv, const i
   p.wait_ns = g_wait_ns.load(std::memory_order_relaxed);
   p.drop_arrive = g_drop_arrive.load(std::memory_order_relaxed);
   const int sm_count = device_sms();
-  auto kern = attn_tc_kernel<DT, D>;
+  auto kern = queue ? attn_tc_kernel<DT, D, true> : attn_tc_kernel<DT, D, false>;
   const int smem = Smem<D>::kTotal;
   cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (ce != cudaSuccess) return cuda_fail(ce, "attn_tc_kernel smem attribute");
