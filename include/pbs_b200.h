@@ -143,7 +143,7 @@ int64_t pbs_launch_count(void);
  * the GPU.  No counterpart in the reference. */
 int pbs_debug_set_attn_wait(int64_t wait_ns, int32_t drop_arrive);
 
-/* Diagnostic.  Stage 2b has two kernels that must give identical masks: a tiled one (16 q blocks per
+/* Diagnostic.  Stage 2b has two kernels that must give identical masks: a tiled one (16 or 8 q blocks per
  * CTA, cut found by bisection; used wherever it applies: up to 2048 blocks per row, pooled rows of 8,
  * 16 or 32 16-byte pieces) and the general one (one q block per CTA, full sort).  impl = 1 forces the
  * general kernel for later calls of this process, 0 restores the default.  The tests compare the two. */

@@ -5,8 +5,8 @@
 // fp32 accumulators.  There is no fp32 tensor-core path, so the bound is the fp32 FMA rate: 4*D FLOP per
 // (query, key) of the kept blocks.  One CTA = 32 query rows; a step = 64 keys of one kept block, brought in by
 // cp.async while the step before is computed (head_dim 64; at 128 two buffers would leave one CTA a SM).
-// 128 threads as 8 x 16: a thread owns 4 rows x 4 keys of S and 4 rows x D/16 columns of O, so 64 FMA pairs feed on
-// 8 shared-memory reads of 16 bytes, and the 16 lanes that share rows reduce them by shuffles and pass P through
+// 128 threads as 8 x 16: a thread owns 4 rows x 4 keys of S and 4 rows x D/16 columns of O, so 32 packed FMA pairs feed
+// on 8 shared-memory reads of 16 bytes, and the 16 lanes that share rows reduce them by shuffles and pass P through
 // shared memory without a block-wide barrier.  The products of two neighbouring head-dim elements go into two partial
 // sums (packed fp32 pairs), which are added at the end of the row.
 // Measured against pbs_attn_simt.cu's kernel (one row and 8 keys a thread, operands re-read for every FMA), 2048 tokens, block 64:
@@ -226,10 +226,10 @@ int run_fp32(const Dims& d, const void* q, Strides qs, const void* pk, const voi
 
 }  // namespace
 
-// Blocks must be whole steps, the row of kept blocks must fit beside two CTAs' tiles, and the grid's second dimension
-// holds the query tiles.
+// Blocks must be whole steps.  The 4096 blocks a row that the library takes at most keep the row of kept blocks (8 KB) beside
+// two CTAs' tiles and the query tiles within the grid's second dimension.
 bool attn_fp32_supported(const Dims& d, int dt) {
-  return dt == PBS_FP32 && (d.D == 64 || d.D == 128) && d.bs % FN == 0 && d.nb <= 8192 && (d.S + FM - 1) / FM <= 65535;
+  return dt == PBS_FP32 && (d.D == 64 || d.D == 128) && d.bs % FN == 0;
 }
 
 int launch_attn_fp32(const Dims& d, const void* q, Strides qs, const void* pk, const void* pv, const int32_t* idx,

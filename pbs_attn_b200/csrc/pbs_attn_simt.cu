@@ -4,9 +4,9 @@
 // :7-90,241-311): fp32 scores scaled by 1/sqrt(D), key visible iff its original position <= the
 // query's, online softmax in base 2, probabilities rounded to the input dtype before P.V, fp32
 // accumulators, output = acc / row sum.  It takes any dtype / block size / head dim the library
-// accepts and is the path for shapes the tcgen05 kernel does not cover (fp32 inputs, head dims other
-// than 64/128, block sizes other than 64/128); it also serves as an on-device cross-check of the
-// tcgen05 kernel in the tests.  One CTA per (32-row query tile, b, h); the block mask row of the
+// accepts and is the path for what the other two kernels do not cover (head dims other than 64/128, 16-bit
+// block sizes other than 64/128, fp32 block sizes that are not whole 64s); it also serves as an on-device
+// cross-check of those two in the tests.  One CTA per (32-row query tile, b, h); the block mask row of the
 // tile's query block decides which 32-key tiles are visited.
 #include "pbs_common.cuh"
 

@@ -21,7 +21,8 @@
 //               over), row sum, P_h written back over the first 32 columns of S_h as packed 16-bit
 //               pairs; final O / l epilogue to global through a per-warp transposition tile
 // K and V come through tensor maps of any strides with the query heads of a group on one head, so a call whose keys keep
-// their order needs no copy of them (a copy costs 97 us of 1.6 ms at 16384 tokens, and 19 of 57 us below one segment).
+// their order needs no copy of them (kernels of a call with and without, in turn: MeanPooling at 16384 tokens 1633 and 1564 us;
+// 187 tokens 30.3 and 14.4, where one set-up kernel takes the place of gather, mask and list kernels).
 // An issuer runs, per list entry and half h: O += P_h V_h, then S_h of the next entry into the
 // columns P_h vacated.  So while a softmax warpgroup works on one half, the MMAs of the other half
 // (and of the other query tile) run, and the next S is ready when the warpgroup comes back for it.

@@ -213,7 +213,7 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return r;
 }
 
-// x / z for a divisor used many times: reciprocal product corrected by one exact-remainder step (the
+// x / z for a divisor used many times: reciprocal product corrected by one exact-remainder step (Markstein 1990; the
 // correctly rounded quotient for all but a few divisors with an all-ones significand, where the result
 // may differ from it in the last bit).
 __device__ __forceinline__ float2 div_by(float2 x, float z, float rz) {
@@ -494,7 +494,7 @@ rowstats_kernel(const float2* __restrict__ partials, float2* __restrict__ rowsta
 // The same merge for few tiles, one warp per row with lane l holding running pair l.  Its loads are 8 bytes apart by
 // whole rows of statistics (neighbouring warps use the rest of the sectors), which only pays while there is a load or
 // four per lane; the kernel above spends that time on handing pairs round a 1024-thread block: 128 heads x 128 rows
-// of 32 tiles 10.8 us there, 8.1 here; at 128 tiles both take the same.
+// of 32 tiles 10.9 us there, 8.5 here (ncu, means of two launches); at 128 tiles both take the same.
 __global__ void __launch_bounds__(256)
 rowstats_few_kernel(const float2* __restrict__ partials, float2* __restrict__ rowstats, int ntile, int bs) {
   const int bh = blockIdx.y, lane = threadIdx.x & 31;

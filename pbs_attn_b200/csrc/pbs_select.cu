@@ -518,8 +518,8 @@ tile_list_kernel(const uint8_t* __restrict__ mask, uint32_t* __restrict__ list, 
 
 // Everything the attention kernel needs for plain causal attention over keys in original order: identity order, all
 // blocks on, and the tile lists.  Key tiles above the diagonal are left out of the lists and only the diagonal one is
-// masked by element (with block_size 64 all four sub-blocks are on).  One CTA per (b, h); a few hundred bytes each, so
-// the launch is what it costs: it takes the place of three (gather of K and V, mask, lists) and of the copy of K and V.
+// masked by element (with block_size 64 all four sub-blocks are on).  One CTA per (b, h), which writes 4 S + nb^2 bytes
+// and the lists: 0.8 KB at 187 tokens, 22 KB at 4096 with block 64, so the launch is most of what it costs (2.6 us): it takes the place of three (gather of K and V, mask, lists) and of the copy of K and V.
 __global__ void __launch_bounds__(128)
 dense_setup_kernel(int32_t* __restrict__ idx, int32_t* __restrict__ first_block, uint8_t* __restrict__ mask,
                    uint32_t* __restrict__ list, int32_t* __restrict__ count, int32_t* __restrict__ status, int S, int bs, int nb) {
