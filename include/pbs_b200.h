@@ -136,9 +136,9 @@ int pbs_version(void);
 int64_t pbs_launch_count(void);
 
 /* Diagnostic.  Every device-side wait of the tcgen05 attention kernel is bounded; wait_ns sets the
- * bound for later launches of this process (0 restores the default of 2 s).  drop_arrive = 1 makes
- * the first softmax warpgroup of CTA 0 withhold one barrier arrive, so that exactly one wait runs
- * out: the kernel then returns with status[0] != 0 instead of a result.  The failure-path test uses
+ * bound for later launches of this process (0 restores the default of 2 s).  drop_arrive = n makes
+ * the first softmax warpgroup of CTA 0 (pbs_attn_fwd: of each of the first n CTAs) withhold one barrier arrive, so that one wait
+ * runs out there: the kernel then returns with status[0] != 0 instead of a result.  The failure-path tests use
  * this (with a bound of a few milliseconds) to exercise the abort path without faulting or hanging
  * the GPU.  No counterpart in the reference. */
 int pbs_debug_set_attn_wait(int64_t wait_ns, int32_t drop_arrive);
@@ -227,8 +227,9 @@ int pbs_build_tile_lists(const pbs_shape_t* shape, const uint8_t* block_mask,
  * pbs_attn/src/pbs.py:191-193, so the inverse permutation is the identity and is folded
  * into the store).  Replaces the launch at pbs_attn/src/pbs.py:220-246 of the kernel
  * pbs_attn/src/kernels/permuted_block_sparse_attention.py:134-311.
- * status: 8 int32 words, zero on entry; word 0 becomes non-zero if a bounded device-side
- * wait ran out (the output is then invalid).  out_replicas: NULL or extra destinations. */
+ * status: 8 int32 words, word 0 zero on entry; it becomes non-zero if a bounded device-side
+ * wait ran out (the output is then invalid, and that of a launch that shares the words and still runs).
+ * out_replicas: NULL or extra destinations. */
 int pbs_attn_fwd(const pbs_shape_t* shape,
                  const void* q, const int64_t q_strides[4],
                  const void* perm_k, const void* perm_v, const int32_t* key_indices,

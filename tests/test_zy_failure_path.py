@@ -53,3 +53,33 @@ def test_a_wait_that_runs_out_is_reported_and_the_next_call_is_correct():
     torch.cuda.synchronize()
     plan.check_status()
     assert torch.equal(again, good)
+
+
+def test_a_stage_call_of_many_ctas_ends_soon_after_the_first_gave_up():
+    """The stage call starts a CTA per share of the work, some 1300 here or nine a SM.  An arrive is withheld in every one: those
+    that start after another gave up do not wait out the limit as well."""
+    from pbs_attn_b200.prefill import Plan
+    lib = _cabi.load()
+    w = Workload("abort", 1, 32, 8, 128, 16384, "bf16", 128, 256, 0.9, 5e5, sinks=4)
+    q, k, v = make_qkv(w, seed=78, device="cuda")
+    plan = Plan(1, 32, 8, 16384, 128, 128, 256, q.dtype, q.device)
+    good = plan.run(q, k, v, torch.empty_like(q), plan.options(0.9, attn_impl="tcgen05"))
+    plan.check_status()
+    out = torch.empty_like(q)
+    start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    try:
+        assert lib.pbs_debug_set_attn_wait(10_000_000, 1 << 30) == 0     # 10 ms bound
+        start.record()
+        plan.attn_fwd(q, out, "tcgen05")
+        end.record()
+        torch.cuda.synchronize()
+    finally:
+        assert lib.pbs_debug_set_attn_wait(0, 0) == 0
+    assert plan.status[0] != 0
+    print("ms until the launch ended:", start.elapsed_time(end))
+    assert start.elapsed_time(end) < 50                              # nine limits are 90
+    with pytest.raises(_cabi.PbsError):
+        plan.check_status()
+    plan.attn_fwd(q, out, "tcgen05")
+    plan.check_status()
+    assert torch.equal(out, good)
