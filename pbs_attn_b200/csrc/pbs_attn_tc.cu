@@ -8,25 +8,38 @@
 // Work item = 256 consecutive queries of one (b, h): two 128-row query tiles that share every K/V
 // tile staged in shared memory.  The item's tile list (built by tile_list_kernel) names the 128-key
 // tiles that either query tile selected.  A persistent CTA (one per SM) draws its items from a queue
-// (in the stage call a CTA takes one entry of it) and walks them with twelve warps in four roles:
-//   warp 0      draws the items and tells the other roles; TMA producer: Q tiles, then K and V tiles of the list
-//               into two 2-deep rings
+// (in the stage call a CTA takes one entry of it) and walks them with twenty warps in four roles:
+//   warp 0      draws the items and tells the other roles; TMA producer: Q tiles, then the list's tiles into a ring of two
+//               stages, each with the V tile of an entry and the K tile of the next one (the issuers need these together)
 //   warps 1, 3  MMA issuers, one per query tile.  A 128-key tile is two half-steps of 64 keys with
 //               their own 64 TMEM columns: S_h = Q K_h^T (SS, both operands K-major, 128B swizzle,
 //               M=128 N=64) and O += P_h V_h (TS: P_h read from TMEM, V MN-major from shared memory)
 //   warp 2      owns the TMEM allocation (all 512 columns: per query tile S_0 S_1 (64 each) and O (128))
-//   warps 4-7   softmax of query tile 0: per half-step tcgen05.ld S_h, mask, exp2 relative to the row
-//   warps 8-11  softmax of query tile 1  maximum in use (the new maximum is computed beside it and only a
-//               row that outgrew the lazy-rescale threshold makes the warp rescale O in TMEM and start
-//               over), row sum, P_h written back over the first 32 columns of S_h as packed 16-bit
-//               pairs; final O / l epilogue to global through a per-warp transposition tile
+//   warps 4-19  softmax, a warpgroup per query tile and key half: per half-step tcgen05.ld S_h, exp2 relative to the row's
+//               reference, row sum, P_h written back over the first 32 columns of S_h as packed 16-bit pairs.  The
+//               first half's warpgroup also divides O by the row sum and stores it through a transposition tile
 // K and V come through tensor maps of any strides with the query heads of a group on one head, so a call whose keys keep
 // their order needs no copy of them (kernels of a call with and without, in turn: MeanPooling at 16384 tokens 1633 and 1564 us;
 // 187 tokens 30.3 and 14.4, where one set-up kernel takes the place of gather, mask and list kernels).
 // An issuer runs, per list entry and half h: O += P_h V_h, then S_h of the next entry into the
-// columns P_h vacated.  So while a softmax warpgroup works on one half, the MMAs of the other half
-// (and of the other query tile) run, and the next S is ready when the warpgroup comes back for it.
-// One issuer's barrier bookkeeping overlaps the other issuer's MMAs.
+// columns P_h vacated.  One issuer's barrier bookkeeping overlaps the other issuer's MMAs.
+//
+// What bounds it.  TMEM has no room for a second S, so each of the four (query tile, key half) chains S -> P -> P V -> next S
+// is serial, and its latency is what counts: about 1300 cycles of softmax and as many of MMAs and hand-overs, while
+// the tensor pipe needs 2560 cycles for the four (K = 16 of S at N = 64 takes 48 cycles and not 32, because shared memory
+// delivers 128 bytes a cycle) and the special-function units 2048.  With one softmax warpgroup per query tile for both halves, as
+// it was, a scheduler had two such warps, in step with each other more often than not, and the exponentials of one waited for the
+// other's; with four there is nearly always one to run.  Measured (attention alone, in turn, 0.25 s blocks): 4 x 2048
+// tokens 217 -> 198 us, 6001 sparse tokens fp16 243 -> 214, head_dim 64 382 -> 313, 8192 tokens 557 -> 527, block_size 64 at 32768
+// tokens 7245 -> 6816, 32768 sparse tokens 4325 -> 3693, four heads at 131072 tokens 14255 -> 13800 (power cap).
+// Three things make four warpgroups pay, each of which alone decides between a gain and a loss:
+//  - the warps of the two halves exchange nothing from step to step.  A row's reference is not its running maximum
+//    but what its first tile gave; it is raised only when a half-step's sum leaves kSumMost, which for bf16 (the range of fp32) hardly
+//    ever happens.  All of that protocol (raise_refs, before_exp) is out of line.  With a check between the halves in every
+//    half-step (a poll, an order of the hand-overs) the kernel was slower than before: 3200 to 3500 cycles a step against 2850.
+//  - registers: 96 a thread at 640 threads, 104 after the issuing warps have given some up.  S is read in two parts of 32
+//    columns; read at once it spills (2 % slower), in parts of 16 or with a part ahead it is slower too.
+//  - nothing that does not need S stands between the wait for S and the arrive on P.
 // Every wait on an mbarrier is bounded (2 s unless pbs_debug_set_attn_wait says otherwise); when one
 // runs out the CTA raises a flag, all roles leave their loops, in-flight copies and MMAs are waited
 // out (bounded), TMEM is freed and status[0] tells the host which wait it was.
@@ -40,12 +53,17 @@
 namespace pbs {
 namespace {
 
-constexpr int kThreads = 384;
-constexpr int NK = 2;                     // K ring depth
-constexpr int NV = 2;                     // V ring depth
+constexpr int kThreads = 640;
+constexpr int kRing = 2;                  // stages of a V tile and the next list entry's K tile
 constexpr int kSched = 4;                 // items the producer may be ahead of the slowest role
 constexpr uint32_t kTmemCols = 512;
-constexpr float kRescaleThreshold = 8.f;  // log2 units: O is rescaled only when the max grows by more
+// A half-step's probabilities are taken as they are while their sum per row is no larger than this: the reference of the
+// exponents need not be the row maximum, only near enough that nothing leaves the range of the 16-bit type (fp16: 65504).
+template <int DT> constexpr float kSumMost = DT == PBS_FP16 ? 0x1p15f : 0x1p60f;
+template <int DT> constexpr float kUpLeast = DT == PBS_FP16 ? 9.f : 54.f;   // log2(kSumMost / 64): a larger sum of 64 has a score above it
+// Registers a thread: the four warps that only issue give up part of what the launch has.
+constexpr int kRegsLaunch = 96, kRegsIssue = 64, kRegsSoftmax = 104;
+static_assert(128 * kRegsIssue + 512 * kRegsSoftmax <= kThreads * kRegsLaunch, "the shares must fit what the launch has");
 
 // ---------------------------------------------------------------------------------------------
 // PTX wrappers
@@ -174,6 +192,17 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
         "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
+        "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
+        "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+      : "memory");
+}
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
@@ -191,21 +220,38 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 }
 __device__ __forceinline__ float ex2(float x) {
   float r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
 
+// Two probabilities as the MMA takes them; `add` sums them up in fp32.  The row sum is that of the rounded probabilities, so that where
+// few of them matter the rounding cancels in O / l: error of a call against 64 bits 2.25e-3 -> 2.23e-3 at 32768 sparse tokens,
+// 2.30e-3 with the sum of the unrounded ones and this kernel's references (which need not be the row maximum).
 template <int DT> struct PackP;
 template <> struct PackP<PBS_BF16> {
   static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
   }
+  static __device__ __forceinline__ void add(float2& a, uint32_t w) {
+    asm("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %2;\n\tadd.rn.f32.bf16 %0, lo, %0;\n\tadd.rn.f32.bf16 %1, hi, %1;\n\t}" : "+f"(a.x), "+f"(a.y) : "r"(w));
+  }
+  static __device__ __forceinline__ uint32_t scale(uint32_t w, float by) {
+    const float2 x = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&w));
+    return pack(x.x * by, x.y * by);
+  }
 };
 template <> struct PackP<PBS_FP16> {
   static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
     __half2 v = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
+  }
+  static __device__ __forceinline__ void add(float2& a, uint32_t w) {
+    asm("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %2;\n\tadd.rn.f32.f16 %0, lo, %0;\n\tadd.rn.f32.f16 %1, hi, %1;\n\t}" : "+f"(a.x), "+f"(a.y) : "r"(w));
+  }
+  static __device__ __forceinline__ uint32_t scale(uint32_t w, float by) {
+    const float2 x = __half22float2(*reinterpret_cast<__half2*>(&w));
+    return pack(x.x * by, x.y * by);
   }
 };
 
@@ -214,9 +260,10 @@ template <> struct PackP<PBS_FP16> {
 // ---------------------------------------------------------------------------------------------
 struct Bars {
   uint64_t q_full[2], q_empty[2];
-  uint64_t k_full[NK], k_empty[NK];
-  uint64_t v_full[NV], v_empty[NV];
+  uint64_t kv_full[kRing], kv_empty[kRing];
   uint64_t s_full[2][2], p_full[2][2], o_full[2][2];   // [query tile][key half]
+  uint64_t l_full[2][4];                                // [query tile][lane quarter] row sums of the second key half are in lsum
+  uint64_t start[2][4];                                 // [query tile][lane quarter] first maxima of both halves are in smax
   uint64_t item_full[kSched], item_empty[kSched];
   uint64_t drain;                                       // teardown after an abort: both issuers' MMAs retired
 };
@@ -244,20 +291,50 @@ struct Ctl {
   int2 item[kSched];            // (b, h) and query group of the items handed to the other roles; x < 0: no more
   uint32_t tmem_base;
   volatile int abort_flag;
+  // Shared by the two softmax warps (one per key half) of a query tile's lane quarter, see raise_refs:
+  uint2 post[2][2][4];          // [query tile][key half][lane quarter] progress, epoch of the references that its last P refers to
+  uint32_t epoch[2][4];         // [query tile][lane quarter] times the references were raised
+  float ref[2][2][128];         // [epoch & 1][query tile] references when they were raised last: the partner may still be reading the ones before
+  float smax[2][2][2][128];     // [entry & 1][query tile][key half] first maxima
+  uint32_t starts[2][2][4];     // [query tile][key half][lane quarter] meetings so far
+  float lsum[2][128], lref[2][128];   // row sums of an item's second key half, and the references they are relative to
   unsigned long long wait_ns;
+  int32_t* status;
 };
 
+template <int D>
+struct Smem {
+  static constexpr int kTileBytes = 128 * D * 2;          // one 128-row tile
+  static constexpr int kQ = 0;                            // 2 tiles
+  static constexpr int kV = kQ + 2 * kTileBytes;          // per stage a V tile and a K tile
+  static constexpr int kK = kV + kTileBytes;
+  static constexpr int kStage = 2 * kTileBytes;
+  static constexpr int kEnd = kV + kRing * kStage;
+};
+constexpr int kStageRow = 80;                             // bytes per staged row piece (64 of data + 16 of padding)
+// What does not depend on head_dim lies in front, at addresses known to the compiler.
+struct __align__(1024) Front {
+  Bars bars;
+  Ctl ctl;
+  alignas(16) int32_t kidx[16][64];                                   // key positions of a masked half tile, per softmax warp
+  alignas(16) unsigned char stage[8][32 * kStageRow];                 // epilogue transposition, per lane quarter of a query tile
+};
+extern __shared__ __align__(1024) unsigned char smem_dyn[];
+__device__ __forceinline__ Front& front() { return *reinterpret_cast<Front*>(smem_dyn); }
+template <int D> constexpr int kSmemBytes = (int)sizeof(Front) + Smem<D>::kEnd;
+
 // Bounded wait: false when the CTA is aborting (this wait or another one ran out of time).
-__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, Ctl* ctl, int32_t* status, int code) {
+__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, int code) {
   if (mbar_try_wait(bar, parity)) return true;
   const uint64_t t0 = global_timer_ns();
   for (uint32_t it = 1;; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((it & 63u) == 0u) {
-      if (ctl->abort_flag) return false;
-      if (global_timer_ns() - t0 > ctl->wait_ns) {
-        ctl->abort_flag = 1;
-        atomicCAS(status, 0, code);
+      Ctl& ctl = front().ctl;
+      if (ctl.abort_flag) return false;
+      if (global_timer_ns() - t0 > ctl.wait_ns) {
+        ctl.abort_flag = 1;
+        atomicCAS(ctl.status, 0, code);
         return false;
       }
     }
@@ -265,15 +342,226 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, Ctl* ctl
 }
 
 // The same for a whole converged warp: every lane polls, the verdict is made warp-uniform.
-__device__ __forceinline__ bool wait_bar_warp(uint32_t bar, uint32_t parity, Ctl* ctl, int32_t* status, int code) {
-  return __all_sync(0xffffffffu, wait_bar(bar, parity, ctl, status, code));
+__device__ __forceinline__ bool wait_bar_warp(uint32_t bar, uint32_t parity, int code) {
+  return __all_sync(0xffffffffu, wait_bar(bar, parity, code));
+}
+
+// Most waits pass at once: the rest is kept out of the hot loops' instruction stream.
+__device__ __noinline__ bool wait_slow(uint32_t bar, uint32_t parity, int code) {
+  return wait_bar_warp(bar, parity, code);
+}
+__device__ __forceinline__ bool wait_hot(uint32_t bar, uint32_t parity, int code) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return wait_slow(bar, parity, code);
+}
+
+// The 64 scores of this thread's row, in TMEM: those of keys after the query become -inf.
+__device__ __noinline__ void mask_half(uint32_t s_addr, const int32_t* kidx, int qpos) {
+#pragma unroll 1
+  for (int c = 0; c < 64; c += 16) {
+    uint32_t r[16];
+    tmem_ld16(s_addr + c, r);
+    tmem_wait_ld();
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int4 k = *reinterpret_cast<const int4*>(kidx + c + 4 * j);
+      if (k.x > qpos) r[4 * j] = 0xff800000u;
+      if (k.y > qpos) r[4 * j + 1] = 0xff800000u;
+      if (k.z > qpos) r[4 * j + 2] = 0xff800000u;
+      if (k.w > qpos) r[4 * j + 3] = 0xff800000u;
+    }
+    tmem_st16(s_addr + c, r);
+  }
+  tmem_wait_st();
+}
+
+// This thread's row of O, in TMEM, times alpha.
+__device__ __noinline__ void rescale_o(uint32_t o_addr, float alpha, int columns) {
+#pragma unroll 1
+  for (int c = 0; c < columns; c += 16) {
+    uint32_t o[16];
+    tmem_ld16(o_addr + c, o);
+    tmem_wait_ld();
+#pragma unroll
+    for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * alpha);
+    tmem_st16(o_addr + c, o);
+  }
+}
+
+// P_h of this thread's row, in TMEM as packed pairs, times a power of two.
+template <int DT>
+__device__ __noinline__ void scale_p(uint32_t p_addr, float alpha) {
+#pragma unroll 1
+  for (int c = 0; c < 32; c += 16) {
+    uint32_t r[16];
+    tmem_ld16(p_addr + c, r);
+    tmem_wait_ld();
+#pragma unroll
+    for (int j = 0; j < 16; ++j) r[j] = PackP<DT>::scale(r[j], alpha);
+    tmem_st16(p_addr + c, r);
+  }
+}
+
+// Waits (bounded) until a warp's progress is at least `least`.
+__device__ __noinline__ bool wait_post(uint32_t addr, uint32_t least, uint2& post, int code) {
+  Ctl& ctl = front().ctl;
+  const uint64_t t0 = global_timer_ns();
+  for (uint32_t it = 1;; ++it) {
+    asm volatile("ld.volatile.shared.v2.u32 {%0, %1}, [%2];" : "=r"(post.x), "=r"(post.y) : "r"(addr) : "memory");
+    if (__all_sync(0xffffffffu, post.x >= least)) return true;
+    if ((it & 63u) == 0u && __any_sync(0xffffffffu, ctl.abort_flag || global_timer_ns() - t0 > ctl.wait_ns)) {
+      ctl.abort_flag = 1;
+      atomicCAS(ctl.status, 0, code);
+      return false;
+    }
+  }
+}
+
+// Largest of the 64 scores of this thread's row, in TMEM.
+__device__ __forceinline__ float row_max64(uint32_t s_addr) {
+  float m = -CUDART_INF_F;
+#pragma unroll
+  for (int c = 0; c < 64; c += 32) {
+    uint32_t r[32];
+    tmem_ld32(s_addr + c, r);
+    tmem_wait_ld();
+    float a = m, b = m;
+#pragma unroll
+    for (int j = 0; j < 32; j += 4) {
+      a = max3(a, __uint_as_float(r[j]), __uint_as_float(r[j + 1]));
+      b = max3(b, __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
+    }
+    m = fmaxf(a, b);
+  }
+  return m;
+}
+
+// The references of a softmax warp's rows.  Both warps of a lane quarter (one per key half) use the same; `ref` is log2 of the factor
+// that the row's P, sum and O lack, -inf where the row has seen no key yet (then 0 is used, and everything is zero so far).
+struct Refs {
+  float ref, l;                                            // of this lane's row; l: row sum of this key half
+  uint32_t epoch;                                          // times they were raised; kFresh: some row has none yet; kGiveUp: a wait ran out
+};
+constexpr uint32_t kFresh = 0x80000000u, kGiveUp = 0xffffffffu;
+// A warp's progress (Ctl::post): 3 * list entries done, and more while it is in one of the functions below.
+constexpr uint32_t kAtStart = 1, kRaising = 2;
+__device__ __forceinline__ void st_post(uint32_t addr, uint32_t progress, uint32_t epoch) {
+  asm volatile("st.volatile.shared.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(progress), "r"(epoch) : "memory");
+}
+
+struct Who {                                               // of this softmax warp: query tile, key half, lane quarter; its lane's row
+  int i, hs, wq, lane, row;
+};
+__device__ __forceinline__ Who who() {
+  const int w = (int)(threadIdx.x >> 5) - 4, lane = threadIdx.x & 31;
+  return Who{w >> 3, (w >> 2) & 1, w & 3, lane, (w & 3) * 32 + lane};
+}
+
+// Takes over references that the partner warp has raised.
+__device__ __forceinline__ void refresh(Refs& r, const Who& w) {
+  const uint32_t now = *const_cast<const volatile uint32_t*>(&front().ctl.epoch[w.i][w.wq]);
+  if (__any_sync(0xffffffffu, now != r.epoch)) {
+    const float ref = *const_cast<const volatile float*>(&front().ctl.ref[now & 1u][w.i][w.row]);
+    if (ref != r.ref && r.l > 0.f) r.l *= ex2(r.ref - ref);
+    r.ref = ref;
+    r.epoch = now;
+  }
+}
+
+// Before the exponentials of a half-step whose keys are masked by position, or while some row has no reference: its first one is
+// its largest score in both halves of the first tile that has one, so that the two warps meet here.
+__device__ __noinline__ Refs before_exp(Refs r, uint32_t ent, uint32_t tmem, uint32_t sc, bool none, bool first_entry, int qpos, float scale_log2e) {
+  const Who w = who();
+  Ctl& ctl = front().ctl;
+  const uint32_t s_addr = tmem + ((uint32_t)(w.wq * 32) << 16) + 128 * w.i + 64 * w.hs;
+  if (!none && (ent & (1u << (18 + w.i)))) mask_half(s_addr, front().kidx[(threadIdx.x >> 5) - 4], qpos);
+  if (!(r.epoch & kFresh)) return r;
+  // An item's first S was issued after all of the item before: nobody raises anything until both are past this meeting.
+  r.epoch = first_entry ? *const_cast<volatile uint32_t*>(&ctl.epoch[w.i][w.wq]) : r.epoch & ~kFresh;
+  const float mine = none ? -CUDART_INF_F : row_max64(s_addr) * scale_log2e;
+  if (w.lane == 0) st_post(smem_u32(&ctl.post[w.i][w.hs][w.wq]), 3u * sc + kAtStart, 0u);
+  volatile float* both = &ctl.smax[sc & 1u][w.i][0][w.row];
+  both[128 * w.hs] = mine;
+  __threadfence_block();
+  __syncwarp();
+  const uint32_t bar = smem_u32(&front().bars.start[w.i][w.wq]);
+  volatile uint32_t* starts = &ctl.starts[w.i][w.hs][w.wq];
+  if (elect_one()) mbar_arrive(bar);
+  if (!wait_bar_warp(bar, *starts & 1u, 14)) { r.epoch = kGiveUp; return r; }
+  __syncwarp();
+  if (w.lane == 0) *starts = *starts + 1u;
+  __syncwarp();
+  if (!first_entry) refresh(r, w);
+  if (r.ref == -CUDART_INF_F) r.ref = fmaxf(mine, both[128 * (w.hs ^ 1)]);
+  if (__any_sync(0xffffffffu, r.ref == -CUDART_INF_F)) r.epoch |= kFresh;
+  return r;
+}
+
+// A half-step k found the references of another epoch, or a sum above kSumMost with them.  S_k is still in TMEM, and since
+// P_k has not been handed over, neither P V of k nor of the partner's k + 1 can start: whoever raises references has O and P_{k+1}
+// to itself.  Raising waits for the P V of k - 1, which the old references belong to, publishes the new ones, scales O, and then
+// looks at k + 1.  Its warp reads the epoch after it has seen its S: if that S is not there yet it will see the new one.  Otherwise
+// its progress says when it is through: with the old epoch its P_{k+1} is scaled here (by a power of two) and its sum by itself once it
+// sees the epoch; or it waits for the P V of k to raise references of its own, and reads the epoch after that.
+template <int DT, int D>
+__device__ __noinline__ Refs raise_refs(Refs r, uint32_t tmem, uint32_t sc, bool first_entry, float scale_log2e) {
+  const Who w = who();
+  Bars& bars = front().bars;
+  Ctl& ctl = front().ctl;
+  const uint32_t fresh = r.epoch & kFresh;
+  r.epoch &= ~kFresh;
+  const uint32_t before = w.hs == 0 ? sc - 1u : sc, after = w.hs == 0 ? sc : sc + 1u;   // entries of half-steps k - 1 and k + 1
+  const uint32_t lanes = (uint32_t)(w.wq * 32) << 16, s_addr = tmem + lanes + 128 * w.i + 64 * w.hs;
+  const float top = row_max64(s_addr) * scale_log2e;
+  refresh(r, w);
+  if (__any_sync(0xffffffffu, top > r.ref + kUpLeast<DT>)) {
+    if (w.lane == 0) st_post(smem_u32(&ctl.post[w.i][w.hs][w.wq]), 3u * sc + kRaising, r.epoch);
+    const bool have_o = !first_entry || w.hs == 1;
+    if (have_o) {
+      if (!wait_bar_warp(smem_u32(&bars.o_full[w.i][w.hs ^ 1]), before & 1u, 10)) { r.epoch = kGiveUp; return r; }
+      tc_fence_after();
+      refresh(r, w);
+    }
+    const bool up = top > r.ref + kUpLeast<DT>;
+    if (__any_sync(0xffffffffu, up)) {
+      const float old = r.ref;
+      if (up) r.ref += ceilf(top - r.ref);
+      const float alpha = up ? ex2(old - r.ref) : 1.f;
+      r.l *= alpha;
+      ++r.epoch;
+      *const_cast<volatile float*>(&ctl.ref[r.epoch & 1u][w.i][w.row]) = r.ref;
+      __threadfence_block();
+      __syncwarp();
+      if (w.lane == 0) *const_cast<volatile uint32_t*>(&ctl.epoch[w.i][w.wq]) = r.epoch;
+      __threadfence_block();
+      __syncwarp();
+      if (have_o) rescale_o(tmem + lanes + 256 + 128 * w.i, alpha, D);
+      if (__all_sync(0xffffffffu, mbar_try_wait(smem_u32(&bars.s_full[w.i][w.hs ^ 1]), after & 1u))) {
+        // (a first half has met the second one of its entry already)
+        uint2 theirs;
+        if (!wait_post(smem_u32(&ctl.post[w.i][w.hs ^ 1][w.wq]), 3u * after + (w.hs == 0 ? kRaising : kAtStart), theirs, 16)) {
+          r.epoch = kGiveUp;
+          return r;
+        }
+        if (theirs.x >= 3u * (after + 1u) && theirs.y != r.epoch) {
+          tc_fence_after();
+          scale_p<DT>(tmem + lanes + 128 * w.i + 64 * (w.hs ^ 1), alpha);
+        }
+      }
+      tmem_wait_st();
+    }
+  }
+  r.epoch |= fresh;
+  return r;
 }
 
 // The n-th item of this CTA, for the roles that the producer feeds (a whole converged warp calls it).
 // False past the last one, or when a wait ran out (then ok is false).
-__device__ __forceinline__ bool next_item(int n, Bars* bars, Ctl* ctl, int32_t* status, bool& ok, int& bh, int& g) {
+__device__ __forceinline__ bool next_item(int n, bool& ok, int& bh, int& g) {
   const int s = n % kSched;
-  ok = wait_bar_warp(smem_u32(&bars->item_full[s]), (n / kSched) & 1u, ctl, status, 12);
+  Bars* bars = &front().bars;
+  Ctl* ctl = &front().ctl;
+  ok = wait_bar_warp(smem_u32(&bars->item_full[s]), (n / kSched) & 1u, 12);
   if (!ok) return false;
   const int2 it = ctl->item[s];
   __syncwarp();
@@ -282,20 +570,6 @@ __device__ __forceinline__ bool next_item(int n, Bars* bars, Ctl* ctl, int32_t* 
   g = it.y;
   return bh >= 0;
 }
-
-template <int D>
-struct Smem {
-  static constexpr int kTileBytes = 128 * D * 2;          // one 128-row tile
-  static constexpr int kQ = 0;                            // 2 tiles
-  static constexpr int kK = kQ + 2 * kTileBytes;          // NK tiles
-  static constexpr int kV = kK + NK * kTileBytes;         // NV tiles
-  static constexpr int kIdx = kV + NV * kTileBytes;       // 8 warps x 128 int32
-  static constexpr int kStage = kIdx + 8 * 128 * 4;       // 8 warps x 32 rows x (64 + 16) bytes: epilogue transposition
-  static constexpr int kStageRow = 80;                    // bytes per staged row piece (64 of data + 16 of padding)
-  static constexpr int kBars = kStage + 8 * 32 * kStageRow;
-  static constexpr int kCtl = kBars + (int)sizeof(Bars);
-  static constexpr int kTotal = kCtl + (int)sizeof(Ctl) + 1024;   // + slack for 1024-byte alignment
-};
 
 // ---------------------------------------------------------------------------------------------
 // The kernel
@@ -309,11 +583,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   using E = Elem<DT>;
   using T = typename E::T;
   using SM = Smem<D>;
-  extern __shared__ unsigned char smem_dyn[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
-  const uint32_t sbase = smem_u32(smem);
-  Bars* bars = reinterpret_cast<Bars*>(smem + SM::kBars);
-  Ctl* ctl = reinterpret_cast<Ctl*>(smem + SM::kCtl);
+  const uint32_t sbase = smem_u32(smem_dyn) + (uint32_t)sizeof(Front);
+  Bars* bars = &front().bars;
+  Ctl* ctl = &front().ctl;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -326,14 +598,21 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         mbar_init(smem_u32(&bars->o_full[i][h]), 1);
       }
     }
-    for (int i = 0; i < NK; ++i) { mbar_init(smem_u32(&bars->k_full[i]), 1); mbar_init(smem_u32(&bars->k_empty[i]), 2); }
-    for (int i = 0; i < NV; ++i) { mbar_init(smem_u32(&bars->v_full[i]), 1); mbar_init(smem_u32(&bars->v_empty[i]), 2); }
-    for (int i = 0; i < kSched; ++i) { mbar_init(smem_u32(&bars->item_full[i]), 1); mbar_init(smem_u32(&bars->item_empty[i]), 10); }
+    for (int i = 0; i < kRing; ++i) { mbar_init(smem_u32(&bars->kv_full[i]), 1); mbar_init(smem_u32(&bars->kv_empty[i]), 2); }
+    for (int i = 0; i < kSched; ++i) { mbar_init(smem_u32(&bars->item_full[i]), 1); mbar_init(smem_u32(&bars->item_empty[i]), 18); }
+    for (int i = 0; i < 2; ++i)
+      for (int wq = 0; wq < 4; ++wq) {
+        mbar_init(smem_u32(&bars->l_full[i][wq]), 1);
+        mbar_init(smem_u32(&bars->start[i][wq]), 2);
+        ctl->epoch[i][wq] = 0u;
+        for (int h = 0; h < 2; ++h) { ctl->post[i][h][wq] = make_uint2(0u, 0u); ctl->starts[i][h][wq] = 0u; }
+      }
     mbar_init(smem_u32(&bars->drain), 2);
     // Without a queue a CTA that starts after another one gave up need not wait out the limit as well (the result is invalid
     // already): its waits give up at once, so that a launch of many CTAs ends soon after the first of them.
     ctl->abort_flag = !QUEUE && blockIdx.x >= 1 && *const_cast<const volatile int32_t*>(p.status) != 0;
     ctl->wait_ns = p.wait_ns;
+    ctl->status = p.status;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 2) {
@@ -356,11 +635,13 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
   constexpr uint32_t kIdescPV = (1u << 4) | (kFmt << 7) | (kFmt << 10) | (1u << 16) | (((uint32_t)D >> 3) << 17) | ((128u >> 4) << 24);
 
 
+  if (warp < 4) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
   if (warp == 0) {
     // =========================================================================== TMA producer
     // The whole warp walks the lists (uniform control flow); one elected lane issues the copies.
     {
-      uint32_t kc = 0, vc = 0, qc[2] = {0, 0};
+      uint32_t rc = 0, qc[2] = {0, 0};
       bool ok = true;
       const uint64_t pol_kv = l2_policy_evict_last(), pol_q = l2_policy_evict_first();
       // The items of this CTA: its first queue entry is its own number, each further one (of a queue) is drawn while
@@ -378,7 +659,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             q_next = p.work.n_items;                       // past the end
           }
         }
-        ok = wait_bar_warp(smem_u32(&bars->item_empty[it % kSched]), ((it / kSched) & 1u) ^ 1u, ctl, p.status, 13);
+        ok = wait_bar_warp(smem_u32(&bars->item_empty[it % kSched]), ((it / kSched) & 1u) ^ 1u, 13);
         if (!ok) break;
         if (elect_one()) {
           ctl->item[it % kSched] = more ? make_int2(bh, g) : make_int2(-1, 0);
@@ -389,7 +670,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         for (int i = 0; i < 2 && ok; ++i) {
           const int r0 = g * 256 + i * 128;
           if (r0 >= p.S) continue;
-          ok = wait_bar_warp(smem_u32(&bars->q_empty[i]), (qc[i] & 1u) ^ 1u, ctl, p.status, 1);
+          ok = wait_bar_warp(smem_u32(&bars->q_empty[i]), (qc[i] & 1u) ^ 1u, 1);
           if (!ok) break;
           const uint32_t bar = smem_u32(&bars->q_full[i]);
           if (elect_one()) {
@@ -401,34 +682,26 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         }
         const int n = p.count[(int64_t)bh * p.G + g];
         const uint32_t* lst = p.list + ((int64_t)bh * p.G + g) * p.T;
-        uint32_t ent = n > 0 ? lst[0] : 0u;
-        for (int e = 0; e < n && ok; ++e) {
-          const int t = (int)(ent & 0xFFFFu);
-          if (e + 1 < n) ent = lst[e + 1];                 // fetched one entry ahead of its use
-          {
-            const uint32_t s = kc % NK;
-            ok = wait_bar_warp(smem_u32(&bars->k_empty[s]), ((kc / NK) & 1u) ^ 1u, ctl, p.status, 2);
-            if (!ok) break;
-            const uint32_t bar = smem_u32(&bars->k_full[s]);
-            if (elect_one()) {
-              mbar_expect_tx(bar, kTile);
+        uint32_t ent = 0u, nxt = n > 0 ? lst[0] : 0u;
+        for (int e = -1; e < n && n > 0 && ok; ++e) {      // V of entry e and K of entry e + 1
+          const uint32_t nn = e + 2 < n ? lst[e + 2] : 0u; // read one entry ahead of its use
+          const uint32_t s = rc % kRing;
+          ok = wait_bar_warp(smem_u32(&bars->kv_empty[s]), ((rc / kRing) & 1u) ^ 1u, 2);
+          if (!ok) break;
+          const uint32_t bar = smem_u32(&bars->kv_full[s]);
+          const bool have_v = e >= 0, have_k = e + 1 < n;
+          if (elect_one()) {
+            mbar_expect_tx(bar, (have_v && have_k ? 2 : 1) * kTile);
+            if (have_v)
               for (int kh = 0; kh < KH; ++kh)
-                tma_load_4d(sbase + SM::kK + s * kTile + kh * kSlab, &map_k, bar, kh * 64, t * 128, h / p.kv_group, b, pol_kv);
-            }
-            ++kc;
-          }
-          {
-            const uint32_t s = vc % NV;
-            ok = wait_bar_warp(smem_u32(&bars->v_empty[s]), ((vc / NV) & 1u) ^ 1u, ctl, p.status, 3);
-            if (!ok) break;
-            const uint32_t bar = smem_u32(&bars->v_full[s]);
-            if (elect_one()) {
-              mbar_expect_tx(bar, kTile);
+                tma_load_4d(sbase + SM::kV + s * SM::kStage + kh * kSlab, &map_v, bar, kh * 64, (int)(ent & 0xFFFFu) * 128, h / p.kv_group, b, pol_kv);
+            if (have_k)
               for (int kh = 0; kh < KH; ++kh)
-                tma_load_4d(sbase + SM::kV + s * kTile + kh * kSlab, &map_v, bar, kh * 64, t * 128, h / p.kv_group, b, pol_kv);
-            }
-            ++vc;
+                tma_load_4d(sbase + SM::kK + s * SM::kStage + kh * kSlab, &map_k, bar, kh * 64, (int)(nxt & 0xFFFFu) * 128, h / p.kv_group, b, pol_kv);
           }
+          ++rc;
+          ent = nxt;
+          nxt = nn;
         }
         if (j == 0 && q < p.work.pairs) {
           j = 1;
@@ -448,7 +721,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     // of one warp (barrier waits, list reads) overlaps the other warp's MMAs on the tensor pipe.
     {
       const int i = warp >> 1;                              // query tile of this issuer
-      uint32_t kc = 0, vc = 0, qc = 0, pc = 0;
+      uint32_t rc = 0, qc = 0, pc = 0;
       bool ok = true;
       const uint32_t use_bit = 1u << (16 + i);
 
@@ -463,7 +736,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       // columns of S, so that the softmax of one half overlaps the MMAs of the other.
       // S_h = Q K_h^T: M = 128, N = 64; K_h = rows 64h .. 64h+63 of the staged K tile.
       auto issue_qk = [&](uint32_t kstage, int h) {
-        const uint64_t b0 = smem_desc(sbase + SM::kK + kstage * kTile + h * 64 * 128, 16, 1024);
+        const uint64_t b0 = smem_desc(sbase + SM::kK + kstage * SM::kStage + h * 64 * 128, 16, 1024);
         const uint32_t d = tS + 64 * h;
         mma_ss_c<false>(d, dq, b0, kIdescQK);
 #pragma unroll
@@ -475,7 +748,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       };
       // O += P_h V_h: P_h (64 keys as 32 columns of 16-bit pairs) sits in the first half of S_h.
       auto issue_pv = [&](uint32_t vstage, bool accumulate, int h) {
-        const uint64_t b0 = smem_desc(sbase + SM::kV + vstage * kTile, kSlab, 1024) + (uint64_t)h * ((4 * 2048) >> 4);
+        const uint64_t b0 = smem_desc(sbase + SM::kV + vstage * SM::kStage, kSlab, 1024) + (uint64_t)h * ((4 * 2048) >> 4);
         const uint32_t a0 = tS + 64 * h;
         mma_ts(tO, a0, b0, kIdescPV, accumulate);
 #pragma unroll
@@ -483,68 +756,44 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         tc_commit(bar_ofull[h]);
       };
 
-      for (int it = 0, bh, g; ok && next_item(it, bars, ctl, p.status, ok, bh, g); ++it) {
+      for (int it = 0, bh, g; ok && next_item(it, ok, bh, g); ++it) {
         const int n = p.count[(int64_t)bh * p.G + g];
         const uint32_t* lst = p.list + ((int64_t)bh * p.G + g) * p.T;
         const bool have = g * 256 + i * 128 < p.S;
         if (have) {
-          ok = wait_bar_warp(smem_u32(&bars->q_full[i]), qc & 1u, ctl, p.status, 4);
+          ok = wait_bar_warp(smem_u32(&bars->q_full[i]), qc & 1u, 4);
           ++qc;
           if (!ok) break;
         }
         bool started = false;                               // O_i holds a partial sum of this item
-        uint32_t cur = n > 0 ? lst[0] : 0u;
-        uint32_t nxt = n > 1 ? lst[1] : 0u;
-        if (n > 0) {
-          // A stage's `full` barrier is awaited even when this tile skips the entry: an issuer must
+        uint32_t cur = 0u, nxt = n > 0 ? lst[0] : 0u;
+        for (int e = -1; e < n && n > 0 && ok; ++e) {
+          const uint32_t nn = (e + 2 < n) ? lst[e + 2] : 0u;    // read one entry ahead of its use
+          // A stage's `full` barrier is awaited even when this tile skips both entries: an issuer must
           // not arrive on `empty` for a later round of the stage before the other issuer has arrived
           // for this one.
-          const uint32_t s = kc % NK;
-          ok = wait_bar_warp(smem_u32(&bars->k_full[s]), (kc / NK) & 1u, ctl, p.status, 5);
+          const uint32_t s = rc % kRing;
+          ok = wait_bar_warp(smem_u32(&bars->kv_full[s]), (rc / kRing) & 1u, 5);
           if (!ok) break;
-          if (cur & use_bit) {
-            tc_fence_after();
-            issue_qk(s, 0);
-            issue_qk(s, 1);
-          }
-          tc_commit(smem_u32(&bars->k_empty[s]));
-          ++kc;
-        }
-        for (int e = 0; e < n && ok; ++e) {
-          const uint32_t nn = (e + 2 < n) ? lst[e + 2] : 0u;    // read two entries ahead of its use
-          const uint32_t vs = vc % NV, ks = kc % NK;
-          ok = wait_bar_warp(smem_u32(&bars->v_full[vs]), (vc / NV) & 1u, ctl, p.status, 6);
-          if (!ok) break;
-          if (nxt) {
-            ok = wait_bar_warp(smem_u32(&bars->k_full[ks]), (kc / NK) & 1u, ctl, p.status, 8);
-            if (!ok) break;
-          }
           // per half: O += P_h V_h of this entry, then S_h of the next entry into the columns that
           // P_h just vacated
 #pragma unroll
           for (int h = 0; h < 2 && ok; ++h) {
             if (cur & use_bit) {
-              ok = wait_bar_warp(smem_u32(&bars->p_full[i][h]), pc & 1u, ctl, p.status, 7);
+              ok = wait_bar_warp(smem_u32(&bars->p_full[i][h]), pc & 1u, 7);
               if (!ok) break;
-              tc_fence_after();
-              issue_pv(vs, started || h == 1, h);
             }
-            if (nxt & use_bit) {
-              tc_fence_after();
-              issue_qk(ks, h);
-            }
+            tc_fence_after();
+            if (cur & use_bit) issue_pv(s, started || h == 1, h);
+            if (nxt & use_bit) issue_qk(s, h);
           }
           if (!ok) break;
           if (cur & use_bit) {
             ++pc;
             started = true;
           }
-          tc_commit(smem_u32(&bars->v_empty[vs]));
-          ++vc;
-          if (nxt) {
-            tc_commit(smem_u32(&bars->k_empty[ks]));
-            ++kc;
-          }
+          tc_commit(smem_u32(&bars->kv_empty[s]));
+          ++rc;
           cur = nxt;
           nxt = nn;
         }
@@ -554,167 +803,149 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
       // Abort path: this commit arrives once every MMA this warp issued has retired.
       if (ctl->abort_flag) tc_commit(smem_u32(&bars->drain));
     }
-  } else if (warp >= 4) {
+  }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));
     // =========================================================================== softmax + epilogue
-    const int i = (warp - 4) >> 2;                         // query tile of this warpgroup
+    const int i = (warp - 4) >> 3;                         // query tile of this warpgroup
+    const int hs = ((warp - 4) >> 2) & 1;                  // key half of this warpgroup
     const int wq = warp & 3;                               // TMEM lane quarter of this warp
     const int row = wq * 32 + lane;
     const uint32_t lane_off = (uint32_t)(wq * 32) << 16;
-    int32_t* kidx = reinterpret_cast<int32_t*>(smem + SM::kIdx) + (warp - 4) * 128;
-    const uint32_t bar_s[2] = {smem_u32(&bars->s_full[i][0]), smem_u32(&bars->s_full[i][1])};
-    const uint32_t bar_p[2] = {smem_u32(&bars->p_full[i][0]), smem_u32(&bars->p_full[i][1])};
-    const uint32_t bar_o[2] = {smem_u32(&bars->o_full[i][0]), smem_u32(&bars->o_full[i][1])};
-    uint32_t sc = 0;                                       // list entries done by this warpgroup
+    const uint32_t s_addr = tmem + 128 * i + lane_off + 64 * hs;
+    const uint32_t bar_s = smem_u32(&bars->s_full[i][hs]), bar_p = smem_u32(&bars->p_full[i][hs]);
+    const uint32_t post = smem_u32(&ctl->post[i][hs][wq]);
+    uint32_t sc = 0, sums = 0;                             // list entries done, row sums handed over
     bool ok = true;
 
-    for (int it = 0, bh, g; ok && next_item(it, bars, ctl, p.status, ok, bh, g); ++it) {
+    for (int it = 0, bh, g; ok && next_item(it, ok, bh, g); ++it) {
       const int r0 = g * 256 + i * 128;
       if (r0 >= p.S) continue;
-      const int b = bh / p.Hq, h = bh % p.Hq;
-      const int qpos = r0 + row;
-      const int n = p.count[(int64_t)bh * p.G + g];
       const uint32_t* lst = p.list + ((int64_t)bh * p.G + g) * p.T;
-      const int32_t* ibase = p.idx ? p.idx + (int64_t)bh * p.S : nullptr;
-      float m_used = -CUDART_INF_F;                        // scaled (log2) max the exponents refer to
-      float l = 0.f;
-      uint32_t steps = 0;                                  // entries of this item done
+      const uint32_t* end = lst + p.count[(int64_t)bh * p.G + g];
+      Refs r{-CUDART_INF_F, 0.f, kFresh};
+      const uint32_t sc0 = sc;
 
-      uint32_t ent_next = n > 0 ? lst[0] : 0u;
-      for (int e = 0; e < n && ok; ++e) {
+      uint32_t ent_next = lst < end ? *lst : 0u;
+      while (lst < end) {
         const uint32_t ent = ent_next;
-        if (e + 1 < n) ent_next = lst[e + 1];              // fetched one entry ahead of its use
+        if (++lst < end) ent_next = *lst;                  // fetched one entry ahead of its use
         if (!(ent & (1u << (16 + i)))) continue;
-        const int t = (int)(ent & 0xFFFFu);
-        const bool elem_mask = ent & (1u << (18 + i));
-        const uint32_t bits = (ent >> (20 + 4 * i)) & 0xFu;
-        if (elem_mask) {
+        // with block_size 64 these rows may not attend this key half at all
+        const bool none = p.bs == 64 && !((ent >> (20 + 4 * i + 2 * (wq >> 1) + hs)) & 1u);
+        if (ent & (1u << (18 + i))) {                      // to be masked by position
+          const int32_t* ibase = p.idx ? p.idx + (int64_t)bh * p.S : nullptr;
+          int32_t* kidx = front().kidx[warp - 4];
+          const int k0 = (int)(ent & 0xFFFFu) * 128 + 64 * hs + lane;
           __syncwarp();
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const int kp = t * 128 + c * 32 + lane;
-            kidx[c * 32 + lane] = kp >= p.S ? 0x7fffffff : ibase ? ibase[kp] : kp;
-          }
+          for (int c = 0; c < 64; c += 32) kidx[c + lane] = k0 + c >= p.S ? 0x7fffffff : ibase ? ibase[k0 + c] : k0 + c;
           __syncwarp();
         }
-
-        // Two half-steps of 64 keys, each an ordinary online-softmax step on its own 64 columns of S.
-#pragma unroll
-        for (int hs = 0; hs < 2; ++hs) {
-          ok = __all_sync(0xffffffffu, wait_bar(bar_s[hs], sc & 1u, ctl, p.status, 9));
+        const bool cold = (ent & (1u << (18 + i))) || (r.epoch & kFresh);
+        // diagnostic hook of the failure-path tests: the very first hand-over of a CTA is withheld, so the issuer's wait
+        // for it runs out and the CTA takes the abort path
+        const bool drop = p.drop_arrive && (QUEUE ? blockIdx.x == 0 : (int)blockIdx.x < p.drop_arrive) && sc == 0 && i == 0 && hs == 0;
+        ok = wait_hot(bar_s, sc & 1u, 9);
+        if (!ok) break;
+        tc_fence_after();
+        if (cold) {
+          r = before_exp(r, ent, tmem, sc, none, sc == sc0, r0 + row, p.scale_log2e);
+          ok = r.epoch != kGiveUp;
           if (!ok) break;
-          tc_fence_after();
-          const uint32_t s_addr = tmem_S[i] + lane_off + 64 * hs;
-
-          // S_h is read from TMEM once and stays in registers for the maximum and the exponentiation.
-          uint32_t sr[2][32];
-          tmem_ld32(s_addr, sr[0]);
-          tmem_ld32(s_addr + 32, sr[1]);
-          tmem_wait_ld();
-          float (&v)[64] = *reinterpret_cast<float (*)[64]>(&sr[0][0]);
-          // masks: keys of the own segment that lie after the query; with block_size 64 the 64x64
-          // sub-block (query half, key half) may not be selected
-          if (elem_mask) {
+        }
+        float sum = 0.f;
+        if (none) {
+          uint32_t zero[32];
 #pragma unroll
-            for (int c = 0; c < 64; ++c)
-              if (kidx[64 * hs + c] > qpos) v[c] = -CUDART_INF_F;
-          }
-          if (p.bs == 64 && !((bits >> (2 * (row >> 6) + hs)) & 1u)) {
-#pragma unroll
-            for (int c = 0; c < 64; ++c) v[c] = -CUDART_INF_F;
-          }
-          // Row maximum (four independent chains) and, without waiting for it, the exponentials relative to
-          // the maximum in use: the lazy rescale keeps that maximum for almost every half-step, so the chain
-          // of maxima leaves the critical path.  When a row's maximum did grow past the threshold (always in
-          // a row's first half-step) the warp rescales and exponentiates again.
-          float mx4[4];
-#pragma unroll
-          for (int a = 0; a < 4; ++a) {
-            float m = max3(v[16 * a], v[16 * a + 1], v[16 * a + 2]);
-#pragma unroll
-            for (int c = 3; c + 1 < 16; c += 2) m = max3(m, v[16 * a + c], v[16 * a + c + 1]);
-            mx4[a] = fmaxf(m, v[16 * a + 15]);
-          }
-          const float2 sc2 = make_float2(p.scale_log2e, p.scale_log2e);
-          float2 acc2[2];
-          // P_h goes back over the first 32 columns of S_h in two stores of 32 keys
-          auto exp_pass = [&](float m_ref) {
-            const float2 nm2 = make_float2(-m_ref, -m_ref);
-            acc2[0] = make_float2(0.f, 0.f);
-            acc2[1] = make_float2(0.f, 0.f);
-            uint32_t pk[16];
+          for (int c = 0; c < 32; ++c) zero[c] = 0u;
+          tmem_st32(s_addr, zero);
+        } else {
+          // All of P_h is formed before any of it goes back over the first 32 columns of S_h, so that S_h is still there
+          // for another pass when the references turn out to be stale or too low.
+          uint32_t pk[32], epoch_now;
+          for (bool last = false;;) {
+            const float2 sc2 = make_float2(p.scale_log2e, p.scale_log2e);
+            const float ref = r.ref == -CUDART_INF_F ? 0.f : r.ref;
+            const float2 nm2 = make_float2(-ref, -ref);
+            float2 acc2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
+              uint32_t sr[32];
+              tmem_ld32(s_addr + 32 * q, sr);
+              // (the epoch is read after S is there: see raise_refs)
+              if (q == 0) asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(epoch_now) : "r"(smem_u32(&ctl->epoch[i][wq])) : "memory");
+              tmem_wait_ld();
+              float (&v)[32] = *reinterpret_cast<float (*)[32]>(&sr[0]);
 #pragma unroll
               for (int c = 0; c < 16; ++c) {
-                const int col = 32 * q + 2 * c;
-                const float2 x = __ffma2_rn(make_float2(v[col], v[col + 1]), sc2, nm2);
+                const float2 x = __ffma2_rn(make_float2(v[2 * c], v[2 * c + 1]), sc2, nm2);
                 const float2 ex = make_float2(ex2(x.x), ex2(x.y));
-                acc2[c & 1] = __fadd2_rn(acc2[c & 1], ex);
-                pk[c] = PackP<DT>::pack(ex.x, ex.y);
-              }
-              tmem_st16(s_addr + 16 * q, pk);
-            }
-          };
-          exp_pass(m_used == -CUDART_INF_F ? 0.f : m_used);
-          const float mt = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2e;
-          const bool grew = mt > m_used + kRescaleThreshold;   // also the first finite maximum
-          if (__any_sync(0xffffffffu, grew)) {
-            float alpha = 1.f;
-            if (grew) {
-              alpha = ex2(m_used - mt);                      // 0 when m_used is -inf
-              m_used = mt;
-              l *= alpha;
-            }
-            if (steps > 0 || hs == 1) {
-              // O_i holds the sum up to the previous half-step: wait for that P V, then scale in place.
-              // Half 0 follows the second half of the previous entry, half 1 the first half of this one.
-              const uint32_t par = hs == 0 ? ((sc - 1u) & 1u) : (sc & 1u);
-              ok = __all_sync(0xffffffffu, wait_bar(bar_o[hs ^ 1], par, ctl, p.status, 10));
-              if (!ok) break;
-              tc_fence_after();
-#pragma unroll
-              for (int c = 0; c < D / 16; ++c) {
-                uint32_t o[16];
-                tmem_ld16(tmem_O[i] + lane_off + c * 16, o);
-                tmem_wait_ld();
-#pragma unroll
-                for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * alpha);
-                tmem_st16(tmem_O[i] + lane_off + c * 16, o);
+                pk[16 * q + c] = PackP<DT>::pack(ex.x, ex.y);
+                PackP<DT>::add(acc2[c & 1], pk[16 * q + c]);
               }
             }
-            exp_pass(m_used == -CUDART_INF_F ? 0.f : m_used);
+            sum = (acc2[0].x + acc2[0].y) + (acc2[1].x + acc2[1].y);
+            if (last || !__any_sync(0xffffffffu, epoch_now != (r.epoch & ~kFresh) || !(sum <= kSumMost<DT>))) break;
+            r = raise_refs<DT, D>(r, tmem, sc, sc == sc0, p.scale_log2e);
+            ok = r.epoch != kGiveUp;
+            if (!ok) break;
+            last = true;
           }
-          tmem_wait_st();
-          tc_fence_before();
-          // diagnostic hook of the failure-path tests: the very first hand-over of a CTA is withheld, so the issuer's wait
-          // for it runs out and the CTA takes the abort path (the comparison costs the whole-path call 0.5 %, the test nothing)
-          const bool drop = QUEUE ? p.drop_arrive && blockIdx.x == 0 : (int)blockIdx.x < p.drop_arrive;
-          if (!(drop && i == 0 && sc == 0 && hs == 0)) mbar_arrive(bar_p[hs]);
-          l += (acc2[0].x + acc2[0].y) + (acc2[1].x + acc2[1].y);
+          if (!ok) break;
+          tmem_st32(s_addr, pk);
         }
-        if (!ok) break;
+        tmem_wait_st();
+        tc_fence_before();
+        if (!drop) mbar_arrive(bar_p);
         ++sc;
-        ++steps;
+        if (lane == 0) st_post(post, 3u * sc, r.epoch & ~kFresh);
+        r.l += sum;
       }
       if (!ok) break;
+      const bool steps = sc != sc0;
+
+      // The second half's warps hand their row sums to the first half's, which write the result.
+      if (hs == 1) {
+        if (steps) {
+          *(volatile float*)&ctl->lsum[i][row] = r.l;
+          *(volatile float*)&ctl->lref[i][row] = r.ref;
+          __threadfence_block();
+          __syncwarp();
+          if (elect_one()) mbar_arrive(smem_u32(&bars->l_full[i][wq]));
+        }
+        continue;
+      }
+      if (steps) {
+        ok = wait_hot(smem_u32(&bars->l_full[i][wq]), sums & 1u, 15);
+        if (!ok) break;
+        ++sums;
+        // either half may have raised the references after the other's last step
+        r.epoch &= ~kFresh;
+        refresh(r, who());
+        const float l1 = *(volatile float*)&ctl->lsum[i][row], ref1 = *(volatile float*)&ctl->lref[i][row];
+        r.l += ref1 == r.ref || l1 == 0.f ? l1 : l1 * ex2(ref1 - r.ref);
+      }
+      const int b = bh / p.Hq, h = bh % p.Hq;
+      const uint32_t bar_o1 = smem_u32(&bars->o_full[i][1]);
 
       // epilogue: O / l in the input dtype, original token order (queries are not permuted)
-      if (steps > 0) {
-        ok = __all_sync(0xffffffffu, wait_bar(bar_o[1], (sc - 1u) & 1u, ctl, p.status, 11));
+      if (steps) {
+        ok = wait_hot(bar_o1, (sc - 1u) & 1u, 11);
         if (!ok) break;
         tc_fence_after();
       }
       // Rows leave through a per-warp transposition tile: a thread owns one row of O in TMEM, but four
       // lanes then store one row's 64-byte piece together, so a store instruction writes 8 rows x 64
       // contiguous bytes instead of 32 rows x 16 -- this matters for the replicas, which travel over NVLink.
-      const float inv = l > 0.f ? 1.f / l : 0.f;
-      unsigned char* stage = smem + SM::kStage + (warp - 4) * 32 * SM::kStageRow;
+      const float inv = r.l > 0.f ? 1.f / r.l : 0.f;
+      unsigned char* stage = front().stage[i * 4 + wq];
       const int64_t obase = (int64_t)b * p.os.b + (int64_t)h * p.os.h;
       const int wrow0 = r0 + wq * 32;                      // first query row of this warp
 #pragma unroll
       for (int c = 0; c < D / 32; ++c) {
         uint32_t o[32];
-        if (steps > 0) {
+        if (steps) {
           tmem_ld32(tmem_O[i] + lane_off + c * 32, o);
           tmem_wait_ld();
         } else {
@@ -728,7 +959,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
           w.y = PackP<DT>::pack(__uint_as_float(o[8 * j + 2]) * inv, __uint_as_float(o[8 * j + 3]) * inv);
           w.z = PackP<DT>::pack(__uint_as_float(o[8 * j + 4]) * inv, __uint_as_float(o[8 * j + 5]) * inv);
           w.w = PackP<DT>::pack(__uint_as_float(o[8 * j + 6]) * inv, __uint_as_float(o[8 * j + 7]) * inv);
-          *reinterpret_cast<uint4*>(stage + lane * SM::kStageRow + j * 16) = w;
+          *reinterpret_cast<uint4*>(stage + lane * kStageRow + j * 16) = w;
         }
         __syncwarp();
 #pragma unroll
@@ -736,7 +967,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
           const int rr = (lane >> 2) + 8 * j, piece = lane & 3;
           const int grow = wrow0 + rr;
           if (grow < p.S) {
-            const uint4 w = *reinterpret_cast<const uint4*>(stage + rr * SM::kStageRow + piece * 16);
+            const uint4 w = *reinterpret_cast<const uint4*>(stage + rr * kStageRow + piece * 16);
             const int64_t off = obase + (int64_t)grow * p.os.s + c * 32 + piece * 8;
             __stcs(reinterpret_cast<uint4*>(reinterpret_cast<T*>(p.out) + off), w);   // written once, not re-read here
             // replicas (peer GPUs of a head-sharded call): plain stores, they travel over NVLink
@@ -814,6 +1045,12 @@ int make_map(CUtensorMap* map, int dt, const void* base, const Dims& d, int head
   return PBS_OK;
 }
 
+template <typename K>
+int launch_regs(K* kernel) {
+  cudaFuncAttributes at;
+  return cudaFuncGetAttributes(&at, kernel) == cudaSuccess ? at.numRegs : -1;
+}
+
 template <int DT, int D>
 int run_tc(const Dims& d, const void* q, Strides qs, const KvSource& kv, const int32_t* idx,
            const uint32_t* list, const int32_t* count, void* out, Strides os, int32_t* status, int32_t* queue,
@@ -836,9 +1073,12 @@ int run_tc(const Dims& d, const void* q, Strides qs, const KvSource& kv, const i
   p.drop_arrive = g_drop_arrive.load(std::memory_order_relaxed);
   const int sm_count = device_sms();
   auto kern = queue ? attn_tc_kernel<DT, D, true> : attn_tc_kernel<DT, D, false>;
-  const int smem = Smem<D>::kTotal;
+  const int smem = kSmemBytes<D>;
   cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (ce != cudaSuccess) return cuda_fail(ce, "attn_tc_kernel smem attribute");
+  // The warps share out what the launch has (kRegsIssue, kRegsSoftmax): more would be waited for without an end.
+  static const bool regs_fit = launch_regs(attn_tc_kernel<DT, D, true>) == kRegsLaunch && launch_regs(attn_tc_kernel<DT, D, false>) == kRegsLaunch;
+  if (!regs_fit) { set_error("attn_tc_kernel was not built with %d registers a thread", kRegsLaunch); return PBS_ERR_CUDA; }
   p.queue = queue;
   p.work = make_schedule(d.B * d.Hq, p.G, sm_count);
   kern<<<queue ? p.work.ctas : entries(p.work), kThreads, smem, st>>>(mq, mk, mv, p);
