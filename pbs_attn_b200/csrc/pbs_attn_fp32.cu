@@ -4,14 +4,18 @@
 // scores scaled by 1/sqrt(D), key visible iff its original position <= the query's, online softmax in base 2,
 // fp32 accumulators.  There is no fp32 tensor-core path, so the bound is the fp32 FMA rate: 4*D FLOP per
 // (query, key) of the kept blocks.  One CTA = 32 query rows; a step = 64 keys of one kept block, brought in by
-// cp.async while the step before is computed (head_dim 64; at 128 two buffers would leave one CTA a SM).
+// cp.async.  Loads are hidden by the other CTAs of the SM (four at head_dim 64, two at 128), not by a second buffer: with one at
+// head_dim 64 there were two CTAs a SM, 4 heads x 8192 tokens 1033 us against 927.
 // 128 threads as 8 x 16: a thread owns 4 rows x 4 keys of S and 4 rows x D/16 columns of O, so 32 packed FMA pairs feed
 // on 8 shared-memory reads of 16 bytes, and the 16 lanes that share rows reduce them by shuffles and pass P through
 // shared memory without a block-wide barrier.  The products of two neighbouring head-dim elements go into two partial
 // sums (packed fp32 pairs), which are added at the end of the row.
-// Measured against pbs_attn_simt.cu's kernel (one row and 8 keys a thread, operands re-read for every FMA), 2048 tokens, block 64:
-// 4 heads of 64 (1.1 G FMA) 1079 -> 127 us, 8 heads of 128 (4.6 G FMA) 1955 -> 277 us = 33 TFLOP/s; 8192 tokens 8230 -> 1032
-// and (block 128) 19880 -> 3456 us = 38 TFLOP/s.
+// A step takes 2 to 4 us, so few query tiles leave the GPU waiting for the longest row: then a cluster of 2, 4 or 8 CTAs shares a query
+// tile's steps and puts O together through distributed shared memory.  While the GPU has places for all CTAs (the line: 4 heads x
+// 2048 tokens with 1 / 4 / 8 CTAs a tile 130 / 83 / 89 us; 8 heads of 128, whose tiles alone take all places, 257 with 1, 282 with 4);
+// 4 heads of 64: 300 tokens 23 -> 18 us, 1000 tokens 58 -> 36, 2048 tokens 124 -> 83 (34 % of the FMA rate), 4 x 4000 tokens 1016 -> 866.
+#include <cooperative_groups.h>
+
 #include "pbs_common.cuh"
 
 namespace pbs {
@@ -25,9 +29,9 @@ constexpr int FP = FM + 4;    // floats per row of the P tile (key-major)
 template <int D>
 struct Fp32Smem {
   static constexpr int kLd = D + 4;                       // padded row: 16-byte reads of 8 neighbouring keys hit all banks
-  static constexpr int kBuf = D == 64 ? 2 : 1;
-  static constexpr int kFloats = FM * kLd + kBuf * FN * (kLd + D) + FN * FP;
-  static size_t bytes(int nb) { return sizeof(float) * kFloats + sizeof(int32_t) * kBuf * FN + sizeof(uint16_t) * ((nb + 7) & ~7); }
+  static constexpr int kCtas = D == 64 ? 4 : 2;           // that a SM holds
+  static constexpr int kFloats = FM * kLd + FN * (kLd + D) + FN * FP;
+  static size_t bytes(int nb) { return sizeof(float) * kFloats + sizeof(int32_t) * FN + sizeof(uint16_t) * ((nb + 7) & ~7); }
 };
 
 __device__ __forceinline__ void cp16(float* dst, const float* src, bool live) {
@@ -35,23 +39,24 @@ __device__ __forceinline__ void cp16(float* dst, const float* src, bool live) {
 }
 
 template <int D>
-__global__ void __launch_bounds__(FT, 2)
+__global__ void __launch_bounds__(FT, Fp32Smem<D>::kCtas)
 attn_fp32_kernel(const float* __restrict__ q, Strides qs, const float* __restrict__ pk, const float* __restrict__ pv,
                  const int32_t* __restrict__ idx, const uint8_t* __restrict__ mask, float* __restrict__ out, Strides os,
                  int Hq, int S, int bs, int nb, float scale_log2e) {
   using SM = Fp32Smem<D>;
-  constexpr int LD = SM::kLd, NBUF = SM::kBuf, C4 = D / 4, OC = D / 16;
+  constexpr int LD = SM::kLd, C4 = D / 4, OC = D / 16;
   extern __shared__ __align__(16) float sm[];
   float* Qs = sm;                                         // [FM][LD]
-  float* Ks = Qs + FM * LD;                               // [NBUF][FN][LD]
-  float* Vs = Ks + NBUF * FN * LD;                        // [NBUF][FN][D]
-  float* Ps = Vs + NBUF * FN * D;                         // [FN][FP]
-  int32_t* kpos = reinterpret_cast<int32_t*>(Ps + FN * FP);               // [NBUF][FN] original positions
-  uint16_t* kept = reinterpret_cast<uint16_t*>(kpos + NBUF * FN);         // kept blocks of this query block
+  float* Ks = Qs + FM * LD;                               // [FN][LD]
+  float* Vs = Ks + FN * LD;                               // [FN][D]
+  float* Ps = Vs + FN * D;                                // [FN][FP]
+  int32_t* kpos = reinterpret_cast<int32_t*>(Ps + FN * FP);               // [FN] original positions
+  uint16_t* kept = reinterpret_cast<uint16_t*>(kpos + FN);                // kept blocks of this query block
   __shared__ int wcount[FT / 32];
 
-  const int bh = blockIdx.x, b = bh / Hq, h = bh % Hq;
-  const int r0 = (gridDim.y - 1 - blockIdx.y) * FM;       // the longest rows start first
+  const int rank = blockIdx.x, ranks = gridDim.x;         // of the cluster that shares the query tile's steps
+  const int bh = blockIdx.y, b = bh / Hq, h = bh % Hq;
+  const int r0 = (gridDim.z - 1 - blockIdx.z) * FM;       // the longest rows start first
   const int qb = r0 / bs;
   const float* qbase = q + (int64_t)b * qs.b + (int64_t)h * qs.h;
   const float* kbase = pk + (int64_t)bh * S * D;
@@ -82,19 +87,23 @@ attn_fp32_kernel(const float* __restrict__ q, Strides qs, const float* __restric
     if (on) kept[at] = (uint16_t)kb;
     __syncthreads();
   }
-  const int per_block = bs / FN, nsteps = nkept * per_block;
-  auto first_key = [&](int s) { return (int)kept[s / per_block] * bs + (s % per_block) * FN; };
+  // this CTA's steps: every ranks-th
+  const int per_block = bs / FN, nsteps = (nkept * per_block - rank + ranks - 1) / ranks;
+  auto first_key = [&](int s) {
+    const int step = s * ranks + rank;
+    return (int)kept[step / per_block] * bs + (step % per_block) * FN;
+  };
   auto load = [&](int s) {
-    const int k0 = first_key(s), buf = s % NBUF;
+    const int k0 = first_key(s);
     for (int i = threadIdx.x; i < FN * C4; i += FT) {
       const int r = i / C4, c = i % C4;
       const bool live = k0 + r < S;
       const int64_t at = (int64_t)(live ? k0 + r : 0) * D + 4 * c;
-      cp16(Ks + (buf * FN + r) * LD + 4 * c, kbase + at, live);
-      cp16(Vs + (buf * FN + r) * D + 4 * c, vbase + at, live);
+      cp16(Ks + r * LD + 4 * c, kbase + at, live);
+      cp16(Vs + r * D + 4 * c, vbase + at, live);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
-    if (threadIdx.x < FN) kpos[buf * FN + threadIdx.x] = k0 + (int)threadIdx.x < S ? ibase[k0 + threadIdx.x] : 0x7fffffff;
+    if (threadIdx.x < FN) kpos[threadIdx.x] = k0 + (int)threadIdx.x < S ? ibase[k0 + threadIdx.x] : 0x7fffffff;
   };
 
   float2 acc[4][OC / 2];
@@ -109,16 +118,8 @@ attn_fp32_kernel(const float* __restrict__ q, Strides qs, const float* __restric
 
   if (nsteps > 0) load(0);
   for (int s = 0; s < nsteps; ++s) {
-    if (NBUF == 2 && s + 1 < nsteps) {
-      load(s + 1);                                        // into the buffer the step before last has left
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    const int buf = s % NBUF;
-    const float* Kt = Ks + buf * FN * LD;
-    const float* Vt = Vs + buf * FN * D;
 
     // S = Q K^T: rows 4 ty + i, keys tx + 16 j
     float2 sp[4][4];
@@ -132,7 +133,7 @@ attn_fp32_kernel(const float* __restrict__ q, Strides qs, const float* __restric
 #pragma unroll
       for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(Qs + (4 * ty + i) * LD + d);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) c[j] = *reinterpret_cast<const float4*>(Kt + (tx + 16 * j) * LD + d);
+      for (int j = 0; j < 4; ++j) c[j] = *reinterpret_cast<const float4*>(Ks + (tx + 16 * j) * LD + d);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -144,7 +145,7 @@ attn_fp32_kernel(const float* __restrict__ q, Strides qs, const float* __restric
     // online softmax; every key's position counts, because the order of a stage call need not stay inside the segments
     int kp[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) kp[j] = kpos[buf * FN + tx + 16 * j];
+    for (int j = 0; j < 4; ++j) kp[j] = kpos[tx + 16 * j];
     float p[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -186,7 +187,7 @@ attn_fp32_kernel(const float* __restrict__ q, Strides qs, const float* __restric
       const float pa[4] = {pr.x, pr.y, pr.z, pr.w};
 #pragma unroll
       for (int jc = 0; jc < OC / 4; ++jc) {
-        const float4 vv = *reinterpret_cast<const float4*>(Vt + kk * D + 64 * jc + 4 * tx);
+        const float4 vv = *reinterpret_cast<const float4*>(Vs + kk * D + 64 * jc + 4 * tx);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           acc[i][2 * jc] = __ffma2_rn(make_float2(pa[i], pa[i]), make_float2(vv.x, vv.y), acc[i][2 * jc]);
@@ -194,21 +195,61 @@ attn_fp32_kernel(const float* __restrict__ q, Strides qs, const float* __restric
         }
       }
     }
-    __syncthreads();                                      // the buffer and the P tile are free again
-    if (NBUF == 1 && s + 1 < nsteps) load(s + 1);
+    __syncthreads();                                      // the tiles are free again
+    if (s + 1 < nsteps) load(s + 1);
   }
-  if (nsteps == 0) asm volatile("cp.async.wait_all;" ::: "memory");   // the query tile's copies end inside the CTA
+  if (nsteps == 0) {                                      // the query tile's copies end before its place is used again
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+  }
+  float* obase = out + (int64_t)b * os.b + (int64_t)h * os.h;
+  if (ranks == 1) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int row = r0 + 4 * ty + i;
+      if (row >= S) continue;
+      const float inv = l_run[i] > 0.f ? 1.f / l_run[i] : 0.f;
+#pragma unroll
+      for (int jc = 0; jc < OC / 4; ++jc)
+        *reinterpret_cast<float4*>(obase + (int64_t)row * os.s + 64 * jc + 4 * tx) =
+            make_float4(acc[i][2 * jc].x * inv, acc[i][2 * jc].y * inv, acc[i][2 * jc + 1].x * inv, acc[i][2 * jc + 1].y * inv);
+    }
+    return;
+  }
+  // The CTAs' parts of O and their row statistics meet in shared memory (the Q tile's and the P tile's place); each CTA puts together and
+  // stores every ranks-th row.
+  float* part = Qs;                                       // [FM][LD]
+  float2* stat = reinterpret_cast<float2*>(Ps);           // [FM] (maximum, sum)
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int row = r0 + 4 * ty + i;
-    if (row >= S) continue;
-    const float inv = l_run[i] > 0.f ? 1.f / l_run[i] : 0.f;
-    float* orow = out + (int64_t)b * os.b + (int64_t)h * os.h + (int64_t)row * os.s;
 #pragma unroll
     for (int jc = 0; jc < OC / 4; ++jc)
-      *reinterpret_cast<float4*>(orow + 64 * jc + 4 * tx) =
-          make_float4(acc[i][2 * jc].x * inv, acc[i][2 * jc].y * inv, acc[i][2 * jc + 1].x * inv, acc[i][2 * jc + 1].y * inv);
+      *reinterpret_cast<float4*>(part + (4 * ty + i) * LD + 64 * jc + 4 * tx) =
+          make_float4(acc[i][2 * jc].x, acc[i][2 * jc].y, acc[i][2 * jc + 1].x, acc[i][2 * jc + 1].y);
+    if (tx == 0) stat[4 * ty + i] = make_float2(m_run[i], l_run[i]);
   }
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.sync();
+  for (int t = threadIdx.x; t < (FM / ranks) * C4; t += FT) {
+    const int r = (t / C4) * ranks + rank, c = t % C4;
+    if (r0 + r >= S) continue;
+    float m = -CUDART_INF_F;
+    for (int x = 0; x < ranks; ++x) m = fmaxf(m, cluster.map_shared_rank(stat, x)[r].x);
+    const float m_ref = m == -CUDART_INF_F ? 0.f : m;
+    float l = 0.f;
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int x = 0; x < ranks; ++x) {
+      const float2 st = cluster.map_shared_rank(stat, x)[r];
+      const float4 v = *reinterpret_cast<const float4*>(cluster.map_shared_rank(part, x) + r * LD + 4 * c);
+      const float w = exp2f(st.x - m_ref);
+      l += w * st.y;
+      o.x += w * v.x; o.y += w * v.y; o.z += w * v.z; o.w += w * v.w;
+    }
+    const float inv = l > 0.f ? 1.f / l : 0.f;
+    *reinterpret_cast<float4*>(obase + (int64_t)(r0 + r) * os.s + 4 * c) = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
+  }
+  cluster.sync();                                         // nobody leaves while its part is read
 }
 
 template <int D>
@@ -217,9 +258,24 @@ int run_fp32(const Dims& d, const void* q, Strides qs, const void* pk, const voi
   const size_t smem = Fp32Smem<D>::bytes(d.nb);
   cudaError_t e = cudaFuncSetAttribute(attn_fp32_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return cuda_fail(e, "attn_fp32_kernel smem attribute");
-  attn_fp32_kernel<D><<<dim3(d.B * d.Hq, (d.S + FM - 1) / FM), FT, smem, st>>>(
-      (const float*)q, qs, (const float*)pk, (const float*)pv, idx, mask, (float*)out, os, d.Hq, d.S, d.bs, d.nb,
-      (float)(1.4426950408889634 / sqrt((double)d.D)));
+  // CTAs a query tile: as many as it takes to fill the GPU's places, at most 8 (a portable cluster) and one a step
+  const int tiles = (d.S + FM - 1) / FM;
+  int ranks = 1;
+  while (ranks < 8 && ranks * FN < d.S && (int64_t)tiles * d.B * d.Hq * ranks < Fp32Smem<D>::kCtas * device_sms()) ranks *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ranks, d.B * d.Hq, tiles);
+  cfg.blockDim = dim3(FT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = ranks;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = ranks > 1 ? 1 : 0;
+  e = cudaLaunchKernelEx(&cfg, attn_fp32_kernel<D>, (const float*)q, qs, (const float*)pk, (const float*)pv, idx, mask, (float*)out, os, d.Hq, d.S,
+                         d.bs, d.nb, (float)(1.4426950408889634 / sqrt((double)d.D)));
+  if (e != cudaSuccess) return cuda_fail(e, "attn_fp32_kernel");
   PBS_CUDA_CHECK_LAUNCH("attn_fp32_kernel");
   return PBS_OK;
 }
@@ -227,7 +283,7 @@ int run_fp32(const Dims& d, const void* q, Strides qs, const void* pk, const voi
 }  // namespace
 
 // Blocks must be whole steps.  The 4096 blocks a row that the library takes at most keep the row of kept blocks (8 KB) beside
-// two CTAs' tiles and the query tiles within the grid's second dimension.
+// the CTA's tiles and the query tiles within the grid's third dimension.
 bool attn_fp32_supported(const Dims& d, int dt) {
   return dt == PBS_FP32 && (d.D == 64 || d.D == 128) && d.bs % FN == 0;
 }

@@ -8,11 +8,13 @@ pytestmark = pytest.mark.gpu
 
 
 # tails of the 32-row query tile and the 64-key step, both head sizes (two buffers / one), both block sizes, one token,
-# the dense fallback, rows that keep nothing ("mean" without the own block) and a strided query tensor
+# the dense fallback, rows that keep nothing ("mean" without the own block) and a strided query tensor; 1 to 8 CTAs share a
+# query tile (1 from 4500 tokens with 8 heads of 64 on, and at one step), some of them without a step
 @pytest.mark.parametrize("tokens,head_dim,block,segment,kind", [
     (1, 64, 64, 64, "pbs"), (33, 64, 64, 128, "pbs"), (250, 128, 128, 256, "pbs"), (640, 64, 64, 128, "pbs"),
     (1500, 64, 128, 256, "strided"), (1023, 128, 64, 64, "pbs"), (2047, 128, 128, 512, "strided"),
-    (1500, 64, 64, 64, "mean"), (777, 128, 128, 128, "mean")])
+    (1500, 64, 64, 64, "mean"), (777, 128, 128, 128, "mean"), (65, 64, 64, 64, "pbs"), (129, 128, 128, 128, "pbs"),
+    (4500, 64, 64, 128, "pbs")])
 def test_fp32_kernel_equals_generic_kernel(tokens, head_dim, block, segment, kind):
     from pbs_attn_b200.prefill import MeanPooling_prefill, permuted_block_sparse_attn_fwd
     w = Workload("fp32", 2, 4, 2, head_dim, tokens, "fp32", block, segment, 0.7, 5e5, sinks=4)
