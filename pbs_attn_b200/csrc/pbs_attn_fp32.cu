@@ -42,7 +42,7 @@ template <int D>
 __global__ void __launch_bounds__(FT, Fp32Smem<D>::kCtas)
 attn_fp32_kernel(const float* __restrict__ q, Strides qs, const float* __restrict__ pk, const float* __restrict__ pv,
                  const int32_t* __restrict__ idx, const uint8_t* __restrict__ mask, float* __restrict__ out, Strides os,
-                 int Hq, int S, int bs, int nb, float scale_log2e) {
+                 int Hq, int S, int bs, int nb, int ranks, float scale_log2e) {
   using SM = Fp32Smem<D>;
   constexpr int LD = SM::kLd, C4 = D / 4, OC = D / 16;
   extern __shared__ __align__(16) float sm[];
@@ -54,9 +54,9 @@ attn_fp32_kernel(const float* __restrict__ q, Strides qs, const float* __restric
   uint16_t* kept = reinterpret_cast<uint16_t*>(kpos + FN);                // kept blocks of this query block
   __shared__ int wcount[FT / 32];
 
-  const int rank = blockIdx.x, ranks = gridDim.x;         // of the cluster that shares the query tile's steps
-  const int bh = blockIdx.y, b = bh / Hq, h = bh % Hq;
-  const int r0 = (gridDim.z - 1 - blockIdx.z) * FM;       // the longest rows start first
+  const int rank = blockIdx.x % ranks;                    // in the cluster of CTAs that shares the query tile's steps
+  const int bh = blockIdx.x / ranks, b = bh / Hq, h = bh % Hq;
+  const int r0 = (gridDim.y - 1 - blockIdx.y) * FM;       // the longest rows start first
   const int qb = r0 / bs;
   const float* qbase = q + (int64_t)b * qs.b + (int64_t)h * qs.h;
   const float* kbase = pk + (int64_t)bh * S * D;
@@ -263,7 +263,7 @@ int run_fp32(const Dims& d, const void* q, Strides qs, const void* pk, const voi
   int ranks = 1;
   while (ranks < 8 && ranks * FN < d.S && (int64_t)tiles * d.B * d.Hq * ranks < Fp32Smem<D>::kCtas * device_sms()) ranks *= 2;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(ranks, d.B * d.Hq, tiles);
+  cfg.gridDim = dim3(d.B * d.Hq * ranks, tiles);
   cfg.blockDim = dim3(FT);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
@@ -274,7 +274,7 @@ int run_fp32(const Dims& d, const void* q, Strides qs, const void* pk, const voi
   cfg.attrs = &at;
   cfg.numAttrs = ranks > 1 ? 1 : 0;
   e = cudaLaunchKernelEx(&cfg, attn_fp32_kernel<D>, (const float*)q, qs, (const float*)pk, (const float*)pv, idx, mask, (float*)out, os, d.Hq, d.S,
-                         d.bs, d.nb, (float)(1.4426950408889634 / sqrt((double)d.D)));
+                         d.bs, d.nb, ranks, (float)(1.4426950408889634 / sqrt((double)d.D)));
   if (e != cudaSuccess) return cuda_fail(e, "attn_fp32_kernel");
   PBS_CUDA_CHECK_LAUNCH("attn_fp32_kernel");
   return PBS_OK;
@@ -283,7 +283,7 @@ int run_fp32(const Dims& d, const void* q, Strides qs, const void* pk, const voi
 }  // namespace
 
 // Blocks must be whole steps.  The 4096 blocks a row that the library takes at most keep the row of kept blocks (8 KB) beside
-// the CTA's tiles and the query tiles within the grid's third dimension.
+// the CTAs' tiles and the query tiles within the grid's second dimension.
 bool attn_fp32_supported(const Dims& d, int dt) {
   return dt == PBS_FP32 && (d.D == 64 || d.D == 128) && d.bs % FN == 0;
 }
