@@ -307,7 +307,7 @@ int pbs_select_blocks(const pbs_shape_t* shape, const void* pooled_q, const void
   PBS_TRY(check_shape(shape));
   PBS_NONNULL(pooled_q); PBS_NONNULL(pooled_k); PBS_NONNULL(first_block); PBS_NONNULL(options); PBS_NONNULL(block_mask);
   return launch_select_blocks(make_dims(*shape), shape->dtype, pooled_q, pooled_k, first_block, *options, block_mask,
-                              block_scores, (cudaStream_t)stream);
+                              block_scores, nullptr, nullptr, (cudaStream_t)stream);
 }
 
 int pbs_build_tile_lists(const pbs_shape_t* shape, const uint8_t* block_mask, uint32_t* tile_list,
@@ -422,10 +422,11 @@ int pbs_prefill_fwd(const pbs_shape_t* shape, const void* q, const int64_t q_str
       PBS_TRY(launch_fill_mask_ones(d, sc->block_mask, st));
     } else {
       PBS_TRY(pbs_pool_queries(shape, q, q_strides, sc->pooled_q, options->query_pool_mode, stream));
-      PBS_TRY(pbs_select_blocks(shape, sc->pooled_q, sc->pooled_k, sc->first_block, options, sc->block_mask, nullptr, stream));
+      const bool lists = impl == PBS_ATTN_TCGEN05;
+      PBS_TRY(launch_select_blocks(d, shape->dtype, sc->pooled_q, sc->pooled_k, sc->first_block, *options, sc->block_mask, nullptr,
+                                   lists ? sc->tile_list : nullptr, lists ? sc->tile_count : nullptr, st));
     }
-    if (impl == PBS_ATTN_TCGEN05)
-      PBS_TRY(pbs_build_tile_lists(&attn_shape, sc->block_mask, sc->tile_list, sc->tile_count, stream));
+    if (dense && impl == PBS_ATTN_TCGEN05) PBS_TRY(launch_build_tile_lists(d, sc->block_mask, sc->tile_list, sc->tile_count, st));
   }
   // The scratch serves one call at a time and its status words were cleared above, so word 7 can count the draws.
   if (impl == PBS_ATTN_TCGEN05)

@@ -184,7 +184,7 @@ int launch_rope(int dt, int B, int H, int S, int D, void* x, Strides xs, const v
                 int64_t cs_b, int64_t cs_s, cudaStream_t st);
 int launch_select_blocks(const Dims& d, int dt, const void* pooled_q, const void* pooled_k,
                          const int32_t* first_block, const pbs_options_t& opt, uint8_t* mask, float* scores,
-                         cudaStream_t st);
+                         uint32_t* list, int32_t* count, cudaStream_t st);   // list not null: the tile lists too
 void set_select_impl(int impl);
 int launch_fill_mask_ones(const Dims& d, uint8_t* mask, cudaStream_t st);
 int launch_build_tile_lists(const Dims& d, const uint8_t* mask, uint32_t* list, int32_t* count, cudaStream_t st);

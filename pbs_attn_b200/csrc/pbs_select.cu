@@ -231,12 +231,49 @@ __device__ __forceinline__ double warp_sum_double(double v) {
 
 // CPR: 16-byte pieces per pooled row; KPT: kv blocks per lane held in registers (32 * KPT >= nb); TS_ROWS: q blocks
 // per CTA (16 or 8)
+// The CTA's rows are whole 256-query groups, so it can also write their tile lists (lists.list not null): as a kernel of its own,
+// that read the mask again, these took 5.6 us (4 x 2048 tokens, 32 heads), 8 (8192 tokens, block 64) or 17 (32768 tokens), and a launch.
+struct TileLists {
+  uint32_t* list;
+  int32_t* count;
+  int S, bs, seg;
+};
+
+// Entry of key tile t in the list of query group g (0: neither query tile uses it).  on(qb, kb): block kb is selected for query block qb.
+// Bits 0-15 tile id (128 keys each); bits 16/17: used by query tile 0/1 of the group (128 rows each); bits 18/19: that query tile must
+// mask this tile element-wise (the tile lies in the query tile's own segment); bits 20-23 / 24-27: which (q block, kv block) sub-blocks
+// of the 128x128 tile are selected for query tile 0 / 1, bit = 2*qi + ki (only bit 0 when block_size is 128).
+template <typename On>
+__device__ __forceinline__ uint32_t tile_entry(int g, int t, int S, int bs, int seg, int nb, On on) {
+  const int sub = 128 / bs;                                // blocks per 128-row / 128-key tile (1 or 2)
+  uint32_t e = 0;
+  for (int m = 0; m < 2; ++m) {
+    const int r0 = g * 256 + m * 128;
+    if (r0 >= S) continue;
+    uint32_t bits = 0;
+    for (int qi = 0; qi < sub; ++qi) {
+      const int qb = r0 / bs + qi;
+      if (qb >= nb) continue;
+      for (int ki = 0; ki < sub; ++ki) {
+        const int kb = t * sub + ki;
+        if (kb < nb && on(qb, kb)) bits |= 1u << (2 * qi + ki);
+      }
+    }
+    if (bits) {
+      e |= (1u << (16 + m)) | (bits << (20 + 4 * m));
+      const int q_seg_first = r0 / seg, k_seg_last = (min(t * 128 + 128, S) - 1) / seg;
+      if (k_seg_last >= q_seg_first) e |= 1u << (18 + m);
+    }
+  }
+  return e ? e | (uint32_t)t : 0u;
+}
+
 template <int DT, int CPR, int KPT, int TS_ROWS>
 __global__ void __launch_bounds__(256)
 select_tiled_kernel(const typename Elem<DT>::T* __restrict__ pooled_q, const typename Elem<DT>::T* __restrict__ pooled_k,
                     const int32_t* __restrict__ first_block, const float* __restrict__ thr_per_head, float thr_scalar,
                     int select_all, int force_first, int diag_candidates, int own_segment, uint8_t* __restrict__ mask,
-                    float* __restrict__ scores, int Hq, int nb, int bps, float sqrt_d, int ncpad) {
+                    float* __restrict__ scores, int Hq, int nb, int bps, float sqrt_d, int ncpad, TileLists lists) {
   using E = Elem<DT>;
   using T = typename E::T;
   constexpr int EPV = 16 / (int)sizeof(T);
@@ -246,6 +283,7 @@ select_tiled_kernel(const typename Elem<DT>::T* __restrict__ pooled_q, const typ
   float* Qs = reinterpret_cast<float*>(smem_raw);          // [TS_ROWS][D] fp32
   T* Kc = reinterpret_cast<T*>(Qs + TS_ROWS * D);          // [2][64][LDK]
   T* lg = Kc + 2 * TS_CHUNK * LDK;                         // [TS_ROWS][ncpad] rounded logits
+  __shared__ uint32_t kept[TS_ROWS][KPT + 1];              // bit i of word k: block 32 k + i is on
 
   const int qb0 = blockIdx.x * TS_ROWS;
   const int bh = blockIdx.y;
@@ -446,13 +484,32 @@ select_tiled_kernel(const typename Elem<DT>::T* __restrict__ pooled_q, const typ
     const bool no_cand_rule = !select_all && ncand == 0;   // the kept block is kv block 0 even with no candidate
     for (int k = 0; 32 * k < nb; ++k) {
       const int i = 32 * k + lane;
-      if (i >= nb) break;
-      bool on = (k < KPT) && ((sel >> k) & 1ull) && (i < ncand || no_cand_rule);
-      on = on || i == fb || (i >= s0 && i < s1);
+      bool on = ((sel >> k) & 1ull) && (i < ncand || no_cand_rule);
+      on = i < nb && (on || i == fb || (i >= s0 && i < s1));
+      const uint32_t word = __ballot_sync(0xffffffffu, on);
+      if (lane == 0) kept[r][k] = word;
+      if (i >= nb) continue;
       row[i] = on ? 1 : 0;
       if (srow && (select_all || i >= ncand)) srow[i] = 0.f;
     }
   }
+  if (!lists.list) return;
+  // ---- the tile lists of the CTA's query groups, a warp each
+  __syncthreads();
+  const int rows_per_group = 256 / lists.bs, ngroups = (lists.S + 255) / 256, ntiles = (lists.S + 127) / 128;
+  if (warp >= TS_ROWS / rows_per_group) return;
+  const int g = qb0 / rows_per_group + warp;
+  if (g >= ngroups) return;
+  uint32_t* out = lists.list + ((int64_t)bh * ngroups + g) * ntiles;
+  int n = 0;
+  for (int t0 = 0; t0 < ntiles; t0 += 32) {
+    const int t = t0 + lane;
+    const uint32_t e = t < ntiles ? tile_entry(g, t, lists.S, lists.bs, lists.seg, nb, [&](int qb, int kb) { return (kept[qb - qb0][kb >> 5] >> (kb & 31)) & 1u; }) : 0u;
+    const unsigned ball = __ballot_sync(0xffffffffu, e != 0);
+    if (e) out[n + __popc(ball & ((1u << lane) - 1))] = e;
+    n += __popc(ball);
+  }
+  if (lane == 0) lists.count[(int64_t)bh * ngroups + g] = n;
 }
 
 __global__ void fill_ones_kernel(uint8_t* p, int64_t n) {
@@ -460,11 +517,7 @@ __global__ void fill_ones_kernel(uint8_t* p, int64_t n) {
   if (i < n) p[i] = 1;
 }
 
-// Tile-list entry: bits 0-15 tile id (128 keys each); bits 16/17: used by query tile 0/1 of the
-// group (128 rows each); bits 18/19: that query tile must mask this tile element-wise (the tile
-// lies in the query tile's own segment); bits 20-23 / 24-27: which (q block, kv block) sub-blocks
-// of the 128x128 tile are selected for query tile 0 / 1, bit = 2*qi + ki (only bit 0 when
-// block_size is 128).
+// Tile lists from a mask: for the stage call, and after the kernel with a row per CTA.
 __global__ void __launch_bounds__(128)
 tile_list_kernel(const uint8_t* __restrict__ mask, uint32_t* __restrict__ list, int32_t* __restrict__ count,
                  int S, int bs, int seg, int nb, int ngroups, int ntiles) {
@@ -475,34 +528,11 @@ tile_list_kernel(const uint8_t* __restrict__ mask, uint32_t* __restrict__ list, 
   __shared__ int wcnt[4];
   if (threadIdx.x == 0) wbase = 0;
   __syncthreads();
-  const int sub = 128 / bs;                              // blocks per 128-row / 128-key tile (1 or 2)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint8_t* rows = mask + (int64_t)bh * nb * nb;
   for (int t0 = 0; t0 < ntiles; t0 += blockDim.x) {
     const int t = t0 + threadIdx.x;
-    uint32_t e = 0;
-    if (t < ntiles) {
-      for (int m = 0; m < 2; ++m) {
-        const int r0 = g * 256 + m * 128;
-        if (r0 >= S) continue;
-        uint32_t bits = 0;
-        for (int qi = 0; qi < sub; ++qi) {
-          const int qb = r0 / bs + qi;
-          if (qb >= nb) continue;
-          for (int ki = 0; ki < sub; ++ki) {
-            const int kb = t * sub + ki;
-            if (kb < nb && mask[((int64_t)bh * nb + qb) * nb + kb]) bits |= 1u << (2 * qi + ki);
-          }
-        }
-        if (bits) {
-          e |= (1u << (16 + m)) | (bits << (20 + 4 * m));
-          const int q_seg_first = r0 / seg, q_seg_last = (min(r0 + 128, S) - 1) / seg;
-          const int k_seg_last = (min(t * 128 + 128, S) - 1) / seg;
-          (void)q_seg_last;
-          if (k_seg_last >= q_seg_first) e |= 1u << (18 + m);
-        }
-      }
-      if (e) e |= (uint32_t)t;
-    }
+    const uint32_t e = t < ntiles ? tile_entry(g, t, S, bs, seg, nb, [&](int qb, int kb) { return rows[(int64_t)qb * nb + kb] != 0; }) : 0u;
     const unsigned ball = __ballot_sync(0xffffffffu, e != 0);
     if (lane == 0) wcnt[warp] = __popc(ball);
     __syncthreads();
@@ -544,21 +574,21 @@ dense_setup_kernel(int32_t* __restrict__ idx, int32_t* __restrict__ first_block,
 
 template <int DT, int CPR, int KPT, int ROWS>
 int run_select_tiled(const Dims& d, const void* pooled_q, const void* pooled_k, const int32_t* first_block,
-                     const pbs_options_t& opt, uint8_t* mask, float* scores, cudaStream_t st) {
+                     const pbs_options_t& opt, uint8_t* mask, float* scores, const TileLists& lists, cudaStream_t st) {
   using T = typename Elem<DT>::T;
   constexpr int EPV = 16 / (int)sizeof(T);
   const int ncpad = ((d.nb + TS_CHUNK - 1) / TS_CHUNK) * TS_CHUNK;
   const size_t smem = (size_t)ROWS * d.D * sizeof(float) + (size_t)2 * TS_CHUNK * (d.D + EPV) * sizeof(T) +
                       (size_t)ROWS * ncpad * sizeof(T);
   auto kern = select_tiled_kernel<DT, CPR, KPT, ROWS>;
-  if (smem > 48 * 1024) {
+  if (smem + ROWS * (KPT + 1) * sizeof(uint32_t) > 48 * 1024) {   // beside the static words of kept blocks
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_fail(e, "select_tiled_kernel smem attribute");
   }
   kern<<<dim3((d.nb + ROWS - 1) / ROWS, d.B * d.Hq), 256, smem, st>>>(
       (const T*)pooled_q, (const T*)pooled_k, first_block, opt.threshold_per_head, opt.threshold, opt.select_all,
       opt.force_select_first_block, opt.diagonal_candidates, opt.no_own_segment ? 0 : 1, mask, scores, d.Hq, d.nb, d.bps,
-      (float)sqrt((double)d.D), ncpad);
+      (float)sqrt((double)d.D), ncpad, lists);
   PBS_CUDA_CHECK_LAUNCH("select_tiled_kernel");
   return PBS_OK;
 }
@@ -570,15 +600,15 @@ int run_select_tiled(const Dims& d, const void* pooled_q, const void* pooled_k, 
 // fp32 D = 128 26.7 / 21.8, 33.7 / 29.1, 42.5 / 36.6, 56.6 / 60.4; at eight all do: bf16 D = 128 40.3 / 36.1 .. 83.9 / 90.6.
 template <int DT, int CPR>
 int run_select_tiled_k(const Dims& d, const void* pooled_q, const void* pooled_k, const int32_t* first_block,
-                       const pbs_options_t& opt, uint8_t* mask, float* scores, cudaStream_t st) {
+                       const pbs_options_t& opt, uint8_t* mask, float* scores, const TileLists& lists, cudaStream_t st) {
   if (d.nb <= 256) {
     if ((int64_t)((d.nb + 7) / 8) * d.B * d.Hq <= 3 * device_sms())
-      return run_select_tiled<DT, CPR, 8, 8>(d, pooled_q, pooled_k, first_block, opt, mask, scores, st);
-    return run_select_tiled<DT, CPR, 8, 16>(d, pooled_q, pooled_k, first_block, opt, mask, scores, st);
+      return run_select_tiled<DT, CPR, 8, 8>(d, pooled_q, pooled_k, first_block, opt, mask, scores, lists, st);
+    return run_select_tiled<DT, CPR, 8, 16>(d, pooled_q, pooled_k, first_block, opt, mask, scores, lists, st);
   }
-  if (d.nb <= 512) return run_select_tiled<DT, CPR, 16, 16>(d, pooled_q, pooled_k, first_block, opt, mask, scores, st);
-  if (d.nb <= 1024) return run_select_tiled<DT, CPR, 32, 16>(d, pooled_q, pooled_k, first_block, opt, mask, scores, st);
-  return run_select_tiled<DT, CPR, 64, 16>(d, pooled_q, pooled_k, first_block, opt, mask, scores, st);
+  if (d.nb <= 512) return run_select_tiled<DT, CPR, 16, 16>(d, pooled_q, pooled_k, first_block, opt, mask, scores, lists, st);
+  if (d.nb <= 1024) return run_select_tiled<DT, CPR, 32, 16>(d, pooled_q, pooled_k, first_block, opt, mask, scores, lists, st);
+  return run_select_tiled<DT, CPR, 64, 16>(d, pooled_q, pooled_k, first_block, opt, mask, scores, lists, st);
 }
 
 // The tiled kernel covers pooled rows of 8, 16 or 32 16-byte pieces and up to 2048 blocks per row.
@@ -588,12 +618,12 @@ bool select_tiled_supported(const Dims& d, int dt) {
 }
 
 int launch_select_tiled(const Dims& d, int dt, const void* pooled_q, const void* pooled_k, const int32_t* first_block,
-                        const pbs_options_t& opt, uint8_t* mask, float* scores, cudaStream_t st) {
+                        const pbs_options_t& opt, uint8_t* mask, float* scores, const TileLists& lists, cudaStream_t st) {
   const int cpr = d.D * elem_bytes(dt) / 16;
 #define PBS_TS(DT)                                                                                                \
-  (cpr == 8 ? run_select_tiled_k<DT, 8>(d, pooled_q, pooled_k, first_block, opt, mask, scores, st)                 \
-   : cpr == 16 ? run_select_tiled_k<DT, 16>(d, pooled_q, pooled_k, first_block, opt, mask, scores, st)             \
-               : run_select_tiled_k<DT, 32>(d, pooled_q, pooled_k, first_block, opt, mask, scores, st))
+  (cpr == 8 ? run_select_tiled_k<DT, 8>(d, pooled_q, pooled_k, first_block, opt, mask, scores, lists, st)                 \
+   : cpr == 16 ? run_select_tiled_k<DT, 16>(d, pooled_q, pooled_k, first_block, opt, mask, scores, lists, st)             \
+               : run_select_tiled_k<DT, 32>(d, pooled_q, pooled_k, first_block, opt, mask, scores, lists, st))
   switch (dt) {
     case PBS_BF16: return PBS_TS(PBS_BF16);
     case PBS_FP16: return PBS_TS(PBS_FP16);
@@ -611,9 +641,11 @@ void set_select_impl(int impl) { g_select_impl.store(impl, std::memory_order_rel
 
 int launch_select_blocks(const Dims& d, int dt, const void* pooled_q, const void* pooled_k,
                          const int32_t* first_block, const pbs_options_t& opt, uint8_t* mask, float* scores,
-                         cudaStream_t st) {
-  if (g_select_impl.load(std::memory_order_relaxed) == 0 && select_tiled_supported(d, dt))
-    return launch_select_tiled(d, dt, pooled_q, pooled_k, first_block, opt, mask, scores, st);
+                         uint32_t* list, int32_t* count, cudaStream_t st) {
+  if (g_select_impl.load(std::memory_order_relaxed) == 0 && select_tiled_supported(d, dt)) {
+    const TileLists lists{list, count, d.S, d.bs, d.seg};
+    return launch_select_tiled(d, dt, pooled_q, pooled_k, first_block, opt, mask, scores, lists, st);
+  }
   const int npow2 = next_pow2(d.nb);
   const size_t smem = (size_t)npow2 * 8 + (size_t)d.D * 4 + (size_t)d.nb * 4;
   dim3 grid(d.nb, d.B * d.Hq);
@@ -650,7 +682,7 @@ int launch_select_blocks(const Dims& d, int dt, const void* pooled_q, const void
 #undef PBS_SEL
 #undef PBS_SEL_E
   PBS_CUDA_CHECK_LAUNCH("select_kernel");
-  return PBS_OK;
+  return list ? launch_build_tile_lists(d, mask, list, count, st) : PBS_OK;
 }
 
 int launch_fill_mask_ones(const Dims& d, uint8_t* mask, cudaStream_t st) {
