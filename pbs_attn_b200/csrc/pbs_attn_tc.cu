@@ -35,7 +35,7 @@
 // Three things make four warpgroups pay, each of which alone decides between a gain and a loss:
 //  - the warps of the two halves exchange nothing from step to step.  A row's reference is not its running maximum
 //    but what its first tile gave; it is raised only when a half-step's sum leaves kSumMost, which for bf16 (the range of fp32) hardly
-//    ever happens.  All of that protocol (raise_refs, before_exp) is out of line.  With a check between the halves in every
+//    ever happens.  All of that protocol (settle, before_exp) is out of line.  With a check between the halves in every
 //    half-step (a poll, an order of the hand-overs) the kernel was slower than before: 3200 to 3500 cycles a step against 2850.
 //  - registers: 96 a thread at 640 threads, 104 after the issuing warps have given some up.  S is read in two parts of 32
 //    columns; read at once it spills (2 % slower), in parts of 16 or with a part ahead it is slower too.
@@ -291,9 +291,10 @@ struct Ctl {
   int2 item[kSched];            // (b, h) and query group of the items handed to the other roles; x < 0: no more
   uint32_t tmem_base;
   volatile int abort_flag;
-  // Shared by the two softmax warps (one per key half) of a query tile's lane quarter, see raise_refs:
+  // Shared by the two softmax warps (one per key half) of a query tile's lane quarter, see settle:
   uint2 post[2][2][4];          // [query tile][key half][lane quarter] progress, epoch of the references that its last P refers to
   uint32_t epoch[2][4];         // [query tile][lane quarter] times the references were raised
+  uint32_t raised_at[2][2][4];  // [epoch & 1][query tile][lane quarter] half-step (2 * list entries done + key half) that raised them last
   float ref[2][2][128];         // [epoch & 1][query tile] references when they were raised last: the partner may still be reading the ones before
   float smax[2][2][2][128];     // [entry & 1][query tile][key half] first maxima
   uint32_t starts[2][2][4];     // [query tile][key half][lane quarter] meetings so far
@@ -457,12 +458,18 @@ __device__ __forceinline__ Who who() {
   return Who{w >> 3, (w >> 2) & 1, w & 3, lane, (w & 3) * 32 + lane};
 }
 
+// 2^(from - to) for references of a row, `to` the later one: they are raised by whole numbers, so this is a power of two.
+__device__ __forceinline__ float ref_scale(float from, float to) {
+  const float n = rintf(from - to);
+  return n >= -126.f ? __int_as_float(((int)fminf(n, 0.f) + 127) << 23) : 0.f;
+}
+
 // Takes over references that the partner warp has raised.
 __device__ __forceinline__ void refresh(Refs& r, const Who& w) {
   const uint32_t now = *const_cast<const volatile uint32_t*>(&front().ctl.epoch[w.i][w.wq]);
   if (__any_sync(0xffffffffu, now != r.epoch)) {
     const float ref = *const_cast<const volatile float*>(&front().ctl.ref[now & 1u][w.i][w.row]);
-    if (ref != r.ref && r.l > 0.f) r.l *= ex2(r.ref - ref);
+    if (ref != r.ref && r.l > 0.f) r.l *= ref_scale(r.ref, ref);
     r.ref = ref;
     r.epoch = now;
   }
@@ -497,60 +504,98 @@ __device__ __noinline__ Refs before_exp(Refs r, uint32_t ent, uint32_t tmem, uin
   return r;
 }
 
-// A half-step k found the references of another epoch, or a sum above kSumMost with them.  S_k is still in TMEM, and since
-// P_k has not been handed over, neither P V of k nor of the partner's k + 1 can start: whoever raises references has O and P_{k+1}
-// to itself.  Raising waits for the P V of k - 1, which the old references belong to, publishes the new ones, scales O, and then
-// looks at k + 1.  Its warp reads the epoch after it has seen its S: if that S is not there yet it will see the new one.  Otherwise
-// its progress says when it is through: with the old epoch its P_{k+1} is scaled here (by a power of two) and its sum by itself once it
-// sees the epoch; or it waits for the P V of k to raise references of its own, and reads the epoch after that.
+// References are raised by whole numbers, so that all is scaled by powers of two, exactly, and the result does not depend on who
+// scales what and when.  A half-step k that finds a sum above kSumMost raises them: it waits for the P V of k - 1, which the old ones
+// belong to, publishes the new ones and scales O.  S_k is still in TMEM, and since P_k has not been handed over, neither P V of k nor of the
+// partner's k + 1 can start: O and P_{k+1} are its own.  P_{k+1} is always formed with the references before and then scaled.  Its warp reads
+// the epoch after it has seen its S: if that S is not there yet it will see the new epoch and scale by itself (scale_late).  Otherwise its
+// progress says when it is through: with the old epoch its P is scaled here and its sum by itself once it sees the epoch; or it
+// waits for the P V of k to raise references of its own, and takes the new ones after that.
+// For a half-step that has seen another epoch or a sum above kSumMost: the references to form P again with; last: these stay.
+struct Verdict {
+  Refs r;
+  bool last;
+};
+__device__ __forceinline__ bool raised_just_now(uint32_t now, const Who& w, uint32_t sc) {   // epoch `now` is the work of half-step k - 1
+  return *const_cast<const volatile uint32_t*>(&front().ctl.raised_at[now & 1u][w.i][w.wq]) + 1u == 2u * sc + w.hs;
+}
 template <int DT, int D>
-__device__ __noinline__ Refs raise_refs(Refs r, uint32_t tmem, uint32_t sc, bool first_entry, float scale_log2e) {
+__device__ __noinline__ Verdict settle(Refs r, uint32_t tmem, uint32_t sc, bool first_entry, float scale_log2e) {
   const Who w = who();
   Bars& bars = front().bars;
   Ctl& ctl = front().ctl;
   const uint32_t fresh = r.epoch & kFresh;
   r.epoch &= ~kFresh;
-  const uint32_t before = w.hs == 0 ? sc - 1u : sc, after = w.hs == 0 ? sc : sc + 1u;   // entries of half-steps k - 1 and k + 1
-  const uint32_t lanes = (uint32_t)(w.wq * 32) << 16, s_addr = tmem + lanes + 128 * w.i + 64 * w.hs;
-  const float top = row_max64(s_addr) * scale_log2e;
-  refresh(r, w);
-  if (__any_sync(0xffffffffu, top > r.ref + kUpLeast<DT>)) {
-    if (w.lane == 0) st_post(smem_u32(&ctl.post[w.i][w.hs][w.wq]), 3u * sc + kRaising, r.epoch);
-    const bool have_o = !first_entry || w.hs == 1;
-    if (have_o) {
-      if (!wait_bar_warp(smem_u32(&bars.o_full[w.i][w.hs ^ 1]), before & 1u, 10)) { r.epoch = kGiveUp; return r; }
-      tc_fence_after();
-      refresh(r, w);
-    }
-    const bool up = top > r.ref + kUpLeast<DT>;
-    if (__any_sync(0xffffffffu, up)) {
-      const float old = r.ref;
-      if (up) r.ref += ceilf(top - r.ref);
-      const float alpha = up ? ex2(old - r.ref) : 1.f;
-      r.l *= alpha;
-      ++r.epoch;
-      *const_cast<volatile float*>(&ctl.ref[r.epoch & 1u][w.i][w.row]) = r.ref;
-      __threadfence_block();
-      __syncwarp();
-      if (w.lane == 0) *const_cast<volatile uint32_t*>(&ctl.epoch[w.i][w.wq]) = r.epoch;
-      __threadfence_block();
-      __syncwarp();
-      if (have_o) rescale_o(tmem + lanes + 256 + 128 * w.i, alpha, D);
-      if (__all_sync(0xffffffffu, mbar_try_wait(smem_u32(&bars.s_full[w.i][w.hs ^ 1]), after & 1u))) {
-        // (a first half has met the second one of its entry already)
-        uint2 theirs;
-        if (!wait_post(smem_u32(&ctl.post[w.i][w.hs ^ 1][w.wq]), 3u * after + (w.hs == 0 ? kRaising : kAtStart), theirs, 16)) {
-          r.epoch = kGiveUp;
-          return r;
-        }
-        if (theirs.x >= 3u * (after + 1u) && theirs.y != r.epoch) {
-          tc_fence_after();
-          scale_p<DT>(tmem + lanes + 128 * w.i + 64 * (w.hs ^ 1), alpha);
-        }
-      }
-      tmem_wait_st();
+  auto verdict = [&](bool last) {
+    if (r.epoch != kGiveUp) r.epoch |= fresh;
+    return Verdict{r, last};
+  };
+  auto refs_of = [&](uint32_t epoch) { return *const_cast<const volatile float*>(&ctl.ref[epoch & 1u][w.i][w.row]); };
+  auto take = [&](uint32_t epoch) {
+    const float ref = refs_of(epoch);
+    if (ref != r.ref && r.l > 0.f) r.l *= ref_scale(r.ref, ref);
+    r.ref = ref;
+    r.epoch = epoch;
+  };
+  const uint32_t now = *const_cast<const volatile uint32_t*>(&ctl.epoch[w.i][w.wq]);
+  if (__any_sync(0xffffffffu, now != r.epoch)) {
+    const bool just_now = raised_just_now(now, w, sc);
+    if (!just_now || now != r.epoch + 1u) {
+      take(just_now ? now - 1u : now);
+      return verdict(false);
     }
   }
+  const uint32_t before = w.hs == 0 ? sc - 1u : sc, after = w.hs == 0 ? sc : sc + 1u;   // entries of half-steps k - 1 and k + 1
+  const uint32_t lanes = (uint32_t)(w.wq * 32) << 16;
+  const float top = row_max64(tmem + lanes + 128 * w.i + 64 * w.hs) * scale_log2e;
+  if (w.lane == 0) st_post(smem_u32(&ctl.post[w.i][w.hs][w.wq]), 3u * sc + kRaising, r.epoch);
+  const bool have_o = !first_entry || w.hs == 1;
+  if (have_o) {
+    if (!wait_bar_warp(smem_u32(&bars.o_full[w.i][w.hs ^ 1]), before & 1u, 10)) { r.epoch = kGiveUp; return verdict(true); }
+    tc_fence_after();
+    refresh(r, w);
+  }
+  const bool up = top > r.ref + kUpLeast<DT>;
+  if (__any_sync(0xffffffffu, up)) {
+    const float old = r.ref;
+    if (up) r.ref += ceilf(top - r.ref);
+    const float alpha = up ? ref_scale(old, r.ref) : 1.f;
+    r.l *= alpha;
+    ++r.epoch;
+    *const_cast<volatile float*>(&ctl.ref[r.epoch & 1u][w.i][w.row]) = r.ref;
+    if (w.lane == 0) *const_cast<volatile uint32_t*>(&ctl.raised_at[r.epoch & 1u][w.i][w.wq]) = 2u * sc + w.hs;
+    __threadfence_block();
+    __syncwarp();
+    if (w.lane == 0) *const_cast<volatile uint32_t*>(&ctl.epoch[w.i][w.wq]) = r.epoch;
+    __threadfence_block();
+    __syncwarp();
+    if (have_o) rescale_o(tmem + lanes + 256 + 128 * w.i, alpha, D);
+    if (__all_sync(0xffffffffu, mbar_try_wait(smem_u32(&bars.s_full[w.i][w.hs ^ 1]), after & 1u))) {
+      // (a first half has met the second one of its entry already)
+      uint2 theirs;
+      if (!wait_post(smem_u32(&ctl.post[w.i][w.hs ^ 1][w.wq]), 3u * after + (w.hs == 0 ? kRaising : kAtStart), theirs, 16)) {
+        r.epoch = kGiveUp;
+        return verdict(true);
+      }
+      if (theirs.x >= 3u * (after + 1u) && theirs.y != r.epoch) {
+        tc_fence_after();
+        scale_p<DT>(tmem + lanes + 128 * w.i + 64 * (w.hs ^ 1), alpha);
+      }
+    }
+    tmem_wait_st();
+  }
+  return verdict(true);
+}
+// After half-step k - 1 raised the references that P_k was formed with: P_k, in TMEM, and the row's sum scaled.
+template <int DT>
+__device__ __noinline__ Refs scale_late(Refs r, uint32_t s_addr) {
+  const Who w = who();
+  const uint32_t fresh = r.epoch & kFresh;
+  r.epoch &= ~kFresh;
+  const float old = r.ref;
+  refresh(r, w);
+  tmem_wait_st();
+  scale_p<DT>(s_addr, r.ref == old ? 1.f : ref_scale(old, r.ref));
   r.epoch |= fresh;
   return r;
 }
@@ -873,7 +918,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             for (int q = 0; q < 2; ++q) {
               uint32_t sr[32];
               tmem_ld32(s_addr + 32 * q, sr);
-              // (the epoch is read after S is there: see raise_refs)
+              // (the epoch is read after S is there: see settle)
               if (q == 0) asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(epoch_now) : "r"(smem_u32(&ctl->epoch[i][wq])) : "memory");
               tmem_wait_ld();
               float (&v)[32] = *reinterpret_cast<float (*)[32]>(&sr[0]);
@@ -886,14 +931,25 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
               }
             }
             sum = (acc2[0].x + acc2[0].y) + (acc2[1].x + acc2[1].y);
-            if (last || !__any_sync(0xffffffffu, epoch_now != (r.epoch & ~kFresh) || !(sum <= kSumMost<DT>))) break;
-            r = raise_refs<DT, D>(r, tmem, sc, sc == sc0, p.scale_log2e);
+            const bool big = !(sum <= kSumMost<DT>);
+            if (last || !__any_sync(0xffffffffu, epoch_now != (r.epoch & ~kFresh) || big)) {
+              tmem_st32(s_addr, pk);
+              break;
+            }
+            if (epoch_now == (r.epoch & ~kFresh) + 1u && raised_just_now(epoch_now, who(), sc) && !__any_sync(0xffffffffu, big)) {
+              tmem_st32(s_addr, pk);
+              const float old = r.ref;
+              r = scale_late<DT>(r, s_addr);
+              if (r.ref != old) sum *= ref_scale(old, r.ref);
+              break;
+            }
+            const Verdict verdict = settle<DT, D>(r, tmem, sc, sc == sc0, p.scale_log2e);
+            r = verdict.r;
             ok = r.epoch != kGiveUp;
             if (!ok) break;
-            last = true;
+            last = verdict.last;
           }
           if (!ok) break;
-          tmem_st32(s_addr, pk);
         }
         tmem_wait_st();
         tc_fence_before();
@@ -924,7 +980,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         r.epoch &= ~kFresh;
         refresh(r, who());
         const float l1 = *(volatile float*)&ctl->lsum[i][row], ref1 = *(volatile float*)&ctl->lref[i][row];
-        r.l += ref1 == r.ref || l1 == 0.f ? l1 : l1 * ex2(ref1 - r.ref);
+        r.l += ref1 == r.ref || l1 == 0.f ? l1 : l1 * ref_scale(ref1, r.ref);
       }
       const int b = bh / p.Hq, h = bh % p.Hq;
       const uint32_t bar_o1 = smem_u32(&bars->o_full[i][1]);
