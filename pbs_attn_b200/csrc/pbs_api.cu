@@ -7,6 +7,7 @@
 #include <cuda.h>
 
 #include "pbs_common.cuh"
+#include "pbs_pool.cuh"
 
 namespace pbs {
 
@@ -236,9 +237,10 @@ int pbs_scratch_sizes(const pbs_shape_t* shape, pbs_scratch_sizes_t* z) {
   return PBS_OK;
 }
 
-int pbs_key_importance(const pbs_shape_t* shape, const void* q, const int64_t q_strides[4],
-                       const void* k, const int64_t k_strides[4], void* logits, void* partials,
-                       void* rowstats, float* importance, void* stream) {
+// Key importance, and where the kernels can do it beside, the query pooling.
+static int key_importance(const pbs_shape_t* shape, const void* q, const int64_t q_strides[4],
+                          const void* k, const int64_t k_strides[4], void* logits, void* partials,
+                          void* rowstats, float* importance, QueryPooling* pool, void* stream) {
   PBS_TRY(check_shape(shape));
   Strides qs, ks;
   PBS_TRY(check_tensor("q", q, q_strides, shape->dtype, &qs));
@@ -250,7 +252,13 @@ int pbs_key_importance(const pbs_shape_t* shape, const void* q, const int64_t q_
   }
   const Dims d = make_dims(*shape);
   if (d.S < d.bs) { set_error("seq_len %d shorter than block_size %d", d.S, d.bs); return PBS_ERR_SHAPE; }
-  return launch_key_importance(d, shape->dtype, q, qs, k, ks, logits, partials, rowstats, importance, (cudaStream_t)stream);
+  return launch_key_importance(d, shape->dtype, q, qs, k, ks, logits, partials, rowstats, importance, pool, (cudaStream_t)stream);
+}
+
+int pbs_key_importance(const pbs_shape_t* shape, const void* q, const int64_t q_strides[4],
+                       const void* k, const int64_t k_strides[4], void* logits, void* partials,
+                       void* rowstats, float* importance, void* stream) {
+  return key_importance(shape, q, q_strides, k, k_strides, logits, partials, rowstats, importance, nullptr, stream);
 }
 
 int pbs_segment_permute(const pbs_shape_t* shape, const float* importance, const void* k,
@@ -410,9 +418,9 @@ int pbs_prefill_fwd(const pbs_shape_t* shape, const void* q, const int64_t q_str
   } else {
     cudaError_t e = cudaMemsetAsync(sc->status, 0, 8 * sizeof(int32_t), st);
     if (e != cudaSuccess) return cuda_fail(e, "clear status");
+    QueryPooling pool{sc->pooled_q, options->query_pool_mode, false};
     if (!identity)
-      PBS_TRY(pbs_key_importance(shape, q, q_strides, k, k_strides, sc->logits, sc->partials, sc->rowstats,
-                                 sc->importance, stream));
+      PBS_TRY(key_importance(shape, q, q_strides, k, k_strides, sc->logits, sc->partials, sc->rowstats, sc->importance, &pool, stream));
     Dims order = d;
     if (identity) { order.nseg = 0; order.L = 0; }
     PBS_TRY(launch_segment_permute(order, shape->dtype, identity ? nullptr : sc->importance, k, ks, v, vs, sc->key_indices,
@@ -421,7 +429,7 @@ int pbs_prefill_fwd(const pbs_shape_t* shape, const void* q, const int64_t q_str
     if (dense) {
       PBS_TRY(launch_fill_mask_ones(d, sc->block_mask, st));
     } else {
-      PBS_TRY(pbs_pool_queries(shape, q, q_strides, sc->pooled_q, options->query_pool_mode, stream));
+      if (!pool.pooled) PBS_TRY(pbs_pool_queries(shape, q, q_strides, sc->pooled_q, options->query_pool_mode, stream));
       const bool lists = impl == PBS_ATTN_TCGEN05;
       PBS_TRY(launch_select_blocks(d, shape->dtype, sc->pooled_q, sc->pooled_k, sc->first_block, *options, sc->block_mask, nullptr,
                                    lists ? sc->tile_list : nullptr, lists ? sc->tile_count : nullptr, st));

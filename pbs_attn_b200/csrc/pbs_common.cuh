@@ -171,8 +171,9 @@ void count_launch();
 
 // Stage launchers (defined one per .cu file).
 int device_sms();             // SMs of the current device, the one a launch goes to
+struct QueryPooling;                     // null, or what the first scoring pass pools beside its own work where it can
 int launch_key_importance(const Dims& d, int dt, const void* q, Strides qs, const void* k, Strides ks,
-                          void* logits, void* partials, void* rowstats, float* importance, cudaStream_t st);
+                          void* logits, void* partials, void* rowstats, float* importance, QueryPooling* pool, cudaStream_t st);
 int launch_segment_permute(const Dims& d, int dt, const float* importance, const void* k, Strides ks,
                            const void* v, Strides vs, int32_t* idx, void* perm_k, void* perm_v,
                            void* pooled_k, int pool_mode, int32_t* first_block, cudaStream_t st);

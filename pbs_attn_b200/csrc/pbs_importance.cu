@@ -21,6 +21,7 @@
 #include <mutex>
 
 #include "pbs_common.cuh"
+#include "pbs_pool.cuh"
 
 namespace pbs {
 namespace {
@@ -221,6 +222,10 @@ __device__ __forceinline__ float2 div_by(float2 x, float z, float rz) {
   return __ffma2_rn(__ffma2_rn(make_float2(-q.x, -q.y), make_float2(z, z), x), r2, q);
 }
 
+// The first pass leaves the memory system idle (0.45 TB/s at 4 x 2048 tokens) and its issue slots half used, so CTAs that pool the query
+// blocks, which is nothing but reading, run among its own (whole calls: 4 x 2048 tokens 381 -> 373 us, 8192 tokens of head_dim 64 491 -> 478,
+// block_size 64 at 32768 tokens 7594 -> 7536, 6001 tokens fp16 and 32768 sparse tokens alike).  Four query blocks a half CTA: with 16 the
+// pooling is a tail of its own (410 us), with one or two 378, all at the head of a group's CTAs instead of the end 391.
 // FASTDIV: rounding a * (1 / sqrt(D)) to the input type gives the same bits as rounding a / sqrt(D)
 // for EVERY value a of that type (established on the host by trying all 65536 of them)
 // DH: head_dim when it is 64 or 128 (loops unroll, index arithmetic folds), 0 = any multiple of 16
@@ -230,7 +235,8 @@ score_mma_kernel(const typename Elem<DT>::T* __restrict__ q, Strides qs,
                  const typename Elem<DT>::T* __restrict__ k, Strides ks,
                  float2* __restrict__ partials, const float2* __restrict__ rowstats, float* __restrict__ importance,
                  typename Elem<DT>::T* __restrict__ logits_out,
-                 int Hq, int group, int S, int D_rt, int bs, int L, int ntile, int tiles_per_cta, float sqrt_d) {
+                 int Hq, int group, int S, int D_rt, int bs, int L, int ntile, int tiles_per_cta, float sqrt_d, int score_ctas,
+                 typename Elem<DT>::T* __restrict__ pooled_q, int pool_mode, int nb) {
   using E = Elem<DT>;
   using T = typename E::T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -246,9 +252,21 @@ score_mma_kernel(const typename Elem<DT>::T* __restrict__ q, Strides qs,
   float3* stats = reinterpret_cast<float3*>(gs + 2 * kMaxGroups * TN);   // [bs] (max, sum, 1 / sum)
 
   // the query heads of a KV group sit next to each other in the grid: they read the same K tiles
-  const int hin = blockIdx.x % group, chunk = blockIdx.x / group;
   const int Hkv = Hq / group;
   const int b = blockIdx.y / Hkv, hkv = blockIdx.y % Hkv;
+  if (PASS == 1 && (int)blockIdx.x >= score_ctas) {
+    // further CTAs of the first pass pool the group's query blocks, one per half of the CTA at a time
+    const int half = threadIdx.x >> 7, step = 2 * (gridDim.x - score_ctas);
+    float* part = reinterpret_cast<float*>(smem_raw) + half * (bs / 16) * D;
+    for (int t = 2 * (blockIdx.x - score_ctas) + half; t < group * nb; t += step) {
+      const int head = b * Hq + hkv * group + t / nb, blk = t % nb;
+      pool_query_block<DT, 8>(q + (int64_t)b * qs.b + (int64_t)(hkv * group + t / nb) * qs.h, qs.s, pooled_q + ((int64_t)head * nb + blk) * D, blk,
+                              pool_mode, S, D, bs, part, threadIdx.x & 127, 128, [half] { asm volatile("bar.sync %0, 128;" ::"r"(half + 1) : "memory"); });
+      asm volatile("bar.sync %0, 128;" ::"r"(half + 1) : "memory");   // the sums' place is free again
+    }
+    return;
+  }
+  const int hin = blockIdx.x % group, chunk = blockIdx.x / group;
   const int h = hkv * group + hin;
   const int bh = b * Hq + h;
   const T* qbase = q + (int64_t)b * qs.b + (int64_t)h * qs.h + (int64_t)(S - bs) * qs.s;
@@ -552,7 +570,7 @@ bool mul_equals_div(int D) {
 
 template <int DT>
 int run(const Dims& d, const void* q, Strides qs, const void* k, Strides ks, void* logits, void* partials,
-        void* rowstats, float* importance, cudaStream_t st) {
+        void* rowstats, float* importance, QueryPooling* pool, cudaStream_t st) {
   using T = typename Elem<DT>::T;
   const int BH = d.B * d.Hq;
   const int ntile = (d.L + TN - 1) / TN;
@@ -569,11 +587,12 @@ int run(const Dims& d, const void* q, Strides qs, const void* k, Strides ks, voi
   bool fastdiv = false;
   if constexpr (DT != PBS_FP32) fastdiv = mma && mul_equals_div<DT>(d.D);
 
+  if (pool) pool->pooled = mma;
   for (int pass = 1; pass <= 2; ++pass) {
     if constexpr (DT != PBS_FP32) {
       if (mma) {
         using Kern = void (*)(const T*, Strides, const T*, Strides, float2*, const float2*, float*, T*, int, int, int, int,
-                              int, int, int, int, float);
+                              int, int, int, int, float, int, T*, int, int);
         auto pick = [&](auto dh) -> Kern {
           constexpr int DH = decltype(dh)::value;
           return pass == 1 ? (fastdiv ? (Kern)score_mma_kernel<DT, 1, true, DH> : (Kern)score_mma_kernel<DT, 1, false, DH>)
@@ -582,13 +601,16 @@ int run(const Dims& d, const void* q, Strides qs, const void* k, Strides ks, voi
         Kern kern = d.D == 128 ? pick(std::integral_constant<int, 128>{})
                     : d.D == 64 ? pick(std::integral_constant<int, 64>{}) : pick(std::integral_constant<int, 0>{});
         const size_t smem = pass == 1 ? smem1 : smem2;
+        // four query blocks per half of a pooling CTA
+        const int score_ctas = chunks * d.group, pool_ctas = pass == 1 && pool ? (d.group * d.nb + 7) / 8 : 0;
         if (smem > 48 * 1024) {
           cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
           if (e != cudaSuccess) return cuda_fail(e, "score_mma_kernel smem attribute");
         }
-        kern<<<dim3(chunks * d.group, d.B * d.Hkv), 256, smem, st>>>(
+        kern<<<dim3(score_ctas + pool_ctas, d.B * d.Hkv), 256, smem, st>>>(
             (const T*)q, qs, (const T*)k, ks, (float2*)partials, (const float2*)rowstats, importance,
-            pass == 1 ? (T*)logits : nullptr, d.Hq, d.group, d.S, d.D, d.bs, d.L, ntile, tiles_per_cta, sq);
+            pass == 1 ? (T*)logits : nullptr, d.Hq, d.group, d.S, d.D, d.bs, d.L, ntile, tiles_per_cta, sq, score_ctas,
+            pool ? (T*)pool->pooled_q : nullptr, pool ? pool->mode : 0, d.nb);
         PBS_CUDA_CHECK_LAUNCH("score_mma_kernel");
       }
     }
@@ -613,12 +635,12 @@ int run(const Dims& d, const void* q, Strides qs, const void* k, Strides ks, voi
 }  // namespace
 
 int launch_key_importance(const Dims& d, int dt, const void* q, Strides qs, const void* k, Strides ks,
-                          void* logits, void* partials, void* rowstats, float* importance, cudaStream_t st) {
+                          void* logits, void* partials, void* rowstats, float* importance, QueryPooling* pool, cudaStream_t st) {
   if (d.L == 0) return PBS_OK;
   switch (dt) {
-    case PBS_BF16: return run<PBS_BF16>(d, q, qs, k, ks, logits, partials, rowstats, importance, st);
-    case PBS_FP16: return run<PBS_FP16>(d, q, qs, k, ks, logits, partials, rowstats, importance, st);
-    default: return run<PBS_FP32>(d, q, qs, k, ks, logits, partials, rowstats, importance, st);
+    case PBS_BF16: return run<PBS_BF16>(d, q, qs, k, ks, logits, partials, rowstats, importance, pool, st);
+    case PBS_FP16: return run<PBS_FP16>(d, q, qs, k, ks, logits, partials, rowstats, importance, pool, st);
+    default: return run<PBS_FP32>(d, q, qs, k, ks, logits, partials, rowstats, importance, pool, st);
   }
 }
 

@@ -10,6 +10,7 @@
 // importance read (4*L), K and V rows read (from L2 for all but one of the Hq/Hkv heads that share a KV
 // head) and written once each (2*S*D*e), indices written (4*S), pooled K written (nb*D*e).
 #include "pbs_common.cuh"
+#include "pbs_pool.cuh"
 
 namespace pbs {
 namespace {
@@ -139,60 +140,16 @@ segment_permute_kernel(const float* __restrict__ importance,
   }
 }
 
-// One CTA per (q block, b, h).  A thread owns one 16-row group x one 16-byte piece of the row: its 16
-// loads are independent (all in flight at once), its sums follow the reference's reduction order (rows
-// one after the other inside a group of 16); a second step adds the group sums in order.
+// One CTA per (q block, b, h).
 template <int DT>
 __global__ void __launch_bounds__(256)
 pool_queries_kernel(const typename Elem<DT>::T* __restrict__ q, Strides qs,
                     typename Elem<DT>::T* __restrict__ pooled_q, int pool_mode,
                     int Hq, int S, int D, int bs, int nb) {
-  using E = Elem<DT>;
-  using T = typename E::T;
-  constexpr int EPV = 16 / (int)sizeof(T);
   __shared__ float part[16 * 256];                         // [16-row group][dim]
-  const int blk = blockIdx.x;
-  const int bh = blockIdx.y;
-  const int b = bh / Hq, h = bh % Hq;
-  const T* qb = q + (int64_t)b * qs.b + (int64_t)h * qs.h;
-  const int r0 = blk * bs, r1 = min(r0 + bs, S);
-  const int groups = bs / 16, cpr = D / EPV;
-  const bool mean = pool_mode == PBS_POOL_MEAN;
-  for (int i = threadIdx.x; i < groups * cpr; i += blockDim.x) {
-    const int g = i / cpr, c = i % cpr;
-    const int g0 = r0 + 16 * g, n = max(0, min(16, r1 - g0));
-    uint4 raw[16];
-#pragma unroll
-    for (int rr = 0; rr < 16; ++rr)
-      if (rr < n) raw[rr] = *reinterpret_cast<const uint4*>(qb + (int64_t)(g0 + rr) * qs.s + c * EPV);
-    float acc[EPV];
-#pragma unroll
-    for (int t = 0; t < EPV; ++t) acc[t] = mean ? 0.f : -CUDART_INF_F;
-#pragma unroll
-    for (int rr = 0; rr < 16; ++rr) {
-      if (rr < n) {
-        const T* e = reinterpret_cast<const T*>(&raw[rr]);
-#pragma unroll
-        for (int t = 0; t < EPV; ++t) acc[t] = mean ? acc[t] + E::ld(e + t) : fmaxf(acc[t], E::ld(e + t));
-      }
-    }
-#pragma unroll
-    for (int t = 0; t < EPV; ++t) part[g * D + c * EPV + t] = acc[t];
-  }
-  __syncthreads();
-  for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    float res;
-    if (mean) {
-      float a1 = 0.f;
-      for (int g = 0; g < groups; ++g) a1 += part[g * D + d];
-      res = a1 / (float)bs;
-    } else {
-      float m = (r1 - r0 < bs) ? 0.f : -CUDART_INF_F;     // zero padding takes part in the max
-      for (int g = 0; g < groups; ++g) m = fmaxf(m, part[g * D + d]);
-      res = m;
-    }
-    pooled_q[((int64_t)bh * nb + blk) * D + d] = E::cvt(res);
-  }
+  const int blk = blockIdx.x, bh = blockIdx.y;
+  pool_query_block<DT, 16>(q + (int64_t)(bh / Hq) * qs.b + (int64_t)(bh % Hq) * qs.h, qs.s, pooled_q + ((int64_t)bh * nb + blk) * D, blk, pool_mode,
+                           S, D, bs, part, threadIdx.x, blockDim.x, [] { __syncthreads(); });
 }
 
 template <int DT>
