@@ -217,6 +217,9 @@ int pbs_select_blocks(const pbs_shape_t* shape, const void* pooled_q, const void
                       const int32_t* first_block, const pbs_options_t* options,
                       uint8_t* block_mask, float* block_scores, void* stream);
 
+/* Writes the 8 status words to pinned host memory that the device can address, in stream order. */
+int pbs_export_status(const int32_t* status, int32_t* host_words, void* stream);
+
 /* Stage 3a.  Per 256-query group, the compact list of 128-key tiles that any of its
  * query blocks selected (consumed by the tcgen05 attention kernel). */
 int pbs_build_tile_lists(const pbs_shape_t* shape, const uint8_t* block_mask,

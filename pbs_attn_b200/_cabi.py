@@ -6,6 +6,8 @@ compute backend: there is no CPU or PyTorch fallback, a missing library raises.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 
 # PBS_B200_LIB points at an alternative build of the same library (e.g. an instrumented one)
@@ -65,6 +67,7 @@ SIGNATURES = {
     "pbs_segment_permute": [_SH, _P, _P, _ST, _P, _ST, _P, _P, _P, _P, C.c_int32, _P, _P],
     "pbs_pool_queries": [_SH, _P, _ST, _P, C.c_int32, _P],
     "pbs_select_blocks": [_SH, _P, _P, _P, C.POINTER(Options), _P, _P, _P],
+    "pbs_export_status": [_P, _P, _P],
     "pbs_build_tile_lists": [_SH, _P, _P, _P, _P],
     "pbs_attn_fwd": [_SH, _P, _ST, _P, _P, _P, _P, _P, _P, _P, _ST, C.c_int32, _P, C.POINTER(OutReplicas), _P],
     "pbs_debug_set_select_impl": [C.c_int32],
@@ -105,6 +108,23 @@ def load():
         fn.argtypes = args
     _lib = lib
     return lib
+
+
+_host = None
+
+
+def load_host():
+    """The native host side of the common call (csrc/host_call.cpp), loaded once; raises RuntimeError if it was not built."""
+    global _host
+    if _host is None:
+        path = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "pbs_host.so")
+        if not os.path.exists(path):
+            raise RuntimeError(f"{path} is missing: build it with `python -m pbs_attn_b200.build`")
+        import torch  # noqa: F401  (the module links against its libraries)
+        loader = importlib.machinery.ExtensionFileLoader("pbs_host", path)
+        _host = importlib.util.module_from_spec(importlib.util.spec_from_loader("pbs_host", loader))
+        loader.exec_module(_host)
+    return _host
 
 
 class PbsError(RuntimeError):

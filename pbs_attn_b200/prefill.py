@@ -94,6 +94,7 @@ class Plan:
         self._status_next = 0
 
     _kv_left_out = False                    # the last whole-path call may have left perm_k / perm_v as they were
+    _native = None                          # the call object of csrc/host_call.cpp, which then keeps the pending status words
     _status_rows = _status_words = None     # views of the ring, made on first use: per-slot tensors and an array of ints
 
     # ------------------------------------------------------------------ helpers
@@ -108,7 +109,17 @@ class Plan:
         raise _cabi.PbsError(f"device-side error flags {list(words)}: a bounded wait in the attention kernel ran out "
                              f"(code {int(words[0])}); the output of that call is invalid")
 
+    def _go_native(self):
+        """The common call of this plan may run without Python (``_cabi.load_host().call``)."""
+        self._native = _cabi.load_host().attach(
+            C.addressof(self.shape), C.addressof(self.scratch), self._status_ring.data_ptr(), self.device.index,
+            C.cast(self.lib.pbs_prefill_fwd, C.c_void_p).value, C.cast(self.lib.pbs_export_status, C.c_void_p).value)
+
     def _inspect_landed_status(self, wait_all: bool = False):
+        if self._native is not None:
+            words = _cabi.load_host().inspect(self._native, wait_all)
+            if words is not None:
+                self._raise_status(words)
         while self._status_pending:
             ev, slot = self._status_pending[0]
             if wait_all or len(self._status_pending) >= _STATUS_SLOTS:
@@ -121,6 +132,8 @@ class Plan:
                 self._raise_status(self._status_words[8 * slot : 8 * slot + 8])
 
     def _queue_status_copy(self, stream):
+        if self._native is not None:
+            return _cabi.load_host().queue(self._native, stream.cuda_stream)
         if self._status_rows is None:
             ring = self._status_ring                        # the views live as long as the plan, and so does the ring
             self._status_words = (C.c_int32 * ring.numel()).from_address(ring.data_ptr())
@@ -229,7 +242,7 @@ class Plan:
     def run(self, q, k, v, out, opt: _cabi.Options):
         """The whole path.  Never synchronises: a device-side error of an EARLIER call (its status words
         have reached the host by now) is raised here; this call's own status is queued for the next."""
-        if self._status_pending:
+        if self._status_pending or self._native is not None:
             self._inspect_landed_status()
         with self._on_device():
             stream = torch.cuda.current_stream(self.device)
@@ -295,7 +308,16 @@ def get_plan(q: torch.Tensor, kv_heads: int, block_size: int, segment_size: int)
         while len(_PLANS) >= _MAX_PLANS:
             _PLANS.pop(next(iter(_PLANS)))
         plan = _PLANS[key] = Plan(B, Hq, kv_heads, S, D, block_size, segment_size, q.dtype, q.device)
+        plan._go_native()
     return plan
+
+
+def _common_call(q, k, v, block_size, segment_size, threshold, force_first, mean_pooling=0, own_segment=True):
+    """The call on a plan that exists, without Python in between; None for everything that the code below has to do."""
+    if not _PLANS:
+        return None
+    return _cabi.load_host().call(_PLANS, q, k, v, block_size, segment_size, threshold,
+                                  (1 if force_first else 0) | mean_pooling | (0 if own_segment else 4))
 
 
 def release_plans():
@@ -337,6 +359,11 @@ def permuted_block_sparse_attn_fwd(
         writes as well (buffers on peer GPUs of a head-sharded call, see ``peer_gather``).
     Runs on the current CUDA stream without synchronising.
     """
+    if (intermediates is None and out is None and out_replicas is None and causal and attn_impl == "auto"
+            and query_pool_mode == "mean" and key_pool_mode == "mean"):
+        result = _common_call(query_states, key_states, value_states, block_size, segment_size, threshold, force_select_first_block)
+        if result is not None:
+            return result
     batch_size, num_q_heads, q_len, head_dim = query_states.shape
     _, num_kv_heads, kv_len, _ = key_states.shape
     assert num_q_heads % num_kv_heads == 0
@@ -393,6 +420,11 @@ def MeanPooling_prefill(
     ``causal=False`` fails with the reference's own assertion: its ``select_blocks`` only supports
     causal selection (pbs_attn/src/utils.py:54), so the baseline never ran non-causally there either.
     """
+    if intermediates is None and causal is True and attn_impl == "auto":
+        result = _common_call(query_states, key_states, value_states, block_size, block_size, threshold, force_select_first_block,
+                              2, force_select_current_block)
+        if result is not None:
+            return result
     batch_size, num_q_heads, q_len, head_dim = query_states.shape
     _, num_kv_heads, kv_len, _ = key_states.shape
     assert num_q_heads % num_kv_heads == 0
