@@ -184,6 +184,11 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       : "r"(taddr)
       : "memory");
 }
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
@@ -508,27 +513,50 @@ __device__ __noinline__ Refs before_exp(Refs r, uint32_t ent, uint32_t tmem, uin
 // scales what and when.  A half-step k that finds a sum above kSumMost raises them: it waits for the P V of k - 1, which the old ones
 // belong to, publishes the new ones and scales O.  S_k is still in TMEM, and since P_k has not been handed over, neither P V of k nor of the
 // partner's k + 1 can start: O and P_{k+1} are its own.  P_{k+1} is always formed with the references before and then scaled.  Its warp reads
-// the epoch after it has seen its S: if that S is not there yet it will see the new epoch and scale by itself (scale_late).  Otherwise its
+// the epoch after it has seen its S: if that S is not there yet it will see the new epoch and scale by itself.  Otherwise its
 // progress says when it is through: with the old epoch its P is scaled here and its sum by itself once it sees the epoch; or it
 // waits for the P V of k to raise references of its own, and takes the new ones after that.
-// For a half-step that has seen another epoch or a sum above kSumMost: the references to form P again with; last: these stay.
-struct Verdict {
+// All of this is for half-steps that have seen another epoch or a sum above kSumMost; it forms and stores their P anew.
+struct Settled {
   Refs r;
-  bool last;
+  float sum;
 };
 __device__ __forceinline__ bool raised_just_now(uint32_t now, const Who& w, uint32_t sc) {   // epoch `now` is the work of half-step k - 1
   return *const_cast<const volatile uint32_t*>(&front().ctl.raised_at[now & 1u][w.i][w.wq]) + 1u == 2u * sc + w.hs;
 }
 template <int DT, int D>
-__device__ __noinline__ Verdict settle(Refs r, uint32_t tmem, uint32_t sc, bool first_entry, float scale_log2e) {
+__device__ __noinline__ Settled settle(Refs r, uint32_t tmem, uint32_t sc, bool first_entry, float scale_log2e) {
   const Who w = who();
   Bars& bars = front().bars;
   Ctl& ctl = front().ctl;
   const uint32_t fresh = r.epoch & kFresh;
   r.epoch &= ~kFresh;
-  auto verdict = [&](bool last) {
-    if (r.epoch != kGiveUp) r.epoch |= fresh;
-    return Verdict{r, last};
+  const uint32_t lanes = (uint32_t)(w.wq * 32) << 16, s_addr = tmem + lanes + 128 * w.i + 64 * w.hs;
+  auto given_up = [&]() {
+    r.epoch = kGiveUp;
+    return Settled{r, 0.f};
+  };
+  // P_k with the references in r, as the hot loop forms it; what is stored is scaled by alpha, the sum of the row is not.  Storing goes behind
+  // reading: 16 scores give 8 columns of P.
+  auto form = [&](bool store, float alpha) {
+    const float ref = r.ref == -CUDART_INF_F ? 0.f : r.ref;
+    const float2 sc2 = make_float2(scale_log2e, scale_log2e), nm2 = make_float2(-ref, -ref);
+    float2 acc2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll 1
+    for (int q = 0; q < 4; ++q) {
+      uint32_t sr[16], pk[8];
+      tmem_ld16(s_addr + 16 * q, sr);
+      tmem_wait_ld();
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const float2 x = __ffma2_rn(make_float2(__uint_as_float(sr[2 * c]), __uint_as_float(sr[2 * c + 1])), sc2, nm2);
+        pk[c] = PackP<DT>::pack(ex2(x.x), ex2(x.y));
+        PackP<DT>::add(acc2[c & 1], pk[c]);
+        if (alpha != 1.f) pk[c] = PackP<DT>::scale(pk[c], alpha);
+      }
+      if (store) tmem_st8(s_addr + 8 * q, pk);
+    }
+    return (acc2[0].x + acc2[0].y) + (acc2[1].x + acc2[1].y);
   };
   auto refs_of = [&](uint32_t epoch) { return *const_cast<const volatile float*>(&ctl.ref[epoch & 1u][w.i][w.row]); };
   auto take = [&](uint32_t epoch) {
@@ -537,21 +565,35 @@ __device__ __noinline__ Verdict settle(Refs r, uint32_t tmem, uint32_t sc, bool 
     r.ref = ref;
     r.epoch = epoch;
   };
-  const uint32_t now = *const_cast<const volatile uint32_t*>(&ctl.epoch[w.i][w.wq]);
-  if (__any_sync(0xffffffffu, now != r.epoch)) {
-    const bool just_now = raised_just_now(now, w, sc);
-    if (!just_now || now != r.epoch + 1u) {
-      take(just_now ? now - 1u : now);
-      return verdict(false);
+  bool late = false;                                       // half-step k - 1 raised the references; P_k is formed with the ones before
+  for (;;) {
+    const uint32_t now = *const_cast<const volatile uint32_t*>(&ctl.epoch[w.i][w.wq]);
+    if (!__any_sync(0xffffffffu, now != r.epoch)) break;
+    late = raised_just_now(now, w, sc);
+    if (late && now == r.epoch + 1u) break;
+    take(late ? now - 1u : now);
+  }
+  float sum = form(false, 1.f);
+  if (!__any_sync(0xffffffffu, !(sum <= kSumMost<DT>))) {
+    float alpha = 1.f;
+    const Refs formed = r;
+    if (late) {
+      refresh(r, w);
+      if (r.ref != formed.ref) alpha = ref_scale(formed.ref, r.ref);
     }
+    const Refs after_it = r;
+    r = formed;
+    sum = form(true, alpha) * alpha;
+    r = after_it;
+    r.epoch |= fresh;
+    return Settled{r, sum};
   }
   const uint32_t before = w.hs == 0 ? sc - 1u : sc, after = w.hs == 0 ? sc : sc + 1u;   // entries of half-steps k - 1 and k + 1
-  const uint32_t lanes = (uint32_t)(w.wq * 32) << 16;
-  const float top = row_max64(tmem + lanes + 128 * w.i + 64 * w.hs) * scale_log2e;
+  const float top = row_max64(s_addr) * scale_log2e;
   if (w.lane == 0) st_post(smem_u32(&ctl.post[w.i][w.hs][w.wq]), 3u * sc + kRaising, r.epoch);
   const bool have_o = !first_entry || w.hs == 1;
   if (have_o) {
-    if (!wait_bar_warp(smem_u32(&bars.o_full[w.i][w.hs ^ 1]), before & 1u, 10)) { r.epoch = kGiveUp; return verdict(true); }
+    if (!wait_bar_warp(smem_u32(&bars.o_full[w.i][w.hs ^ 1]), before & 1u, 10)) return given_up();
     tc_fence_after();
     refresh(r, w);
   }
@@ -573,31 +615,16 @@ __device__ __noinline__ Verdict settle(Refs r, uint32_t tmem, uint32_t sc, bool 
     if (__all_sync(0xffffffffu, mbar_try_wait(smem_u32(&bars.s_full[w.i][w.hs ^ 1]), after & 1u))) {
       // (a first half has met the second one of its entry already)
       uint2 theirs;
-      if (!wait_post(smem_u32(&ctl.post[w.i][w.hs ^ 1][w.wq]), 3u * after + (w.hs == 0 ? kRaising : kAtStart), theirs, 16)) {
-        r.epoch = kGiveUp;
-        return verdict(true);
-      }
+      if (!wait_post(smem_u32(&ctl.post[w.i][w.hs ^ 1][w.wq]), 3u * after + (w.hs == 0 ? kRaising : kAtStart), theirs, 16)) return given_up();
       if (theirs.x >= 3u * (after + 1u) && theirs.y != r.epoch) {
         tc_fence_after();
         scale_p<DT>(tmem + lanes + 128 * w.i + 64 * (w.hs ^ 1), alpha);
       }
     }
-    tmem_wait_st();
   }
-  return verdict(true);
-}
-// After half-step k - 1 raised the references that P_k was formed with: P_k, in TMEM, and the row's sum scaled.
-template <int DT>
-__device__ __noinline__ Refs scale_late(Refs r, uint32_t s_addr) {
-  const Who w = who();
-  const uint32_t fresh = r.epoch & kFresh;
-  r.epoch &= ~kFresh;
-  const float old = r.ref;
-  refresh(r, w);
-  tmem_wait_st();
-  scale_p<DT>(s_addr, r.ref == old ? 1.f : ref_scale(old, r.ref));
+  sum = form(true, 1.f);
   r.epoch |= fresh;
-  return r;
+  return Settled{r, sum};
 }
 
 // The n-th item of this CTA, for the roles that the producer feeds (a whole converged warp calls it).
@@ -906,50 +933,39 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
           for (int c = 0; c < 32; ++c) zero[c] = 0u;
           tmem_st32(s_addr, zero);
         } else {
-          // All of P_h is formed before any of it goes back over the first 32 columns of S_h, so that S_h is still there
-          // for another pass when the references turn out to be stale or too low.
+          // All of P_h is formed before any of it goes back over the first 32 columns of S_h, so that S_h is still there when
+          // the references turn out to be stale or too low.
           uint32_t pk[32], epoch_now;
-          for (bool last = false;;) {
-            const float2 sc2 = make_float2(p.scale_log2e, p.scale_log2e);
-            const float ref = r.ref == -CUDART_INF_F ? 0.f : r.ref;
-            const float2 nm2 = make_float2(-ref, -ref);
-            float2 acc2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+          const float2 sc2 = make_float2(p.scale_log2e, p.scale_log2e);
+          const float ref = r.ref == -CUDART_INF_F ? 0.f : r.ref;
+          const float2 nm2 = make_float2(-ref, -ref);
+          float2 acc2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              uint32_t sr[32];
-              tmem_ld32(s_addr + 32 * q, sr);
-              // (the epoch is read after S is there: see settle)
-              if (q == 0) asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(epoch_now) : "r"(smem_u32(&ctl->epoch[i][wq])) : "memory");
-              tmem_wait_ld();
-              float (&v)[32] = *reinterpret_cast<float (*)[32]>(&sr[0]);
+          for (int q = 0; q < 2; ++q) {
+            uint32_t sr[32];
+            tmem_ld32(s_addr + 32 * q, sr);
+            // (the epoch is read after S is there: see settle)
+            if (q == 0) asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(epoch_now) : "r"(smem_u32(&ctl->epoch[i][wq])) : "memory");
+            tmem_wait_ld();
+            float (&v)[32] = *reinterpret_cast<float (*)[32]>(&sr[0]);
 #pragma unroll
-              for (int c = 0; c < 16; ++c) {
-                const float2 x = __ffma2_rn(make_float2(v[2 * c], v[2 * c + 1]), sc2, nm2);
-                const float2 ex = make_float2(ex2(x.x), ex2(x.y));
-                pk[16 * q + c] = PackP<DT>::pack(ex.x, ex.y);
-                PackP<DT>::add(acc2[c & 1], pk[16 * q + c]);
-              }
+            for (int c = 0; c < 16; ++c) {
+              const float2 x = __ffma2_rn(make_float2(v[2 * c], v[2 * c + 1]), sc2, nm2);
+              const float2 ex = make_float2(ex2(x.x), ex2(x.y));
+              pk[16 * q + c] = PackP<DT>::pack(ex.x, ex.y);
+              PackP<DT>::add(acc2[c & 1], pk[16 * q + c]);
             }
-            sum = (acc2[0].x + acc2[0].y) + (acc2[1].x + acc2[1].y);
-            const bool big = !(sum <= kSumMost<DT>);
-            if (last || !__any_sync(0xffffffffu, epoch_now != (r.epoch & ~kFresh) || big)) {
-              tmem_st32(s_addr, pk);
-              break;
-            }
-            if (epoch_now == (r.epoch & ~kFresh) + 1u && raised_just_now(epoch_now, who(), sc) && !__any_sync(0xffffffffu, big)) {
-              tmem_st32(s_addr, pk);
-              const float old = r.ref;
-              r = scale_late<DT>(r, s_addr);
-              if (r.ref != old) sum *= ref_scale(old, r.ref);
-              break;
-            }
-            const Verdict verdict = settle<DT, D>(r, tmem, sc, sc == sc0, p.scale_log2e);
-            r = verdict.r;
+          }
+          sum = (acc2[0].x + acc2[0].y) + (acc2[1].x + acc2[1].y);
+          if (!__any_sync(0xffffffffu, epoch_now != (r.epoch & ~kFresh) || !(sum <= kSumMost<DT>))) {
+            tmem_st32(s_addr, pk);
+          } else {
+            const Settled settled = settle<DT, D>(r, tmem, sc, sc == sc0, p.scale_log2e);
+            r = settled.r;
+            sum = settled.sum;
             ok = r.epoch != kGiveUp;
             if (!ok) break;
-            last = verdict.last;
           }
-          if (!ok) break;
         }
         tmem_wait_st();
         tc_fence_before();
