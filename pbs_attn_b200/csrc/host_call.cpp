@@ -14,6 +14,7 @@
 #include <torch/csrc/utils/object_ptr.h>
 
 #include <cstdlib>
+#include <vector>
 
 #include "../../include/pbs_b200.h"
 
@@ -29,7 +30,7 @@ using ExportFn = decltype(&pbs_export_status);
 struct Call {
   const pbs_shape_t* shape;
   const pbs_scratch_t* scratch;
-  int32_t* ring;                       // pinned, kSlots x 8
+  int32_t* ring;                       // pinned, kSlots x 8, from the pool below
   int device;
   PrefillFn prefill;
   ExportFn export_status;
@@ -39,24 +40,50 @@ struct Call {
 
 Call* get(PyObject* capsule) { return static_cast<Call*>(PyCapsule_GetPointer(capsule, kName)); }
 
-void destroy(PyObject* capsule) {
-  Call* c = static_cast<Call*>(PyCapsule_GetPointer(capsule, kName));
-  for (int i = 0; i < c->made; ++i) (void)cudaEventDestroy(c->landed[i]);
-  delete c;
+// Rings of calls that are gone, and calls whose plan is gone while the device may still write to their rings.  The interpreter's lock guards
+// both; there are never more of them than there were plans at a time.
+std::vector<int32_t*> free_rings;
+std::vector<Call*> leaving;
+
+// Recycles what has left and landed.
+void sweep() {
+  size_t kept = 0;
+  for (Call* c : leaving) {
+    while (c->count > 0 && cudaEventQuery(c->landed[c->first]) != cudaErrorNotReady) {
+      c->first = (c->first + 1) % kSlots;
+      --c->count;
+    }
+    if (c->count > 0) {
+      leaving[kept++] = c;
+      continue;
+    }
+    for (int i = 0; i < c->made; ++i) (void)cudaEventDestroy(c->landed[i]);
+    free_rings.push_back(c->ring);
+    delete c;
+  }
+  leaving.resize(kept);
 }
+
+void destroy(PyObject* capsule) { leaving.push_back(static_cast<Call*>(PyCapsule_GetPointer(capsule, kName))); }
 
 bool capturing(cudaStream_t st) {
   cudaStreamCaptureStatus s;
   return cudaStreamIsCapturing(st, &s) != cudaSuccess || s != cudaStreamCaptureStatusNone;
 }
 
-// Sends the status words of the call just enqueued to its slot of the ring.  A captured call sends them at each replay, at
-// times unknown here, so nobody waits for them.
-cudaError_t queue_status(Call* c, cudaStream_t st) {
+// Sends the status words of the call just enqueued to its slot of the ring.  Not those of a captured call: it is replayed at times unknown
+// here, perhaps after the plan is gone (check_status reads the device's words).  by_copy: for calls that go through Python, the
+// host-tensor call's among them, whose kernels would wait behind the copies out with a store to the host (16384 tokens 4.95 ms so, 5.19 with
+// the kernel).
+cudaError_t queue_status(Call* c, cudaStream_t st, bool by_copy) {
+  if (capturing(st)) return cudaSuccess;
   if (c->count >= kSlots) return cudaSuccess;              // several threads on one plan: this call goes unwatched
   const int slot = c->next;
-  cudaError_t e = c->export_status(static_cast<const int32_t*>(c->scratch->status), c->ring + 8 * slot, st) == PBS_OK ? cudaSuccess : cudaErrorLaunchFailure;
-  if (e != cudaSuccess || capturing(st)) return e;
+  const int32_t* words = static_cast<const int32_t*>(c->scratch->status);
+  cudaError_t e = cudaSuccess;
+  if (by_copy) e = cudaMemcpyAsync(c->ring + 8 * slot, words, 8 * sizeof(int32_t), cudaMemcpyDeviceToHost, st);
+  else if (c->export_status(words, c->ring + 8 * slot, st) != PBS_OK) e = cudaErrorLaunchFailure;
+  if (e != cudaSuccess) return e;
   while (c->made <= slot) {
     if ((e = cudaEventCreateWithFlags(&c->landed[c->made], cudaEventDisableTiming)) != cudaSuccess) return e;
     ++c->made;
@@ -73,10 +100,11 @@ int landed_error(Call* c, bool wait_all) {
   while (c->count > 0) {
     cudaEvent_t ev = c->landed[c->first];
     if (wait_all || c->count >= kSlots) {
+      const int slot = c->first;
       Py_BEGIN_ALLOW_THREADS
       (void)cudaEventSynchronize(ev);
       Py_END_ALLOW_THREADS
-      if (c->count == 0) return -1;                        // another thread has been here
+      if (c->count == 0 || c->first != slot) continue;     // another thread has been here
     } else if (cudaEventQuery(ev) != cudaSuccess) {
       break;                                               // not there yet; an error of the device shows at the next library call
     }
@@ -88,10 +116,19 @@ int landed_error(Call* c, bool wait_all) {
 }
 
 PyObject* py_attach(PyObject*, PyObject* args) {
-  unsigned long long shape, scratch, ring, fn, fn2;
+  unsigned long long shape, scratch, fn, fn2;
   int device;
-  if (!PyArg_ParseTuple(args, "KKKiKK", &shape, &scratch, &ring, &device, &fn, &fn2)) return nullptr;
-  Call* c = new Call{reinterpret_cast<const pbs_shape_t*>(shape), reinterpret_cast<const pbs_scratch_t*>(scratch), reinterpret_cast<int32_t*>(ring),
+  if (!PyArg_ParseTuple(args, "KKiKK", &shape, &scratch, &device, &fn, &fn2)) return nullptr;
+  sweep();
+  int32_t* ring = nullptr;
+  if (free_rings.empty()) {
+    const cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&ring), kSlots * 8 * sizeof(int32_t), cudaHostAllocPortable);
+    if (e != cudaSuccess) return PyErr_Format(PyExc_RuntimeError, "pinned memory for the status words: %s", cudaGetErrorString(e));
+  } else {
+    ring = free_rings.back();
+    free_rings.pop_back();
+  }
+  Call* c = new Call{reinterpret_cast<const pbs_shape_t*>(shape), reinterpret_cast<const pbs_scratch_t*>(scratch), ring,
                      device, reinterpret_cast<PrefillFn>(fn), reinterpret_cast<ExportFn>(fn2), {}, 0, 0, 0, 0};
   return PyCapsule_New(c, kName, destroy);
 }
@@ -120,7 +157,7 @@ PyObject* py_queue(PyObject*, PyObject* args) {
   if (!PyArg_ParseTuple(args, "OK", &capsule, &stream)) return nullptr;
   Call* c = get(capsule);
   if (!c) return nullptr;
-  const cudaError_t e = queue_status(c, reinterpret_cast<cudaStream_t>(stream));
+  const cudaError_t e = queue_status(c, reinterpret_cast<cudaStream_t>(stream), true);
   if (e != cudaSuccess) return PyErr_Format(PyExc_RuntimeError, "copy of the status words: %s", cudaGetErrorString(e));
   Py_RETURN_NONE;
 }
@@ -198,14 +235,14 @@ PyObject* py_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Py_END_ALLOW_THREADS
   if (rc != PBS_OK) Py_RETURN_NONE;                        // refused before anything was enqueued: Python says why
   if (PyObject_SetAttrString(plan, "_kv_left_out", in_place ? Py_True : Py_False) < 0) return nullptr;
-  e = queue_status(c, st);
+  e = queue_status(c, st, false);
   if (e != cudaSuccess) return PyErr_Format(PyExc_RuntimeError, "copy of the status words: %s", cudaGetErrorString(e));
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
 }
 
 PyMethodDef methods[] = {
-    {"attach", py_attach, METH_VARARGS, "attach(shape, scratch, ring, device, prefill, export_status): addresses of a plan's buffers -> its call object"},
+    {"attach", py_attach, METH_VARARGS, "attach(shape, scratch, device, prefill, export_status): addresses of a plan's buffers -> its call object"},
     {"inspect", py_inspect, METH_VARARGS, "inspect(call, wait_all): None or the status words of a failed call"},
     {"queue", py_queue, METH_VARARGS, "queue(call, stream): send the status words of the call just enqueued"},
     {"call", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_call)), METH_FASTCALL,

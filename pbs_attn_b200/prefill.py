@@ -112,7 +112,7 @@ class Plan:
     def _go_native(self):
         """The common call of this plan may run without Python (``_cabi.load_host().call``)."""
         self._native = _cabi.load_host().attach(
-            C.addressof(self.shape), C.addressof(self.scratch), self._status_ring.data_ptr(), self.device.index,
+            C.addressof(self.shape), C.addressof(self.scratch), self.device.index,
             C.cast(self.lib.pbs_prefill_fwd, C.c_void_p).value, C.cast(self.lib.pbs_export_status, C.c_void_p).value)
 
     def _inspect_landed_status(self, wait_all: bool = False):

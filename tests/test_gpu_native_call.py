@@ -58,6 +58,18 @@ def test_left_to_python():
         permuted_block_sparse_attn_fwd(q, k, v, 64, 96, 0.8, True)
 
 
+def test_plans_that_leave_with_calls_in_flight():
+    from pbs_attn_b200.prefill import permuted_block_sparse_attn_fwd, release_plans
+    cases = [_inputs(tokens=t, seed=t) for t in (200, 330, 450, 700)]
+    release_plans()
+    want = [permuted_block_sparse_attn_fwd(*c, 64, 128, 0.8, True) for c in cases]
+    for _ in range(5):                                     # four shapes, two plans kept: every call evicts one
+        got = [[permuted_block_sparse_attn_fwd(*c, 64, 128, 0.8, True) for _ in range(3)][-1] for c in cases]
+    release_plans()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(want, got))
+
+
 def test_captured_call_replays():
     from pbs_attn_b200.prefill import permuted_block_sparse_attn_fwd, release_plans
     release_plans()
