@@ -34,7 +34,7 @@
 // tokens 7245 -> 6816, 32768 sparse tokens 4325 -> 3693, four heads at 131072 tokens 14255 -> 13800 (power cap).
 // Three things make four warpgroups pay, each of which alone decides between a gain and a loss:
 //  - the warps of the two halves exchange nothing from step to step.  A row's reference is not its running maximum
-//    but what its first tile gave; it is raised only when a half-step's sum leaves kSumMost, which for bf16 (the range of fp32) hardly
+//    but what its first tile gave; it is raised only when a half-step's sum leaves kSumMost, which hardly
 //    ever happens.  All of that protocol (settle, before_exp) is out of line.  With a check between the halves in every
 //    half-step (a poll, an order of the hand-overs) the kernel was slower than before: 3200 to 3500 cycles a step against 2850.
 //  - registers: 96 a thread at 640 threads, 104 after the issuing warps have given some up.  S is read in two parts of 32
@@ -57,10 +57,16 @@ constexpr int kThreads = 640;
 constexpr int kRing = 2;                  // stages of a V tile and the next list entry's K tile
 constexpr int kSched = 4;                 // items the producer may be ahead of the slowest role
 constexpr uint32_t kTmemCols = 512;
-// A half-step's probabilities are taken as they are while their sum per row is no larger than this: the reference of the
-// exponents need not be the row maximum, only near enough that nothing leaves the range of the 16-bit type (fp16: 65504).
-template <int DT> constexpr float kSumMost = DT == PBS_FP16 ? 0x1p15f : 0x1p60f;
-template <int DT> constexpr float kUpLeast = DT == PBS_FP16 ? 9.f : 54.f;   // log2(kSumMost / 64): a larger sum of 64 has a score above it
+// A half-step's probabilities are taken as they are while their sum per row is no larger than this: the reference of the exponents need
+// not be the row maximum, only near enough that nothing leaves its range.  For fp16 that is P's (65504).  For bf16 it is what V, which may be
+// as large as fp32's numbers, leaves for O, the sum of P V before it is divided: with 2^8 |O| is at most 2^8 |V| a half-step.
+// References that are raised often cost much (8192 tokens of head_dim 64 478 us a call, 577 with this limit and references at the
+// maximum), so bf16's lie kLift above the maximum that they are taken from: scores may still rise by 2^20 (sum of 64), at
+// which the rare path was as rare as with 2^60; at 2^14 32768 sparse tokens took 4579 us against 4385.  P and O of a row are
+// then 2^-12 of what they could be, which leaves all of |V| down to fp32's least normal number its 8 bits in O.
+template <int DT> constexpr float kSumMost = DT == PBS_FP16 ? 0x1p15f : 0x1p8f;
+template <int DT> constexpr float kUpLeast = DT == PBS_FP16 ? 9.f : 2.f;    // log2(kSumMost / 64): a larger sum of 64 has a score above it
+template <int DT> constexpr float kLift = DT == PBS_FP16 ? 0.f : 12.f;
 // Registers a thread: the four warps that only issue give up part of what the launch has.
 constexpr int kRegsLaunch = 96, kRegsIssue = 64, kRegsSoftmax = 104;
 static_assert(128 * kRegsIssue + 512 * kRegsSoftmax <= kThreads * kRegsLaunch, "the shares must fit what the launch has");
@@ -481,7 +487,8 @@ __device__ __forceinline__ void refresh(Refs& r, const Who& w) {
 }
 
 // Before the exponentials of a half-step whose keys are masked by position, or while some row has no reference: its first one is
-// its largest score in both halves of the first tile that has one, so that the two warps meet here.
+// kLift above its largest score in both halves of the first tile that has one, so that the two warps meet here.
+template <int DT>
 __device__ __noinline__ Refs before_exp(Refs r, uint32_t ent, uint32_t tmem, uint32_t sc, bool none, bool first_entry, int qpos, float scale_log2e) {
   const Who w = who();
   Ctl& ctl = front().ctl;
@@ -504,7 +511,7 @@ __device__ __noinline__ Refs before_exp(Refs r, uint32_t ent, uint32_t tmem, uin
   if (w.lane == 0) *starts = *starts + 1u;
   __syncwarp();
   if (!first_entry) refresh(r, w);
-  if (r.ref == -CUDART_INF_F) r.ref = fmaxf(mine, both[128 * (w.hs ^ 1)]);
+  if (r.ref == -CUDART_INF_F) r.ref = fmaxf(mine, both[128 * (w.hs ^ 1)]) + kLift<DT>;
   if (__any_sync(0xffffffffu, r.ref == -CUDART_INF_F)) r.epoch |= kFresh;
   return r;
 }
@@ -600,7 +607,7 @@ __device__ __noinline__ Settled settle(Refs r, uint32_t tmem, uint32_t sc, bool 
   const bool up = top > r.ref + kUpLeast<DT>;
   if (__any_sync(0xffffffffu, up)) {
     const float old = r.ref;
-    if (up) r.ref += ceilf(top - r.ref);
+    if (up) r.ref += ceilf(top - r.ref) + kLift<DT>;
     const float alpha = up ? ref_scale(old, r.ref) : 1.f;
     r.l *= alpha;
     ++r.epoch;
@@ -922,7 +929,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         if (!ok) break;
         tc_fence_after();
         if (cold) {
-          r = before_exp(r, ent, tmem, sc, none, sc == sc0, r0 + row, p.scale_log2e);
+          r = before_exp<DT>(r, ent, tmem, sc, none, sc == sc0, r0 + row, p.scale_log2e);
           ok = r.epoch != kGiveUp;
           if (!ok) break;
         }
