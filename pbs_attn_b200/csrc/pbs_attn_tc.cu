@@ -469,7 +469,8 @@ __device__ __forceinline__ Who who() {
   return Who{w >> 3, (w >> 2) & 1, w & 3, lane, (w & 3) * 32 + lane};
 }
 
-// 2^(from - to) for references of a row, `to` the later one: they are raised by whole numbers, so this is a power of two.
+// 2^(from - to) for references of a row, `to` the later one: they are raised by whole numbers, so this is a power of two, or by more than
+// 127, and then it is 0.
 __device__ __forceinline__ float ref_scale(float from, float to) {
   const float n = rintf(from - to);
   return n >= -126.f ? __int_as_float(((int)fminf(n, 0.f) + 127) << 23) : 0.f;
@@ -517,7 +518,8 @@ __device__ __noinline__ Refs before_exp(Refs r, uint32_t ent, uint32_t tmem, uin
 }
 
 // References are raised by whole numbers, so that all is scaled by powers of two, exactly, and the result does not depend on who
-// scales what and when.  A half-step k that finds a sum above kSumMost raises them: it waits for the P V of k - 1, which the old ones
+// scales what and when.  Only where nothing is left of what was, by more than 127, to the maximum itself: from references of 10^10 (keys
+// that a caller has pushed far down) a whole number leads to within a unit of 1024, not to the maximum.  A half-step k that finds a sum above kSumMost raises them: it waits for the P V of k - 1, which the old ones
 // belong to, publishes the new ones and scales O.  S_k is still in TMEM, and since P_k has not been handed over, neither P V of k nor of the
 // partner's k + 1 can start: O and P_{k+1} are its own.  P_{k+1} is always formed with the references before and then scaled.  Its warp reads
 // the epoch after it has seen its S: if that S is not there yet it will see the new epoch and scale by itself.  Otherwise its
@@ -607,7 +609,7 @@ __device__ __noinline__ Settled settle(Refs r, uint32_t tmem, uint32_t sc, bool 
   const bool up = top > r.ref + kUpLeast<DT>;
   if (__any_sync(0xffffffffu, up)) {
     const float old = r.ref;
-    if (up) r.ref += ceilf(top - r.ref) + kLift<DT>;
+    if (up) r.ref = (top - r.ref > 127.f ? top : r.ref + ceilf(top - r.ref)) + kLift<DT>;
     const float alpha = up ? ref_scale(old, r.ref) : 1.f;
     r.l *= alpha;
     ++r.epoch;

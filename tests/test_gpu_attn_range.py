@@ -46,3 +46,20 @@ def test_large_and_small_values_under_rising_scores(rise, exponent):
     bound = (2.0 ** -8 + 2.0 ** -10 + 2.0 ** -14) * scale + 2.0 ** -8 * want.abs()
     assert torch.isfinite(got).all()
     assert ((got - want).abs() <= bound).all(), float(((got - want).abs() / bound).max())
+
+
+@pytest.mark.parametrize("first", [1e4, 1e7, 1e10])
+@pytest.mark.parametrize("level", [-3.0, 0.0, 3.0])
+def test_first_keys_far_below_the_others(first, level):
+    """The first tile's scores lie `first` (log2 units) below zero, all others near 392 * level / 3: the reference has to reach these."""
+    g = torch.Generator().manual_seed(6)
+    q, k, v = (torch.randn(S, D, generator=g) for _ in range(3))
+    q[:, 0] = 2.0 ** 10
+    k[:, 0] = level
+    k[:128, 0] = -first / 2.0 ** 10 * D ** 0.5 / 1.4426950408889634
+    q, k, v = (t.bfloat16() for t in (q, k, v))
+    got = _attend(q, k, v)[128:]                           # (the rows before see nothing else)
+    want, scale = (t[128:] for t in _exact(q, k, v))
+    # as above: scores of magnitudes below 2^10
+    bound = (2.0 ** -8 + 2.0 ** -10 + 2.0 ** -14) * scale + 2.0 ** -8 * want.abs()
+    assert ((got - want).abs() <= bound).all(), float(((got - want).abs() / bound).max())
