@@ -476,9 +476,9 @@ __device__ __forceinline__ float ref_scale(float from, float to) {
   return n >= -126.f ? __int_as_float(((int)fminf(n, 0.f) + 127) << 23) : 0.f;
 }
 
-// Takes over references that the partner warp has raised.
-__device__ __forceinline__ void refresh(Refs& r, const Who& w) {
-  const uint32_t now = *const_cast<const volatile uint32_t*>(&front().ctl.epoch[w.i][w.wq]);
+// Takes over references that the partner warp has raised, up to epoch `now`.
+__device__ __forceinline__ uint32_t epoch_of(const Who& w) { return *const_cast<const volatile uint32_t*>(&front().ctl.epoch[w.i][w.wq]); }
+__device__ __forceinline__ void refresh(Refs& r, const Who& w, uint32_t now) {
   if (__any_sync(0xffffffffu, now != r.epoch)) {
     const float ref = *const_cast<const volatile float*>(&front().ctl.ref[now & 1u][w.i][w.row]);
     if (ref != r.ref && r.l > 0.f) r.l *= ref_scale(r.ref, ref);
@@ -496,8 +496,12 @@ __device__ __noinline__ Refs before_exp(Refs r, uint32_t ent, uint32_t tmem, uin
   const uint32_t s_addr = tmem + ((uint32_t)(w.wq * 32) << 16) + 128 * w.i + 64 * w.hs;
   if (!none && (ent & (1u << (18 + w.i)))) mask_half(s_addr, front().kidx[(threadIdx.x >> 5) - 4], qpos);
   if (!(r.epoch & kFresh)) return r;
-  // An item's first S was issued after all of the item before: nobody raises anything until both are past this meeting.
-  r.epoch = first_entry ? *const_cast<volatile uint32_t*>(&ctl.epoch[w.i][w.wq]) : r.epoch & ~kFresh;
+  // An item's first S was issued after all of the item before: nobody raises anything until both are past this meeting.  In a later entry
+  // the first half may raise references in this very entry once it is past the meeting: what the second half takes over here is of before
+  // that, so that its P is formed with the same references whether it is seen or not (settle); the first half needs all that the second has
+  // raised in the entry before, which is complete when they meet.
+  uint32_t epoch = epoch_of(w);
+  r.epoch = first_entry ? epoch : r.epoch & ~kFresh;
   const float mine = none ? -CUDART_INF_F : row_max64(s_addr) * scale_log2e;
   if (w.lane == 0) st_post(smem_u32(&ctl.post[w.i][w.hs][w.wq]), 3u * sc + kAtStart, 0u);
   volatile float* both = &ctl.smax[sc & 1u][w.i][0][w.row];
@@ -511,7 +515,8 @@ __device__ __noinline__ Refs before_exp(Refs r, uint32_t ent, uint32_t tmem, uin
   __syncwarp();
   if (w.lane == 0) *starts = *starts + 1u;
   __syncwarp();
-  if (!first_entry) refresh(r, w);
+  if (w.hs == 0) epoch = epoch_of(w);
+  if (!first_entry) refresh(r, w, epoch);
   if (r.ref == -CUDART_INF_F) r.ref = fmaxf(mine, both[128 * (w.hs ^ 1)]) + kLift<DT>;
   if (__any_sync(0xffffffffu, r.ref == -CUDART_INF_F)) r.epoch |= kFresh;
   return r;
@@ -576,7 +581,7 @@ __device__ __noinline__ Settled settle(Refs r, uint32_t tmem, uint32_t sc, bool 
   };
   bool late = false;                                       // half-step k - 1 raised the references; P_k is formed with the ones before
   for (;;) {
-    const uint32_t now = *const_cast<const volatile uint32_t*>(&ctl.epoch[w.i][w.wq]);
+    const uint32_t now = epoch_of(w);
     if (!__any_sync(0xffffffffu, now != r.epoch)) break;
     late = raised_just_now(now, w, sc);
     if (late && now == r.epoch + 1u) break;
@@ -587,7 +592,7 @@ __device__ __noinline__ Settled settle(Refs r, uint32_t tmem, uint32_t sc, bool 
     float alpha = 1.f;
     const Refs formed = r;
     if (late) {
-      refresh(r, w);
+      refresh(r, w, epoch_of(w));
       if (r.ref != formed.ref) alpha = ref_scale(formed.ref, r.ref);
     }
     const Refs after_it = r;
@@ -604,7 +609,7 @@ __device__ __noinline__ Settled settle(Refs r, uint32_t tmem, uint32_t sc, bool 
   if (have_o) {
     if (!wait_bar_warp(smem_u32(&bars.o_full[w.i][w.hs ^ 1]), before & 1u, 10)) return given_up();
     tc_fence_after();
-    refresh(r, w);
+    refresh(r, w, epoch_of(w));
   }
   const bool up = top > r.ref + kUpLeast<DT>;
   if (__any_sync(0xffffffffu, up)) {
@@ -1003,7 +1008,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         ++sums;
         // either half may have raised the references after the other's last step
         r.epoch &= ~kFresh;
-        refresh(r, who());
+        refresh(r, who(), epoch_of(who()));
         const float l1 = *(volatile float*)&ctl->lsum[i][row], ref1 = *(volatile float*)&ctl->lref[i][row];
         r.l += ref1 == r.ref || l1 == 0.f ? l1 : l1 * ref_scale(ref1, r.ref);
       }
