@@ -36,12 +36,14 @@ struct Call {
   ExportFn export_status;
   cudaEvent_t landed[kSlots];
   int made, first, count, next;        // events created; pending slots: first .. first + count - 1
+  int told;                            // so many of these, the oldest, are no longer looked at: an error among them has been raised
+  bool unwatched;                      // words are on their way to the ring that no event tells of
 };
 
 Call* get(PyObject* capsule) { return static_cast<Call*>(PyCapsule_GetPointer(capsule, kName)); }
 
 // Rings of calls that are gone, and calls whose plan is gone while the device may still write to their rings.  The interpreter's lock guards
-// both; there are never more of them than there were plans at a time.
+// both; there are never more of them than there were plans at a time and plans that left with calls in flight.
 std::vector<int32_t*> free_rings;
 std::vector<Call*> leaving;
 
@@ -58,7 +60,7 @@ void sweep() {
       continue;
     }
     for (int i = 0; i < c->made; ++i) (void)cudaEventDestroy(c->landed[i]);
-    free_rings.push_back(c->ring);
+    if (!c->unwatched) free_rings.push_back(c->ring);
     delete c;
   }
   leaving.resize(kept);
@@ -81,14 +83,17 @@ cudaError_t queue_status(Call* c, cudaStream_t st, bool by_copy) {
   const int slot = c->next;
   const int32_t* words = static_cast<const int32_t*>(c->scratch->status);
   cudaError_t e = cudaSuccess;
-  if (by_copy) e = cudaMemcpyAsync(c->ring + 8 * slot, words, 8 * sizeof(int32_t), cudaMemcpyDeviceToHost, st);
-  else if (c->export_status(words, c->ring + 8 * slot, st) != PBS_OK) e = cudaErrorLaunchFailure;
-  if (e != cudaSuccess) return e;
   while (c->made <= slot) {
     if ((e = cudaEventCreateWithFlags(&c->landed[c->made], cudaEventDisableTiming)) != cudaSuccess) return e;
     ++c->made;
   }
-  if ((e = cudaEventRecord(c->landed[slot], st)) != cudaSuccess) return e;
+  if (by_copy) e = cudaMemcpyAsync(c->ring + 8 * slot, words, 8 * sizeof(int32_t), cudaMemcpyDeviceToHost, st);
+  else if (c->export_status(words, c->ring + 8 * slot, st) != PBS_OK) e = cudaErrorLaunchFailure;
+  if (e != cudaSuccess) return e;
+  if ((e = cudaEventRecord(c->landed[slot], st)) != cudaSuccess) {
+    c->unwatched = true;
+    return e;
+  }
   c->next = (slot + 1) % kSlots;
   ++c->count;
   return cudaSuccess;
@@ -108,7 +113,8 @@ int landed_error(Call* c, bool wait_all) {
     } else if (cudaEventQuery(ev) != cudaSuccess) {
       break;                                               // not there yet; an error of the device shows at the next library call
     }
-    if (*const_cast<volatile int32_t*>(c->ring + 8 * c->first) != 0) return c->first;
+    if (c->told > 0) --c->told;
+    else if (*const_cast<volatile int32_t*>(c->ring + 8 * c->first) != 0) return c->first;
     c->first = (c->first + 1) % kSlots;
     --c->count;
   }
@@ -129,11 +135,12 @@ PyObject* py_attach(PyObject*, PyObject* args) {
     free_rings.pop_back();
   }
   Call* c = new Call{reinterpret_cast<const pbs_shape_t*>(shape), reinterpret_cast<const pbs_scratch_t*>(scratch), ring,
-                     device, reinterpret_cast<PrefillFn>(fn), reinterpret_cast<ExportFn>(fn2), {}, 0, 0, 0, 0};
+                     device, reinterpret_cast<PrefillFn>(fn), reinterpret_cast<ExportFn>(fn2), {}, 0, 0, 0, 0, 0, false};
   return PyCapsule_New(c, kName, destroy);
 }
 
-// inspect(call, wait_all): None, or the status words of a call that failed (all pending ones are then forgotten)
+// inspect(call, wait_all): None, or the status words of a call that failed (what all pending ones report is then not looked at any more; their
+// slots stay taken until the words have landed)
 PyObject* py_inspect(PyObject*, PyObject* args) {
   PyObject* capsule;
   int wait_all;
@@ -143,8 +150,7 @@ PyObject* py_inspect(PyObject*, PyObject* args) {
   if (!wait_all && capturing(c10::cuda::getCurrentCUDAStream(c->device).stream())) Py_RETURN_NONE;   // an event query would end the capture
   const int slot = landed_error(c, wait_all != 0);
   if (slot < 0) Py_RETURN_NONE;
-  c->count = 0;
-  c->first = c->next;
+  c->told = c->count;
   PyObject* words = PyList_New(8);
   for (int i = 0; words && i < 8; ++i) PyList_SET_ITEM(words, i, PyLong_FromLong(c->ring[8 * slot + i]));
   return words;
