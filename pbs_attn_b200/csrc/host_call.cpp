@@ -121,10 +121,20 @@ int landed_error(Call* c, bool wait_all) {
   return -1;
 }
 
+// A plan may be made while its stream is captured: what is done here belongs to no graph and must not end the capture.
+struct Relaxed {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  Relaxed() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~Relaxed() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 PyObject* py_attach(PyObject*, PyObject* args) {
+  HANDLE_TH_ERRORS
   unsigned long long shape, scratch, fn, fn2;
   int device;
   if (!PyArg_ParseTuple(args, "KKiKK", &shape, &scratch, &device, &fn, &fn2)) return nullptr;
+  const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));   // pinned memory brings up the current device, which may be another one
+  const Relaxed relaxed;
   sweep();
   int32_t* ring = nullptr;
   if (free_rings.empty()) {
@@ -137,6 +147,7 @@ PyObject* py_attach(PyObject*, PyObject* args) {
   Call* c = new Call{reinterpret_cast<const pbs_shape_t*>(shape), reinterpret_cast<const pbs_scratch_t*>(scratch), ring,
                      device, reinterpret_cast<PrefillFn>(fn), reinterpret_cast<ExportFn>(fn2), {}, 0, 0, 0, 0, 0, false};
   return PyCapsule_New(c, kName, destroy);
+  END_HANDLE_TH_ERRORS
 }
 
 // inspect(call, wait_all): None, or the status words of a call that failed (what all pending ones report is then not looked at any more; their
