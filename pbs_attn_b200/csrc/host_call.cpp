@@ -22,6 +22,7 @@ namespace {
 
 constexpr int kSlots = 16;             // calls whose status words may be in flight to the host at once
 constexpr const char* kName = "pbs_attn_b200.call";
+const cudaStream_t kNoStream = reinterpret_cast<cudaStream_t>(~uintptr_t{0});
 
 using PrefillFn = decltype(&pbs_prefill_fwd);
 using ExportFn = decltype(&pbs_export_status);
@@ -37,6 +38,7 @@ struct Call {
   cudaEvent_t landed[kSlots];
   int made, first, count, next;        // events created; pending slots: first .. first + count - 1
   int told;                            // so many of these, the oldest, are no longer looked at: an error among them has been raised
+  cudaStream_t last;                   // stream of the last call (kNoStream: none yet); its event is the latest pending one, if any is
   bool unwatched;                      // words are on their way to the ring that no event tells of
 };
 
@@ -79,7 +81,6 @@ bool capturing(cudaStream_t st) {
 // the kernel).
 cudaError_t queue_status(Call* c, cudaStream_t st, bool by_copy) {
   if (capturing(st)) return cudaSuccess;
-  if (c->count >= kSlots) return cudaSuccess;              // several threads on one plan: this call goes unwatched
   const int slot = c->next;
   const int32_t* words = static_cast<const int32_t*>(c->scratch->status);
   cudaError_t e = cudaSuccess;
@@ -94,6 +95,7 @@ cudaError_t queue_status(Call* c, cudaStream_t st, bool by_copy) {
     c->unwatched = true;
     return e;
   }
+  c->last = st;
   c->next = (slot + 1) % kSlots;
   ++c->count;
   return cudaSuccess;
@@ -145,7 +147,7 @@ PyObject* py_attach(PyObject*, PyObject* args) {
     free_rings.pop_back();
   }
   Call* c = new Call{reinterpret_cast<const pbs_shape_t*>(shape), reinterpret_cast<const pbs_scratch_t*>(scratch), ring,
-                     device, reinterpret_cast<PrefillFn>(fn), reinterpret_cast<ExportFn>(fn2), {}, 0, 0, 0, 0, 0, false};
+                     device, reinterpret_cast<PrefillFn>(fn), reinterpret_cast<ExportFn>(fn2), {}, 0, 0, 0, 0, 0, kNoStream, false};
   return PyCapsule_New(c, kName, destroy);
   END_HANDLE_TH_ERRORS
 }
@@ -165,6 +167,20 @@ PyObject* py_inspect(PyObject*, PyObject* args) {
   PyObject* words = PyList_New(8);
   for (int i = 0; words && i < 8; ++i) PyList_SET_ITEM(words, i, PyLong_FromLong(c->ring[8 * slot + i]));
   return words;
+}
+
+// follow(call, stream): the next call, on this stream, comes after the last one.  The plan's device is current.
+PyObject* py_follow(PyObject*, PyObject* args) {
+  PyObject* capsule;
+  unsigned long long stream;
+  if (!PyArg_ParseTuple(args, "OK", &capsule, &stream)) return nullptr;
+  Call* c = get(capsule);
+  if (!c) return nullptr;
+  const cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (c->count == 0 || st == c->last || capturing(st)) Py_RETURN_NONE;   // (a capture cannot wait for work outside)
+  const cudaError_t e = cudaStreamWaitEvent(st, c->landed[(c->next + kSlots - 1) % kSlots], 0);
+  if (e != cudaSuccess) return PyErr_Format(PyExc_RuntimeError, "wait for the last call of the plan: %s", cudaGetErrorString(e));
+  Py_RETURN_NONE;
 }
 
 // queue(call, stream): the plan's device is current
@@ -193,6 +209,27 @@ bool readable(const at::Tensor& t, bool distinct_heads) {
   if (((st[0] | st[1] | st[2]) * t.element_size()) % 16 || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16) return false;
   return !distinct_heads || ((st[0] > 0 || sz[0] == 1) && (st[1] > 0 || sz[1] == 1));
 }
+
+// A plan's lock for as long as this lives, if nobody has it.
+class TryLock {
+ public:
+  explicit TryLock(PyObject* plan) : lock_(PyObject_GetAttrString(plan, "_lock")) {
+    if (!lock_) return;
+    THPObjectPtr got(PyObject_CallMethod(lock_.get(), "acquire", "O", Py_False));
+    held = got.get() == Py_True;
+  }
+  ~TryLock() {
+    if (!held) return;
+    PyObject *type, *value, *trace;
+    PyErr_Fetch(&type, &value, &trace);
+    THPObjectPtr done(PyObject_CallMethod(lock_.get(), "release", nullptr));
+    PyErr_Restore(type, value, trace);
+  }
+  bool held = false;
+
+ private:
+  THPObjectPtr lock_;
+};
 
 enum Flags { kForceFirst = 1, kMeanPooling = 2, kNoOwnSegment = 4 };
 
@@ -230,9 +267,15 @@ PyObject* py_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!capsule) return nullptr;
   if (!PyCapsule_IsValid(capsule.get(), kName)) Py_RETURN_NONE;
   Call* c = get(capsule.get());
+  const TryLock lock(plan);                                // the scratch serves one call at a time: Python waits for its turn
+  if (!lock.held) {
+    if (PyErr_Occurred()) return nullptr;
+    Py_RETURN_NONE;
+  }
   const c10::cuda::CUDAGuard guard(device);
   const cudaStream_t st = c10::cuda::getCurrentCUDAStream(device.index()).stream();
-  if (capturing(st) || landed_error(c, false) >= 0) Py_RETURN_NONE;   // (or an earlier call failed)
+  // (another stream than last time has to wait, and the scratch's memory to be told of it)
+  if (capturing(st) || st != c->last || landed_error(c, false) >= 0) Py_RETURN_NONE;   // (or an earlier call failed)
   at::Tensor out = at::empty_like(q);
   if (!readable(out, false)) Py_RETURN_NONE;
   pbs_options_t opt = {};
@@ -261,6 +304,7 @@ PyObject* py_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyMethodDef methods[] = {
     {"attach", py_attach, METH_VARARGS, "attach(shape, scratch, device, prefill, export_status): addresses of a plan's buffers -> its call object"},
     {"inspect", py_inspect, METH_VARARGS, "inspect(call, wait_all): None or the status words of a failed call"},
+    {"follow", py_follow, METH_VARARGS, "follow(call, stream): let the stream wait for the last call if that was on another one"},
     {"queue", py_queue, METH_VARARGS, "queue(call, stream): send the status words of the call just enqueued"},
     {"call", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_call)), METH_FASTCALL,
      "call(plans, q, k, v, block_size, segment_size, threshold, flags): the result, or None where Python has to do it"},

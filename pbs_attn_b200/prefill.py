@@ -9,6 +9,7 @@ from __future__ import annotations
 import ctypes as C
 import math
 import os
+import threading
 from typing import Optional, Union
 
 import torch
@@ -87,11 +88,19 @@ class Plan:
             self.perm_v, self.pooled_q, self.pooled_k, self.first_block, self.block_mask, self.tile_list,
             self.tile_count, self.status)])
         self._thr_dev = None
+        self._lock = threading.Lock()
+        self._streams = {torch.cuda.current_stream(dev).cuda_stream}
         # deferred status check: after every whole-path call the 8 status words are copied to pinned
         # host memory (asynchronously); the copies that have landed are inspected on entry to the next call
         self._status_ring = torch.zeros(_STATUS_SLOTS, 8, dtype=torch.int32).pin_memory()
         self._status_pending = []          # [(event, slot)], oldest first
         self._status_next = 0
+
+    # The scratch serves one call at a time, whoever makes it: calls are enqueued under the lock, and one on another stream than the
+    # last waits for that.  Streams that the memory has been used on, so that the allocator does not hand it on too early.
+    _lock = threading.Lock()
+    _streams = None
+    _last_stream = None                     # (of calls without the native part, which keeps its own)
 
     _kv_left_out = False                    # the last whole-path call may have left perm_k / perm_v as they were
     _native = None                          # the call object of csrc/host_call.cpp, which then keeps the pending status words
@@ -167,7 +176,7 @@ class Plan:
                             _cabi.POOL[query_pool_mode], _cabi.POOL[key_pool_mode], _cabi.ATTN_IMPL[attn_impl],
                             int(bool(no_permutation)), int(bool(diagonal_candidates)), int(bool(no_own_segment)), kv_in_place,
                             C.pointer(out_replicas) if out_replicas is not None else None)
-        opt._keep = out_replicas            # the struct must outlive the call
+        opt._keep = (out_replicas, self._thr_dev)       # these must outlive the call, also where another thread makes options meanwhile
         if kv_in_place and (no_permutation or self.dense) and self.dtype != torch.float32 and attn_impl != "simt":
             opt.reads_kv_in_place = True
         return opt
@@ -175,7 +184,8 @@ class Plan:
     def check_status(self):
         """Synchronises and raises if a kernel reported a device-side error (in the last call or in an
         earlier whole-path call whose status has not been inspected yet)."""
-        self._inspect_landed_status(wait_all=True)
+        with self._lock:
+            self._inspect_landed_status(wait_all=True)
         st = self.status.cpu()
         if int(st[0]) != 0:
             self._raise_status(st.tolist())
@@ -239,13 +249,28 @@ class Plan:
                                               _ptr(self.status), None, self._stream()), "pbs_attn_fwd")
 
     # ------------------------------------------------------------------ whole path
+    def _follow(self, stream):
+        """What is enqueued next, on ``stream``, comes after the last call (captures are ordered by whoever replays them)."""
+        handle = stream.cuda_stream
+        if self._native is not None:
+            _cabi.load_host().follow(self._native, handle)
+        elif self._status_pending and handle != self._last_stream and not torch.cuda.is_current_stream_capturing():
+            stream.wait_event(self._status_pending[-1][0])
+        self._last_stream = handle
+        if self._streams is not None and handle not in self._streams and not torch.cuda.is_current_stream_capturing():
+            self._streams.add(handle)
+            for t in (self.partials, self.rowstats, self.importance, self.key_indices, self.perm_k, self.perm_v, self.pooled_q, self.pooled_k,
+                      self.first_block, self.block_mask, self.tile_list, self.tile_count, self.status):
+                t.record_stream(stream)
+
     def run(self, q, k, v, out, opt: _cabi.Options):
         """The whole path.  Never synchronises: a device-side error of an EARLIER call (its status words
         have reached the host by now) is raised here; this call's own status is queued for the next."""
-        if self._status_pending or self._native is not None:
-            self._inspect_landed_status()
-        with self._on_device():
+        with self._lock, self._on_device():
+            if self._status_pending or self._native is not None:
+                self._inspect_landed_status()
             stream = torch.cuda.current_stream(self.device)
+            self._follow(stream)
             _cabi.check(self.lib.pbs_prefill_fwd(C.byref(self.shape), _ptr(q), _strides(q), _ptr(k), _strides(k),
                                                  _ptr(v), _strides(v), _ptr(out), _strides(out), C.byref(opt),
                                                  C.byref(self.scratch), C.c_void_p(stream.cuda_stream)), "pbs_prefill_fwd")
