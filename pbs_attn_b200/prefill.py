@@ -486,6 +486,23 @@ class _HostPipeline:
         self.copy_out = torch.cuda.Stream(device)
         mk = lambda h: [torch.empty(B, h, S, D, dtype=dtype, device=device) for _ in range(2)]
         self.q, self.k, self.v, self.o = mk(hq_c), mk(hkv_c), mk(hkv_c), mk(hq_c)
+        self.lock = threading.Lock()
+        self.streams = {torch.cuda.current_stream(device).cuda_stream}
+        self.last = None                               # (stream, event) of the last call
+
+    def follow(self, main):
+        """The buffers serve one call at a time: one on another stream than the last waits for that, and the allocator is told."""
+        if self.last is not None and self.last[0] != main.cuda_stream:
+            main.wait_event(self.last[1])
+        if main.cuda_stream not in self.streams:
+            self.streams.add(main.cuda_stream)
+            for t in self.q + self.k + self.v + self.o:
+                t.record_stream(main)
+
+    def leave(self, main):
+        done = torch.cuda.Event()
+        done.record(main)
+        self.last = (main.cuda_stream, done)
 
 
 _HOST_PIPES: dict = {}
@@ -551,50 +568,53 @@ def permuted_block_sparse_attn_fwd_host(
     plan = get_plan(pipe.q[0], hkv_c, block_size, segment_size)
     opt = plan.options(threshold, force_select_first_block, query_pool_mode, key_pool_mode, kv_in_place=True)
     main = torch.cuda.current_stream(dev)
-    start = torch.cuda.Event()
-    start.record(main)
-    pipe.copy_in.wait_event(start)
-    pipe.copy_out.wait_event(start)
-    q_read = [None, None]            # last compute that read q/o staging slot s
-    kv_read = [None, None]           # last compute that read k/v staging slot s
-    o_read = [None, None]            # last download that read output slot s
-    kv_slot, kv_loaded, n_kv = 0, None, 0
-    for c in range(chunks):
-        s = c & 1
-        qs = slice(c * hq_c, (c + 1) * hq_c)
-        kv0 = (c * hq_c) // group
-        ks = slice(kv0, kv0 + hkv_c)
-        with torch.cuda.stream(pipe.copy_in):
-            if q_read[s] is not None:
-                pipe.copy_in.wait_event(q_read[s])
-            copies = [(pipe.q[s], query_states[:, qs])]
-            if kv_loaded != kv0:                       # a KV head shared with the previous chunk stays
-                kv_slot = n_kv & 1
-                n_kv += 1
-                kv_loaded = kv0
-                if kv_read[kv_slot] is not None:
-                    pipe.copy_in.wait_event(kv_read[kv_slot])
-                copies += [(pipe.k[kv_slot], key_states[:, ks]), (pipe.v[kv_slot], value_states[:, ks])]
-            for dst, src in copies:
+    with pipe.lock:
+        pipe.follow(main)
+        start = torch.cuda.Event()
+        start.record(main)
+        pipe.copy_in.wait_event(start)
+        pipe.copy_out.wait_event(start)
+        q_read = [None, None]            # last compute that read q/o staging slot s
+        kv_read = [None, None]           # last compute that read k/v staging slot s
+        o_read = [None, None]            # last download that read output slot s
+        kv_slot, kv_loaded, n_kv = 0, None, 0
+        for c in range(chunks):
+            s = c & 1
+            qs = slice(c * hq_c, (c + 1) * hq_c)
+            kv0 = (c * hq_c) // group
+            ks = slice(kv0, kv0 + hkv_c)
+            with torch.cuda.stream(pipe.copy_in):
+                if q_read[s] is not None:
+                    pipe.copy_in.wait_event(q_read[s])
+                copies = [(pipe.q[s], query_states[:, qs])]
+                if kv_loaded != kv0:                       # a KV head shared with the previous chunk stays
+                    kv_slot = n_kv & 1
+                    n_kv += 1
+                    kv_loaded = kv0
+                    if kv_read[kv_slot] is not None:
+                        pipe.copy_in.wait_event(kv_read[kv_slot])
+                    copies += [(pipe.k[kv_slot], key_states[:, ks]), (pipe.v[kv_slot], value_states[:, ks])]
+                for dst, src in copies:
+                    for b in range(B):
+                        dst[b].copy_(src[b], non_blocking=True)
+                ev_in = torch.cuda.Event()
+                ev_in.record(pipe.copy_in)
+            main.wait_event(ev_in)
+            if o_read[s] is not None:
+                main.wait_event(o_read[s])
+            plan.run(pipe.q[s], pipe.k[kv_slot], pipe.v[kv_slot], pipe.o[s], opt)
+            done = torch.cuda.Event()
+            done.record(main)
+            q_read[s] = done
+            kv_read[kv_slot] = done
+            with torch.cuda.stream(pipe.copy_out):
+                pipe.copy_out.wait_event(done)
                 for b in range(B):
-                    dst[b].copy_(src[b], non_blocking=True)
-            ev_in = torch.cuda.Event()
-            ev_in.record(pipe.copy_in)
-        main.wait_event(ev_in)
-        if o_read[s] is not None:
-            main.wait_event(o_read[s])
-        plan.run(pipe.q[s], pipe.k[kv_slot], pipe.v[kv_slot], pipe.o[s], opt)
-        done = torch.cuda.Event()
-        done.record(main)
-        q_read[s] = done
-        kv_read[kv_slot] = done
-        with torch.cuda.stream(pipe.copy_out):
-            pipe.copy_out.wait_event(done)
-            for b in range(B):
-                out[b, qs].copy_(pipe.o[s][b], non_blocking=True)
-            o_read[s] = torch.cuda.Event()
-            o_read[s].record(pipe.copy_out)
-    for ev in o_read:
-        if ev is not None:
-            main.wait_event(ev)
+                    out[b, qs].copy_(pipe.o[s][b], non_blocking=True)
+                o_read[s] = torch.cuda.Event()
+                o_read[s].record(pipe.copy_out)
+        for ev in o_read:
+            if ev is not None:
+                main.wait_event(ev)
+        pipe.leave(main)
     return out
