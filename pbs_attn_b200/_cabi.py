@@ -9,6 +9,7 @@ import ctypes as C
 import importlib.machinery
 import importlib.util
 import os
+import warnings
 
 # PBS_B200_LIB points at an alternative build of the same library (e.g. an instrumented one)
 _LIB_PATH = os.environ.get("PBS_B200_LIB") or os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "libpbs_b200.so")
@@ -114,17 +115,20 @@ _host = None
 
 
 def load_host():
-    """The native host side of the common call (csrc/host_call.cpp), loaded once; raises RuntimeError if it was not built."""
+    """The native host side of the common call (csrc/host_call.cpp), loaded once.  None where it was not built or was built for another
+    torch or Python (it is tied to their binary interfaces): calls then go through Python."""
     global _host
     if _host is None:
-        path = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "pbs_host.so")
-        if not os.path.exists(path):
-            raise RuntimeError(f"{path} is missing: build it with `python -m pbs_attn_b200.build`")
-        import torch  # noqa: F401  (the module links against its libraries)
-        loader = importlib.machinery.ExtensionFileLoader("pbs_host", path)
-        _host = importlib.util.module_from_spec(importlib.util.spec_from_loader("pbs_host", loader))
-        loader.exec_module(_host)
-    return _host
+        from . import build
+        path = build.host_path()
+        if os.path.exists(path):
+            loader = importlib.machinery.ExtensionFileLoader("pbs_host", path)
+            _host = importlib.util.module_from_spec(importlib.util.spec_from_loader("pbs_host", loader))
+            loader.exec_module(_host)
+        else:
+            warnings.warn(f"{path} is missing (`python -m pbs_attn_b200.build`): calls go through Python")
+            _host = False
+    return _host or None
 
 
 class PbsError(RuntimeError):

@@ -92,7 +92,7 @@ class Plan:
         self._streams = {torch.cuda.current_stream(dev).cuda_stream}
         # deferred status check: after every whole-path call the 8 status words are copied to pinned
         # host memory (asynchronously); the copies that have landed are inspected on entry to the next call
-        self._status_ring = torch.zeros(_STATUS_SLOTS, 8, dtype=torch.int32).pin_memory()
+        self._status_ring = None           # (of calls without the native part, which keeps its own)
         self._status_pending = []          # [(event, slot)], oldest first
         self._status_next = 0
 
@@ -120,7 +120,8 @@ class Plan:
 
     def _go_native(self):
         """The common call of this plan may run without Python (``_cabi.load_host().call``)."""
-        self._native = _cabi.load_host().attach(
+        host = _cabi.load_host()
+        self._native = host and host.attach(
             C.addressof(self.shape), C.addressof(self.scratch), self.device.index,
             C.cast(self.lib.pbs_prefill_fwd, C.c_void_p).value, C.cast(self.lib.pbs_export_status, C.c_void_p).value)
 
@@ -144,6 +145,8 @@ class Plan:
         if self._native is not None:
             return _cabi.load_host().queue(self._native, stream.cuda_stream)
         if self._status_rows is None:
+            if self._status_ring is None:
+                self._status_ring = torch.zeros(_STATUS_SLOTS, 8, dtype=torch.int32).pin_memory()
             ring = self._status_ring                        # the views live as long as the plan, and so does the ring
             self._status_words = (C.c_int32 * ring.numel()).from_address(ring.data_ptr())
             self._status_rows = ring.unbind(0)
@@ -339,9 +342,10 @@ def get_plan(q: torch.Tensor, kv_heads: int, block_size: int, segment_size: int)
 
 def _common_call(q, k, v, block_size, segment_size, threshold, force_first, mean_pooling=0, own_segment=True):
     """The call on a plan that exists, without Python in between; None for everything that the code below has to do."""
-    if not _PLANS:
+    host = _cabi.load_host() if _PLANS else None
+    if host is None:
         return None
-    return _cabi.load_host().call(_PLANS, q, k, v, block_size, segment_size, threshold,
+    return host.call(_PLANS, q, k, v, block_size, segment_size, threshold,
                                   (1 if force_first else 0) | mean_pooling | (0 if own_segment else 4))
 
 
