@@ -39,6 +39,7 @@ struct Call {
   int made, first, count, next;        // events created; pending slots: first .. first + count - 1
   int told;                            // so many of these, the oldest, are no longer looked at: an error among them has been raised
   cudaStream_t last;                   // stream of the last call (kNoStream: none yet); its event is the latest pending one, if any is
+  PyThread_type_lock turn;             // held while a call is enqueued
   bool unwatched;                      // words are on their way to the ring that no event tells of
 };
 
@@ -63,6 +64,7 @@ void sweep() {
     }
     for (int i = 0; i < c->made; ++i) (void)cudaEventDestroy(c->landed[i]);
     if (!c->unwatched) free_rings.push_back(c->ring);
+    PyThread_free_lock(c->turn);
     delete c;
   }
   leaving.resize(kept);
@@ -138,16 +140,21 @@ PyObject* py_attach(PyObject*, PyObject* args) {
   const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));   // pinned memory brings up the current device, which may be another one
   const Relaxed relaxed;
   sweep();
+  const PyThread_type_lock turn = PyThread_allocate_lock();
+  if (!turn) return PyErr_NoMemory();
   int32_t* ring = nullptr;
   if (free_rings.empty()) {
     const cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&ring), kSlots * 8 * sizeof(int32_t), cudaHostAllocPortable);
-    if (e != cudaSuccess) return PyErr_Format(PyExc_RuntimeError, "pinned memory for the status words: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+      PyThread_free_lock(turn);
+      return PyErr_Format(PyExc_RuntimeError, "pinned memory for the status words: %s", cudaGetErrorString(e));
+    }
   } else {
     ring = free_rings.back();
     free_rings.pop_back();
   }
   Call* c = new Call{reinterpret_cast<const pbs_shape_t*>(shape), reinterpret_cast<const pbs_scratch_t*>(scratch), ring,
-                     device, reinterpret_cast<PrefillFn>(fn), reinterpret_cast<ExportFn>(fn2), {}, 0, 0, 0, 0, 0, kNoStream, false};
+                     device, reinterpret_cast<PrefillFn>(fn), reinterpret_cast<ExportFn>(fn2), {}, 0, 0, 0, 0, 0, kNoStream, turn, false};
   return PyCapsule_New(c, kName, destroy);
   END_HANDLE_TH_ERRORS
 }
@@ -167,6 +174,23 @@ PyObject* py_inspect(PyObject*, PyObject* args) {
   PyObject* words = PyList_New(8);
   for (int i = 0; words && i < 8; ++i) PyList_SET_ITEM(words, i, PyLong_FromLong(c->ring[8 * slot + i]));
   return words;
+}
+
+// enter(call), leave(call): take and give back the turn
+PyObject* py_enter(PyObject*, PyObject* capsule) {
+  Call* c = get(capsule);
+  if (!c) return nullptr;
+  Py_BEGIN_ALLOW_THREADS
+  PyThread_acquire_lock(c->turn, WAIT_LOCK);
+  Py_END_ALLOW_THREADS
+  Py_RETURN_NONE;
+}
+
+PyObject* py_leave(PyObject*, PyObject* capsule) {
+  Call* c = get(capsule);
+  if (!c) return nullptr;
+  PyThread_release_lock(c->turn);
+  Py_RETURN_NONE;
 }
 
 // follow(call, stream): the next call, on this stream, comes after the last one.  The plan's device is current.
@@ -210,25 +234,14 @@ bool readable(const at::Tensor& t, bool distinct_heads) {
   return !distinct_heads || ((st[0] > 0 || sz[0] == 1) && (st[1] > 0 || sz[1] == 1));
 }
 
-// A plan's lock for as long as this lives, if nobody has it.
-class TryLock {
- public:
-  explicit TryLock(PyObject* plan) : lock_(PyObject_GetAttrString(plan, "_lock")) {
-    if (!lock_) return;
-    THPObjectPtr got(PyObject_CallMethod(lock_.get(), "acquire", "O", Py_False));
-    held = got.get() == Py_True;
+// A call's turn for as long as this lives, if nobody has it.
+struct TryTurn {
+  Call* c;
+  const bool held;
+  explicit TryTurn(Call* call) : c(call), held(PyThread_acquire_lock(call->turn, NOWAIT_LOCK)) {}
+  ~TryTurn() {
+    if (held) PyThread_release_lock(c->turn);
   }
-  ~TryLock() {
-    if (!held) return;
-    PyObject *type, *value, *trace;
-    PyErr_Fetch(&type, &value, &trace);
-    THPObjectPtr done(PyObject_CallMethod(lock_.get(), "release", nullptr));
-    PyErr_Restore(type, value, trace);
-  }
-  bool held = false;
-
- private:
-  THPObjectPtr lock_;
 };
 
 enum Flags { kForceFirst = 1, kMeanPooling = 2, kNoOwnSegment = 4 };
@@ -267,11 +280,8 @@ PyObject* py_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!capsule) return nullptr;
   if (!PyCapsule_IsValid(capsule.get(), kName)) Py_RETURN_NONE;
   Call* c = get(capsule.get());
-  const TryLock lock(plan);                                // the scratch serves one call at a time: Python waits for its turn
-  if (!lock.held) {
-    if (PyErr_Occurred()) return nullptr;
-    Py_RETURN_NONE;
-  }
+  const TryTurn turn(c);                                   // the scratch serves one call at a time: Python waits for its turn
+  if (!turn.held) Py_RETURN_NONE;
   const c10::cuda::CUDAGuard guard(device);
   const cudaStream_t st = c10::cuda::getCurrentCUDAStream(device.index()).stream();
   // (another stream than last time has to wait, and the scratch's memory to be told of it)
@@ -304,6 +314,8 @@ PyObject* py_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyMethodDef methods[] = {
     {"attach", py_attach, METH_VARARGS, "attach(shape, scratch, device, prefill, export_status): addresses of a plan's buffers -> its call object"},
     {"inspect", py_inspect, METH_VARARGS, "inspect(call, wait_all): None or the status words of a failed call"},
+    {"enter", py_enter, METH_O, "enter(call): wait for the call's turn and take it"},
+    {"leave", py_leave, METH_O, "leave(call): give the turn back"},
     {"follow", py_follow, METH_VARARGS, "follow(call, stream): let the stream wait for the last call if that was on another one"},
     {"queue", py_queue, METH_VARARGS, "queue(call, stream): send the status words of the call just enqueued"},
     {"call", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_call)), METH_FASTCALL,

@@ -40,6 +40,19 @@ def _readable(t: torch.Tensor, need_distinct_heads: bool = False) -> torch.Tenso
     return t if ok else t.contiguous()
 
 
+class _Turn:
+    """The lock of a plan whose common call runs without Python."""
+
+    def __init__(self, host, call):
+        self._host, self._call = host, call
+
+    def __enter__(self):
+        self._host.enter(self._call)
+
+    def __exit__(self, *exc):
+        self._host.leave(self._call)
+
+
 class Plan:
     """Shape, scratch buffers and stage calls for one (shape, device).
 
@@ -121,9 +134,12 @@ class Plan:
     def _go_native(self):
         """The common call of this plan may run without Python (``_cabi.load_host().call``)."""
         host = _cabi.load_host()
-        self._native = host and host.attach(
+        if host is None:
+            return
+        self._native = host.attach(
             C.addressof(self.shape), C.addressof(self.scratch), self.device.index,
             C.cast(self.lib.pbs_prefill_fwd, C.c_void_p).value, C.cast(self.lib.pbs_export_status, C.c_void_p).value)
+        self._lock = _Turn(host, self._native)
 
     def _inspect_landed_status(self, wait_all: bool = False):
         if self._native is not None:
@@ -335,8 +351,9 @@ def get_plan(q: torch.Tensor, kv_heads: int, block_size: int, segment_size: int)
     if plan is None:
         while len(_PLANS) >= _MAX_PLANS:
             _PLANS.pop(next(iter(_PLANS)))
-        plan = _PLANS[key] = Plan(B, Hq, kv_heads, S, D, block_size, segment_size, q.dtype, q.device)
+        plan = Plan(B, Hq, kv_heads, S, D, block_size, segment_size, q.dtype, q.device)
         plan._go_native()
+        _PLANS[key] = plan
     return plan
 
 
