@@ -6,6 +6,7 @@ for device memory and streams only; all arithmetic happens in the CUDA library.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import math
 import os
@@ -350,7 +351,7 @@ def get_plan(q: torch.Tensor, kv_heads: int, block_size: int, segment_size: int)
     plan = _PLANS.get(key)
     if plan is None:
         while len(_PLANS) >= _MAX_PLANS:
-            _PLANS.pop(next(iter(_PLANS)))
+            _PLANS.pop(next(iter(_PLANS), None), None)      # (another thread may have been here)
         plan = Plan(B, Hq, kv_heads, S, D, block_size, segment_size, q.dtype, q.device)
         plan._go_native()
         _PLANS[key] = plan
@@ -403,7 +404,8 @@ def permuted_block_sparse_attn_fwd(
         share memory with key_states or value_states;
       * ``out_replicas``: further destinations with ``out``'s strides that the attention kernel
         writes as well (buffers on peer GPUs of a head-sharded call, see ``peer_gather``).
-    Runs on the current CUDA stream without synchronising.
+    Runs on the current CUDA stream without synchronising.  Calls of one shape share their scratch: on several streams or
+    threads they come one after the other.
     """
     if (intermediates is None and out is None and out_replicas is None and causal and attn_impl == "auto"
             and query_pool_mode == "mean" and key_pool_mode == "mean"):
@@ -511,19 +513,25 @@ class _HostPipeline:
         self.streams = {torch.cuda.current_stream(device).cuda_stream}
         self.last = None                               # (stream, event) of the last call
 
-    def follow(self, main):
-        """The buffers serve one call at a time: one on another stream than the last waits for that, and the allocator is told."""
-        if self.last is not None and self.last[0] != main.cuda_stream:
-            main.wait_event(self.last[1])
-        if main.cuda_stream not in self.streams:
-            self.streams.add(main.cuda_stream)
-            for t in self.q + self.k + self.v + self.o:
-                t.record_stream(main)
-
-    def leave(self, main):
-        done = torch.cuda.Event()
-        done.record(main)
-        self.last = (main.cuda_stream, done)
+    @contextlib.contextmanager
+    def turn(self, main):
+        """The buffers serve one call at a time: one on another stream than the last waits for that, also if it failed half-way, and the
+        allocator is told of the stream."""
+        with self.lock:
+            if self.last is not None and self.last[0] != main.cuda_stream:
+                main.wait_event(self.last[1])
+            if main.cuda_stream not in self.streams:
+                self.streams.add(main.cuda_stream)
+                for t in self.q + self.k + self.v + self.o:
+                    t.record_stream(main)
+            try:
+                yield
+            finally:
+                for side in (self.copy_in, self.copy_out):
+                    main.wait_stream(side)
+                done = torch.cuda.Event()
+                done.record(main)
+                self.last = (main.cuda_stream, done)
 
 
 _HOST_PIPES: dict = {}
@@ -589,8 +597,7 @@ def permuted_block_sparse_attn_fwd_host(
     plan = get_plan(pipe.q[0], hkv_c, block_size, segment_size)
     opt = plan.options(threshold, force_select_first_block, query_pool_mode, key_pool_mode, kv_in_place=True)
     main = torch.cuda.current_stream(dev)
-    with pipe.lock:
-        pipe.follow(main)
+    with pipe.turn(main):
         start = torch.cuda.Event()
         start.record(main)
         pipe.copy_in.wait_event(start)
@@ -634,8 +641,4 @@ def permuted_block_sparse_attn_fwd_host(
                     out[b, qs].copy_(pipe.o[s][b], non_blocking=True)
                 o_read[s] = torch.cuda.Event()
                 o_read[s].record(pipe.copy_out)
-        for ev in o_read:
-            if ev is not None:
-                main.wait_event(ev)
-        pipe.leave(main)
     return out

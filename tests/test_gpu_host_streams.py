@@ -46,3 +46,27 @@ def test_host_calls_on_several_streams(threads):
                 work(i, [n])
     torch.cuda.synchronize()
     assert all(torch.equal(g, w) for gs, w in zip(got, want) for g in gs)
+
+
+def test_a_call_that_fails_half_way(monkeypatch):
+    from pbs_attn_b200 import prefill
+    a, b = _inputs(2)
+    want = _call(b)
+    torch.cuda.synchronize()
+    run, calls = prefill.Plan.run, []
+
+    def second_fails(self, *args):
+        calls.append(1)
+        if len(calls) == 2:
+            raise RuntimeError("second chunk")
+        return run(self, *args)
+
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    monkeypatch.setattr(prefill.Plan, "run", second_fails)
+    with torch.cuda.stream(streams[0]), pytest.raises(RuntimeError, match="second chunk"):
+        torch.cuda._sleep(50_000_000)
+        _call(a)
+    with torch.cuda.stream(streams[1]):
+        got = _call(b)
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
