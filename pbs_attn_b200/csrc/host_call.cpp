@@ -79,8 +79,8 @@ bool capturing(cudaStream_t st) {
 
 // Sends the status words of the call just enqueued to its slot of the ring.  Not those of a captured call: it is replayed at times unknown
 // here, perhaps after the plan is gone (check_status reads the device's words).  by_copy: for calls that go through Python, the
-// host-tensor call's among them, whose kernels would wait behind the copies out with a store to the host (16384 tokens 4.95 ms so, 5.19 with
-// the kernel).
+// host-tensor call's among them, whose own copies out it queues with (16384 tokens 4.95 ms so, 5.19 with the kernel); for all others the
+// kernel is ahead (pbs_api.cu has the figures).
 cudaError_t queue_status(Call* c, cudaStream_t st, bool by_copy) {
   if (capturing(st)) return cudaSuccess;
   const int slot = c->next;

@@ -128,8 +128,9 @@ int check_pool(int mode) {
   return PBS_OK;
 }
 
-// For short calls a kernel and not a copy: between short kernels the copy engine's turn costs more than the call (187 tokens, calls back to
-// back: 28.2 us with a copy, 21.5 so).
+// A kernel and not a copy, whose turn on the copy engine costs more than a short call and waits for whatever the program copies out beside
+// it.  us a call, kernel / copy, back to back and while another stream copies 32 MB pieces to the host: 187 tokens 21.5 / 27.7 and 52 / 812,
+// 1024 102 / 106 and 175 / 1080, 4096 271 / 275 and 346 / 1106, 8192 700 / 696 and 752 / 1160, 16384 2246 / 2237 and 2266 / 2268.
 __global__ void export_status_kernel(const int32_t* __restrict__ status, int32_t* __restrict__ host_words) {
   host_words[threadIdx.x] = status[threadIdx.x];
 }

@@ -24,7 +24,7 @@
 // An issuer runs, per list entry and half h: O += P_h V_h, then S_h of the next entry into the
 // columns P_h vacated.  One issuer's barrier bookkeeping overlaps the other issuer's MMAs.
 //
-// What bounds it.  TMEM has no room for a second S, so each of the four (query tile, key half) chains S -> P -> P V -> next S
+// What bounds it.  At head_dim 128 TMEM has no room for a second S (at 64 it would have, unused), so each of the four (query tile, key half) chains S -> P -> P V -> next S
 // is serial, and its latency is what counts: about 1300 cycles of softmax and as many of MMAs and hand-overs, while
 // the tensor pipe needs 2560 cycles for the four (K = 16 of S at N = 64 takes 48 cycles and not 32, because shared memory
 // delivers 128 bytes a cycle) and the special-function units 2048.  With one softmax warpgroup per query tile for both halves, as
@@ -235,9 +235,10 @@ __device__ __forceinline__ float ex2(float x) {
   return r;
 }
 
-// Two probabilities as the MMA takes them; `add` sums them up in fp32.  The row sum is that of the rounded probabilities, so that where
-// few of them matter the rounding cancels in O / l: error of a call against 64 bits 2.25e-3 -> 2.23e-3 at 32768 sparse tokens,
-// 2.30e-3 with the sum of the unrounded ones and this kernel's references (which need not be the row maximum).
+// Two probabilities as the MMA takes them; `add` sums them up in fp32.  The row sum is that of the weights that P V uses, so that O / l is an
+// average of V with weights that add up to one.  Relative error of a call against 64 bits, 1e-3, so / with the sum of the unrounded ones / with
+// that and running maxima, as it was: 32768 sparse tokens 2.227 / 2.307 / 2.253, 8192 tokens of head_dim 64 2.184 / 2.254 / 2.256, 4 x 2048 2.064 /
+// 2.096 / 2.133; lowest so in all 14 cases tried, fp16 among them.  (The unrounded sum takes 1 to 3 % less time.)
 template <int DT> struct PackP;
 template <> struct PackP<PBS_BF16> {
   static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
@@ -524,8 +525,8 @@ __device__ __noinline__ Refs before_exp(Refs r, uint32_t ent, uint32_t tmem, uin
 
 // References are raised by whole numbers, so that all is scaled by powers of two, exactly, and the result does not depend on who
 // scales what and when.  Only where nothing is left of what was, by more than 127, to the maximum itself: from references of 10^10 (keys
-// that a caller has pushed far down) a whole number leads to within a unit of 1024, not to the maximum.  A half-step k that finds a sum above kSumMost raises them: it waits for the P V of k - 1, which the old ones
-// belong to, publishes the new ones and scales O.  S_k is still in TMEM, and since P_k has not been handed over, neither P V of k nor of the
+// that a caller has pushed far down) a whole number leads to within a unit of 1024, not to the maximum.  A half-step k that finds a sum above
+// kSumMost raises them: it waits for the P V of k - 1, which the old ones belong to, publishes the new ones and scales O.  S_k is still in TMEM, and since P_k has not been handed over, neither P V of k nor of the
 // partner's k + 1 can start: O and P_{k+1} are its own.  P_{k+1} is always formed with the references before and then scaled.  Its warp reads
 // the epoch after it has seen its S: if that S is not there yet it will see the new epoch and scale by itself.  Otherwise its
 // progress says when it is through: with the old epoch its P is scaled here and its sum by itself once it sees the epoch; or it

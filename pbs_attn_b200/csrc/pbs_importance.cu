@@ -225,7 +225,9 @@ __device__ __forceinline__ float2 div_by(float2 x, float z, float rz) {
 // The first pass leaves the memory system idle (0.45 TB/s at 4 x 2048 tokens) and its issue slots half used, so CTAs that pool the query
 // blocks, which is nothing but reading, run among its own (whole calls: 4 x 2048 tokens 381 -> 373 us, 8192 tokens of head_dim 64 491 -> 478,
 // block_size 64 at 32768 tokens 7594 -> 7536, 6001 tokens fp16 and 32768 sparse tokens alike).  Four query blocks a half CTA: with 16 the
-// pooling is a tail of its own (410 us), with one or two 378, all at the head of a group's CTAs instead of the end 391.
+// pooling is a tail of its own (410 us), with one or two 378, all at the head of a group's CTAs instead of the end 391.  The first pass
+// spills 8 to 40 bytes with it and counts 16 barriers (one per half, by a run-time number); with halves that walk in step behind __syncthreads it
+// does neither and takes as long (4 x 2048 tokens 369.2 and 369.0 us a call, 8192 of head_dim 64 479.3 and 479.9, 32768 sparse 4364 and 4367).
 // FASTDIV: rounding a * (1 / sqrt(D)) to the input type gives the same bits as rounding a / sqrt(D)
 // for EVERY value a of that type (established on the host by trying all 65536 of them)
 // DH: head_dim when it is 64 or 128 (loops unroll, index arithmetic folds), 0 = any multiple of 16

@@ -20,12 +20,10 @@ namespace pbs {
 // the last full wave and what is left over; those are dealt out group by group, the longest of all heads left first.
 // The counter of the draws has to belong to one launch alone.  The whole-path call has such a word (its scratch serves one
 // call at a time and is cleared at its start); the stage call has not, because its status words may be shared by launches
-// that overlap.  It starts a CTA per entry instead, in the same order, which costs a start-up an entry (with two softmax
-// warpgroups a CTA, as all figures here): 4 x 2048 tokens
-// 209 us (queue 200, fixed pairs 222), 6001 sparse tokens 221 (221, 246), head_dim 64 378 (378, 441), longer ones alike.
-// Measured against fixed pairs (this kernel alone, 32 heads): 4 x 2048 tokens 229 -> 208 us, 6001 sparse tokens
-// 253 -> 224, 8192 tokens 533 -> 486 (head_dim 64: 448 -> 384), 32768 sparse tokens 4.25 -> 4.13 ms; with 13 waves or
-// more of equal pairs nothing changes (4 heads of 131072 tokens: 14.3 ms both ways).
+// that overlap.  It starts a CTA per entry instead, in the same order, which costs a start-up an entry.
+// us of a whole call with the queue / a CTA per entry / fixed pairs, 32 heads: 4 x 2048 tokens 368 / 377 / 396, 6001 sparse tokens (fp16) 346 /
+// 348 / 379, 8192 of head_dim 64 478 / 481 / 535, a layer of 8192 1287 / 1295 / 1326, 32768 sparse 4337 / 4338 / 4490; 4 heads of 131072
+// tokens 14.36 / 14.34 / 14.49 ms.
 struct Schedule {
   int n_items, G, BH;               // query groups of all heads; groups a head; heads of all sequences
   int ctas;                         // CTAs that share the work out of a queue, at most one a SM
