@@ -44,7 +44,7 @@ from pbs_attn_b200.synth import WORKLOADS, Workload, make_qkv, make_qkv_heads  #
 # capture summarised in the named file under profiles/, with the commit whose kernel was captured: a later
 # change of the kernel makes the figure stale until the capture is repeated.  Other workloads have none.
 ATTN_KERNEL_DRAM_TRAFFIC = {
-    "llama8b_heads_s131072": {"bytes": 20.20e9, "commit": "8ed0ae1", "profile": "profiles/attn_tc_kernel_llama8b_s32768.txt"},
+    "llama8b_heads_s131072": {"bytes": 7.86e9, "commit": "43f29a5", "profile": "profiles/attn_tc_kernel_dram_s131072.txt"},
 }
 
 METRIC = "prefill_attn_selected_block_tflops"
