@@ -232,6 +232,8 @@ int pbs_build_tile_lists(const pbs_shape_t* shape, const uint8_t* block_mask,
  * pbs_attn/src/kernels/permuted_block_sparse_attention.py:134-311.
  * status: 8 int32 words, word 0 zero on entry; it becomes non-zero if a bounded device-side
  * wait ran out (the output is then invalid, and that of a launch that shares the words and still runs).
+ * Range of V: the sum of P V is held in fp32 before it is divided by the row sum.  For bf16 it is at most 2^8 |V| per 64 keys
+ * that a row attends, so |V| up to 2^109 is safe for 131072 keys (2^119 for 128); fp16 values cannot leave it.
  * out_replicas: NULL or extra destinations. */
 int pbs_attn_fwd(const pbs_shape_t* shape,
                  const void* q, const int64_t q_strides[4],
